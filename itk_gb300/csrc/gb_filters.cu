@@ -10,13 +10,13 @@
 //   ShrinkImageFilter geometry                  Filtering/ImageGrid/include/itkShrinkImageFilter.hxx:230-290
 //   metric's default gradient filter settings   Registration/Metricsv4/include/itkImageToImageMetricv4.hxx:488-503
 //
-// Each 1-D pass is one thread per image line: the causal recursion runs
-// forward and is stored, the anticausal recursion runs backward and is added,
-// both with the reference's edge-extension start-up.  Lines along y and z are
-// adjacent in x across the threads of a warp, so their loads coalesce; lines
-// along x read one element per thread per step and lean on L1.  The
-// coefficients come from FP64 on the host; the recursions run in FP32 (the
-// reference filters in double and, for float images, stores float between the
+// A 1-D pass keeps whole image lines in shared memory: a block copies a tile of
+// lines in once, runs the causal and the anticausal recursion of each line side by
+// side (they start at opposite ends) and writes their sum, so a pass reads and
+// writes the image once.  Passes that share their input share the copy, and the
+// gradient's last axis forms all three components and the direction product in one
+// kernel.  The coefficients come from FP64 on the host; the recursions run in FP32
+// (the reference filters in double and, for float images, stores float between the
 // smoothing passes).
 #include <cuda_runtime.h>
 
@@ -29,12 +29,20 @@
 
 namespace gb {
 
-// IIR coefficients of one pass: N0..N3, D1..D4, M1..M4, BN1..BN4, BM1..BM4.
+// IIR coefficients of one pass: N0..N3, D1..D4, M1..M4, and the steady states of the
+// causal and anticausal parts over a constant line of ones.
 struct RGCoef {
-  double n[4], d[4], m[4], bn[4], bm[4];
+  double n[4], d[4], m[4], edge_n, edge_m;
+};
+// The same as one five-tap recursion in either direction (step s is element s of the
+// causal part, the element s before the last of the anticausal part):
+//   o_s = sum_{k=0..4} a_k x_{s-k} - sum_{k=1..4} d_k o_{s-k}.
+// Before the line, x is its first element x_0 and o its steady state x_0 edge.
+struct RGTaps {
+  float a[5], d[4], edge;
 };
 struct RGCoefF {
-  float n[4], d[4], m[4], bn[4], bm[4];
+  RGTaps dir[2];  // causal, anticausal
 };
 
 // Deriche-style recursive Gaussian with the parameters of Farneback and
@@ -62,6 +70,9 @@ static int rg_setup(double sigma, double spacing, int order, bool normalize_acro
   c.d[1] = 4 * cos2 * cos1 * e1 * e2;
   c.d[1] += e1 * e1 + e2 * e2;
   c.d[0] = -2 * (e2 * cos2 + e1 * cos1);
+  // the recursion runs with FP32 coefficients: the normalization below is that of the rounded
+  // poles, so that their rounding (of the order of the gain over a wide kernel) drops out
+  for (int k = 0; k < 4; ++k) c.d[k] = (double)(float)c.d[k];
   const double SD = 1.0 + c.d[0] + c.d[1] + c.d[2] + c.d[3];
   const double DD = c.d[0] + 2 * c.d[1] + 3 * c.d[2] + 4 * c.d[3];
   // numerator of the causal part
@@ -92,114 +103,341 @@ static int rg_setup(double sigma, double spacing, int order, bool normalize_acro
   c.m[1] = sgn * (c.n[2] - c.d[1] * c.n[0]);
   c.m[2] = sgn * (c.n[3] - c.d[2] * c.n[0]);
   c.m[3] = sgn * (-c.d[3] * c.n[0]);
-  // edge-extension start-up terms
+  // edge extension
   const double sn = c.n[0] + c.n[1] + c.n[2] + c.n[3];
   const double sm = c.m[0] + c.m[1] + c.m[2] + c.m[3];
   const double sdd = 1.0 + c.d[0] + c.d[1] + c.d[2] + c.d[3];
-  for (int k = 0; k < 4; ++k) {
-    c.bn[k] = c.d[k] * sn / sdd;
-    c.bm[k] = c.d[k] * sm / sdd;
-  }
+  c.edge_n = sn / sdd;
+  c.edge_m = sm / sdd;
   return GB_OK;
 }
 
 static RGCoefF to_float(const RGCoef& c) {
   RGCoefF f;
+  // the last (smallest) tap takes up the others' roundings, which keeps the taps' sum
+  double rn = 0.0, rm = 0.0;
   for (int k = 0; k < 4; ++k) {
-    f.n[k] = (float)c.n[k];
-    f.d[k] = (float)c.d[k];
-    f.m[k] = (float)c.m[k];
-    f.bn[k] = (float)c.bn[k];
-    f.bm[k] = (float)c.bm[k];
+    f.dir[0].a[k] = (float)(c.n[k] + (k == 3 ? rn : 0.0));
+    f.dir[1].a[k + 1] = (float)(c.m[k] + (k == 3 ? rm : 0.0));
+    rn += c.n[k] - (double)f.dir[0].a[k];
+    rm += c.m[k] - (double)f.dir[1].a[k + 1];
+    f.dir[0].d[k] = f.dir[1].d[k] = (float)c.d[k];
   }
+  f.dir[0].a[4] = f.dir[1].a[0] = 0.f;
+  f.dir[0].edge = (float)c.edge_n;
+  f.dir[1].edge = (float)c.edge_m;
   return f;
 }
 
-// One pass along an axis.  Line l = (j1, j2) starts at j1 * s1 + j2 * s2 and has
-// ln elements `step` apart.  out = (causal + anticausal) * scale; in != out.
-__global__ void __launch_bounds__(128) k_rg_lines(const float* __restrict__ in, float* __restrict__ out, RGCoefF c,
-                                                  int64_t ln, int64_t step, int64_t n1, int64_t s1, int64_t n2,
-                                                  int64_t s2, float scale) {
-  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= n1 * n2) return;
-  const float* x = in + (id % n1) * s1 + (id / n1) * s2;
-  float* y = out + (id % n1) * s1 + (id / n1) * s2;
-  // causal: y_i = sum_k n_k x_{i-k} - sum_k d_k y_{i-k}; before the line x = x_0 and
-  // the feedback of the missing outputs is x_0 bn_k
-  const float v1 = __ldg(x);
-  const float x1 = __ldg(x + step), x2 = __ldg(x + 2 * step), x3 = __ldg(x + 3 * step);
-  float o0 = v1 * c.n[0] + v1 * c.n[1] + v1 * c.n[2] + v1 * c.n[3];
-  o0 -= v1 * c.bn[0] + v1 * c.bn[1] + v1 * c.bn[2] + v1 * c.bn[3];
-  float o1 = x1 * c.n[0] + v1 * c.n[1] + v1 * c.n[2] + v1 * c.n[3];
-  o1 -= o0 * c.d[0] + v1 * c.bn[1] + v1 * c.bn[2] + v1 * c.bn[3];
-  float o2 = x2 * c.n[0] + x1 * c.n[1] + v1 * c.n[2] + v1 * c.n[3];
-  o2 -= o1 * c.d[0] + o0 * c.d[1] + v1 * c.bn[2] + v1 * c.bn[3];
-  float o3 = x3 * c.n[0] + x2 * c.n[1] + x1 * c.n[2] + v1 * c.n[3];
-  o3 -= o2 * c.d[0] + o1 * c.d[1] + o0 * c.d[2] + v1 * c.bn[3];
-  y[0] = o0;
-  y[step] = o1;
-  y[2 * step] = o2;
-  y[3 * step] = o3;
-  float xm1 = x3, xm2 = x2, xm3 = x1;        // x_{i-1}, x_{i-2}, x_{i-3}
-  float ym1 = o3, ym2 = o2, ym3 = o1, ym4 = o0;  // y_{i-1} .. y_{i-4}
-  for (int64_t i = 4; i < ln; ++i) {
-    const float xi = __ldg(x + i * step);
-    float o = xi * c.n[0] + xm1 * c.n[1] + xm2 * c.n[2] + xm3 * c.n[3];
-    o -= ym1 * c.d[0] + ym2 * c.d[1] + ym3 * c.d[2] + ym4 * c.d[3];
-    y[i * step] = o;
-    xm3 = xm2;
-    xm2 = xm1;
-    xm1 = xi;
-    ym4 = ym3;
-    ym3 = ym2;
-    ym2 = ym1;
-    ym1 = o;
+__device__ __forceinline__ void copy_async4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+// n copies from src, src + hop, ... to dst, dst + inc, ..., their addresses formed ahead in
+// groups (a copy holds its address register until it has been read).
+template <bool WIDE>
+__device__ __forceinline__ void copy_async_rows(float* dst, int inc, const float* src, int64_t hop, int n) {
+  constexpr int kGroup = 8;
+  for (; n >= kGroup; n -= kGroup) {
+    const float* p[kGroup];
+#pragma unroll
+    for (int u = 0; u < kGroup; ++u) p[u] = src + u * hop;
+#pragma unroll
+    for (int u = 0; u < kGroup; ++u) WIDE ? copy_async16(dst + u * inc, p[u]) : copy_async4(dst + u * inc, p[u]);
+    src += kGroup * hop;
+    dst += kGroup * inc;
   }
-  // anticausal: z_{i-1} = sum_k m_k x_{i-1+k} - sum_k d_k z_{i-1+k}, x = x_{ln-1} beyond the end
-  const int64_t L = ln - 1;
-  const float v2 = __ldg(x + L * step);
-  const float a1 = __ldg(x + (L - 1) * step), a2 = __ldg(x + (L - 2) * step);
-  float z0 = v2 * c.m[0] + v2 * c.m[1] + v2 * c.m[2] + v2 * c.m[3];  // z_{L}
-  z0 -= v2 * c.bm[0] + v2 * c.bm[1] + v2 * c.bm[2] + v2 * c.bm[3];
-  float z1 = v2 * c.m[0] + v2 * c.m[1] + v2 * c.m[2] + v2 * c.m[3];  // z_{L-1}
-  z1 -= z0 * c.d[0] + v2 * c.bm[1] + v2 * c.bm[2] + v2 * c.bm[3];
-  float z2 = a1 * c.m[0] + v2 * c.m[1] + v2 * c.m[2] + v2 * c.m[3];  // z_{L-2}
-  z2 -= z1 * c.d[0] + z0 * c.d[1] + v2 * c.bm[2] + v2 * c.bm[3];
-  float z3 = a2 * c.m[0] + a1 * c.m[1] + v2 * c.m[2] + v2 * c.m[3];  // z_{L-3}
-  z3 -= z2 * c.d[0] + z1 * c.d[1] + z0 * c.d[2] + v2 * c.bm[3];
-  y[L * step] = (y[L * step] + z0) * scale;
-  y[(L - 1) * step] = (y[(L - 1) * step] + z1) * scale;
-  y[(L - 2) * step] = (y[(L - 2) * step] + z2) * scale;
-  y[(L - 3) * step] = (y[(L - 3) * step] + z3) * scale;
-  // z_{i-1} for i = L-3 .. 1 from x_i, x_{i+1}, x_{i+2}, x_{i+3} and z_i .. z_{i+3}
-  float r1 = a2, r2 = a1, r3 = v2;               // x_{i+1}, x_{i+2}, x_{i+3} at i = L - 3
-  float zp1 = z3, zp2 = z2, zp3 = z1, zp4 = z0;  // z_i, z_{i+1}, z_{i+2}, z_{i+3}
-  for (int64_t i = L - 3; i > 0; --i) {
-    const float xi = __ldg(x + i * step);
-    float z = xi * c.m[0] + r1 * c.m[1] + r2 * c.m[2] + r3 * c.m[3];
-    z -= zp1 * c.d[0] + zp2 * c.d[1] + zp3 * c.d[2] + zp4 * c.d[3];
-    y[(i - 1) * step] = (y[(i - 1) * step] + z) * scale;
-    r3 = r2;
-    r2 = r1;
-    r1 = xi;
-    zp4 = zp3;
-    zp3 = zp2;
-    zp2 = zp1;
-    zp1 = z;
+  for (; n > 0; --n, src += hop, dst += inc) WIDE ? copy_async16(dst, src) : copy_async4(dst, src);
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The recursion's state, advanced one element at a time: what the elements so far add to
+// each of the next four outputs.  In this form an element's terms are independent of one
+// another, two multiply-adds separate an output from the next, and the terms of an output
+// are added oldest (and smallest) first, so the roundings stay small.  (Summed from the
+// last inputs and outputs instead, an output's nine terms ran one after another: 36 to 41
+// cycles an element, with one or two warps a scheduler to hide them.)
+struct RGLine {
+  float n1, n2, n3, n4;
+  __device__ __forceinline__ void start(const RGTaps& c, float x0) {
+    const float o = x0 * c.edge;
+    n4 = fmaf(c.a[4], x0, -c.d[3] * o);
+    n3 = fmaf(-c.d[2], o, fmaf(c.a[3], x0, n4));
+    n2 = fmaf(-c.d[1], o, fmaf(c.a[2], x0, n3));
+    n1 = fmaf(-c.d[0], o, fmaf(c.a[1], x0, n2));
+  }
+  __device__ __forceinline__ float step(const RGTaps& c, float x) {
+    const float o = fmaf(c.a[0], x, n1);
+    n1 = fmaf(-c.d[0], o, fmaf(c.a[1], x, n2));
+    n2 = fmaf(-c.d[1], o, fmaf(c.a[2], x, n3));
+    n3 = fmaf(-c.d[2], o, fmaf(c.a[3], x, n4));
+    n4 = fmaf(-c.d[3], o, c.a[4] * x);
+    return o;
+  }
+};
+
+// `count` elements of one line: x walks the shared-memory input by inc floats; put(outputs)
+// takes them in the same order, in groups of kRGRun and then one by one, after put.fetch has
+// requested what it adds to the next ones.  The next group of inputs is requested before the present one's outputs are stored (the compiler cannot
+// move a load above a store to shared memory).
+constexpr int kRGRun = 8;
+template <typename Put>
+__device__ __forceinline__ void rg_run(RGLine& l, const RGTaps& c, const float*& x, int inc, int count, Put& put) {
+  float v[kRGRun];
+  if (count >= kRGRun) {
+#pragma unroll
+    for (int u = 0; u < kRGRun; ++u) v[u] = x[u * inc];
+    put.fetch(kRGRun);
+    x += kRGRun * inc;
+    for (count -= kRGRun; count >= kRGRun; count -= kRGRun) {
+      float w[kRGRun];
+#pragma unroll
+      for (int u = 0; u < kRGRun; ++u) w[u] = x[u * inc];
+      x += kRGRun * inc;
+#pragma unroll
+      for (int u = 0; u < kRGRun; ++u) v[u] = l.step(c, v[u]);
+      put(v);
+      put.fetch(kRGRun);
+#pragma unroll
+      for (int u = 0; u < kRGRun; ++u) v[u] = w[u];
+    }
+#pragma unroll
+    for (int u = 0; u < kRGRun; ++u) v[u] = l.step(c, v[u]);
+    put(v);
+  }
+  for (; count > 0; --count, x += inc) {
+    put.fetch(1);
+    float one[1] = {l.step(c, *x)};
+    put(one);
   }
 }
 
-static cudaError_t rg_pass(cudaStream_t st, const float* in, float* out, const int64_t size[3], int axis,
-                           const RGCoef& c, float scale) {
-  const int64_t ln = size[axis];
-  const int64_t step = axis == 0 ? 1 : (axis == 1 ? size[0] : size[0] * size[1]);
-  // the two other axes, the faster-varying one first (x whenever it is not the filtered axis)
+// put of a recursion's first half: parked in shared memory.
+struct RGPark {
+  float* sum;
+  int inc;
+  __device__ __forceinline__ void fetch(int) {}
+  template <int N>
+  __device__ __forceinline__ void operator()(const float (&v)[N]) {
+#pragma unroll
+    for (int u = 0; u < N; ++u) sum[u * inc] = v[u];
+    sum += N * inc;
+  }
+};
+// put of its second half: the other recursion's parked part added and scaled, in place.
+struct RGAdd {
+  float* sum;
+  int inc;
+  float scale;
+  float e[kRGRun];
+  __device__ __forceinline__ void fetch(int n) {
+#pragma unroll
+    for (int u = 0; u < kRGRun; ++u)
+      if (u < n) e[u] = sum[u * inc];
+  }
+  template <int N>
+  __device__ __forceinline__ void operator()(const float (&v)[N]) {
+#pragma unroll
+    for (int u = 0; u < N; ++u) sum[u * inc] = (e[u] + v[u]) * scale;
+    sum += N * inc;
+  }
+};
+// The same, written to the output image.
+struct RGStore {
+  const float* sum;
+  int inc;
+  float scale;
+  float* dst;
+  int64_t step;
+  bool live;
+  float e[kRGRun];
+  __device__ __forceinline__ void fetch(int n) {
+#pragma unroll
+    for (int u = 0; u < kRGRun; ++u)
+      if (u < n) e[u] = sum[u * inc];
+    sum += n * inc;
+  }
+  template <int N>
+  __device__ __forceinline__ void operator()(const float (&v)[N]) {
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+      if (live) dst[u * step] = (e[u] + v[u]) * scale;
+    dst += N * step;
+  }
+};
+
+// One pass along an axis with NOUT outputs of the same input (NOUT pairs of warps: the
+// causal and the anticausal recursion of each output, a thread per line).  A block owns
+// kRGLines consecutive lines; line l starts at (l % n1) * s1 + (l / n1) * s2 and has ln
+// elements `step` apart.  X: the lines run along x (l * ln, step 1) and lie in shared
+// memory at an odd pitch, else element i of the tile's lines is row i: both without bank
+// conflicts.  The first `half` outputs of each recursion are parked in shared memory;
+// past that the other one has left its part there, and the sum is final.
+// One read and NOUT writes of the image; bound by the tiles in flight (8 or 12 bytes of
+// shared memory an element: two to four blocks per SM, each copying, filtering and storing
+// in turn).  Measured at 256x256x200 (one output along z, x, y; two outputs along x, y):
+// 33, 39, 28; 63, 49 us, where one thread per line through global memory took 141, 303,
+// 185; 605, 357 us.  A row of 32 lines is copied in 16-byte pieces where the lines come in
+// aligned groups of four: 4-byte copies took twice as long to issue.
+constexpr int kRGLines = 32;
+struct RGOut {
+  float* p;
+  float scale;
+  RGCoefF c;
+};
+struct RGPass {
+  const float* in;
+  RGOut out[2];
+  int64_t lines, step, n1, s1, s2;
+  int ln;
+  int wide;  // lines in groups of four at 16-byte boundaries (axes other than x)
+};
+__host__ __device__ inline int rg_pitch(int ln) { return ln | 1; }  // odd: a column of lines hits every bank
+static size_t rg_tile_bytes(bool x, int ln) { return sizeof(float) * kRGLines * (size_t)(x ? rg_pitch(ln) : ln); }
+
+// The recursion DIR (1 causal, -1 anticausal) of output o of the tile's lines.
+template <bool X, int DIR>
+__device__ __forceinline__ void rg_tile(const RGPass& a, float* tile, int o, int64_t l0, int64_t base, bool live) {
+  constexpr int kInc = X ? DIR : DIR * kRGLines;
+  const int ln = a.ln, lane = threadIdx.x & 31;
+  const int pitch = rg_pitch(ln), size = X ? kRGLines * pitch : kRGLines * ln;
+  const RGTaps c = a.out[o].c.dir[DIR < 0];
+  const float scale = a.out[o].scale;
+  const int half = DIR < 0 ? ln / 2 : (ln + 1) / 2;
+  const int first = X ? lane * pitch + (DIR < 0 ? ln - 1 : 0) : lane + (DIR < 0 ? (ln - 1) * kRGLines : 0);
+  const float* x = tile + first;
+  float* sum = tile + (1 + o) * size + first;
+  RGLine s;
+  s.start(c, *x);
+  RGPark park{sum, kInc};
+  rg_run(s, c, x, kInc, half, park);
+  __syncthreads();
+  sum += half * kInc;
+  if (X) {
+    RGAdd add{sum, kInc, scale};
+    rg_run(s, c, x, kInc, ln - half, add);
+  } else {
+    RGStore store{sum, kInc, scale, a.out[o].p + base + (DIR < 0 ? ln - 1 - half : half) * a.step,
+                  DIR * a.step, live};
+    rg_run(s, c, x, kInc, ln - half, store);
+  }
+}
+
+template <bool X, int NOUT>
+__global__ void __launch_bounds__(64 * NOUT) k_rg_pass(RGPass a) {
+  extern __shared__ float tile[];
+  const int ln = a.ln, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t l0 = (int64_t)blockIdx.x * kRGLines, l = l0 + lane;
+  const bool live = l < a.lines;
+  const int pitch = rg_pitch(ln);
+  const int size = X ? kRGLines * pitch : kRGLines * ln;
+  const int64_t base = X ? l * ln : (l % a.n1) * a.s1 + (l / a.n1) * a.s2;
+  if (X) {
+    const int rows = (int)min((int64_t)kRGLines, a.lines - l0);
+    for (int r = warp; r < rows; r += 2 * NOUT) {
+      const float* src = a.in + (l0 + r) * ln;
+      float* dst = tile + r * pitch;
+#pragma unroll 4
+      for (int i = lane; i < ln; i += 32) copy_async4(dst + i, src + i);
+    }
+  } else if (a.wide) {  // four lines at a time: a warp copies four rows
+    const int64_t w = l0 + 4 * (lane & 7);
+    const int i = 4 * warp + (lane >> 3);
+    if (w < a.lines && i < ln)
+      copy_async_rows<true>(tile + i * kRGLines + 4 * (lane & 7), 8 * NOUT * kRGLines,
+                            a.in + (w % a.n1) * a.s1 + (w / a.n1) * a.s2 + i * a.step, 8 * NOUT * a.step,
+                            (ln - i + 8 * NOUT - 1) / (8 * NOUT));
+  } else if (live && warp < ln) {
+    copy_async_rows<false>(tile + warp * kRGLines + lane, 2 * NOUT * kRGLines, a.in + base + warp * a.step,
+                           2 * NOUT * a.step, (ln - warp + 2 * NOUT - 1) / (2 * NOUT));
+  }
+  copy_async_wait();
+  __syncthreads();
+  // causal and anticausal warps take the same code with their own strides
+  if (warp & 1) rg_tile<X, -1>(a, tile, warp >> 1, l0, base, live);
+  else rg_tile<X, 1>(a, tile, warp >> 1, l0, base, live);
+  if (X) {
+    // rows leave in order
+    __syncthreads();
+    const int o = warp >> 1, rows = (int)min((int64_t)kRGLines, a.lines - l0);
+    const float* sum = tile + (1 + o) * size;
+    for (int r = warp & 1; r < rows; r += 2) {
+      float* dst = a.out[o].p + (l0 + r) * ln;
+      const float* src = sum + r * pitch;
+#pragma unroll 4
+      for (int i = lane; i < ln; i += 32) dst[i] = src[i];
+    }
+  }
+}
+
+// The same for lines too long for a tile: one thread per line, the causal part through
+// the output image.
+__global__ void __launch_bounds__(128) k_rg_long(RGPass a) {
+  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= a.lines) return;
+  const int64_t base = (id % a.n1) * a.s1 + (id / a.n1) * a.s2;
+  const float* x = a.in + base;
+  float* y = a.out[0].p + base;
+  const RGCoefF& c = a.out[0].c;
+  RGLine s;
+  s.start(c.dir[0], __ldg(x));
+  for (int64_t i = 0; i < a.ln; ++i) y[i * a.step] = s.step(c.dir[0], __ldg(x + i * a.step));
+  s.start(c.dir[1], __ldg(x + (a.ln - 1) * a.step));
+  for (int64_t i = a.ln - 1; i >= 0; --i)
+    y[i * a.step] = (y[i * a.step] + s.step(c.dir[1], __ldg(x + i * a.step))) * a.out[0].scale;
+}
+
+// Largest dynamic shared memory of a block.
+constexpr size_t kRGMaxShared = 227 * 1024;
+
+// The axis's lines: element step and count, and where line l = (j1, j2) starts; the two
+// other axes, the faster-varying one first (x whenever it is not the filtered axis).
+static RGPass rg_lines(const float* in, const int64_t size[3], int axis) {
+  RGPass a;
+  memset(&a, 0, sizeof(a));
+  a.in = in;
+  a.ln = (int)size[axis];
+  a.step = axis == 0 ? 1 : (axis == 1 ? size[0] : size[0] * size[1]);
   const int a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
-  const int64_t s1 = a1 == 0 ? 1 : size[0], s2 = a2 == 1 ? size[0] : size[0] * size[1];
-  const int64_t lines = size[a1] * size[a2];
-  const unsigned blocks = (unsigned)((lines + 127) / 128);
-  k_rg_lines<<<blocks, 128, 0, st>>>(in, out, to_float(c), ln, step, size[a1], s1, size[a2], s2, scale);
+  a.n1 = size[a1];
+  a.s1 = a1 == 0 ? 1 : size[0];
+  a.s2 = a2 == 1 ? size[0] : size[0] * size[1];
+  a.lines = size[a1] * size[a2];
+  a.wide = axis != 0 && size[0] % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0 ? 1 : 0;
+  return a;
+}
+
+template <bool X, int NOUT>
+static cudaError_t rg_launch(cudaStream_t st, const RGPass& a, size_t shared) {
+  // the same limit on every call: threads filtering images of different sizes share it
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_rg_pass<X, NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRGMaxShared);
+  if (e != cudaSuccess) return e;
+  k_rg_pass<X, NOUT><<<(unsigned)((a.lines + kRGLines - 1) / kRGLines), 64 * NOUT, shared, st>>>(a);
   return cudaGetLastError();
+}
+
+// nout (1 or 2) filters of one image along an axis.
+static cudaError_t rg_pass(cudaStream_t st, const float* in, const int64_t size[3], int axis, const RGOut* out,
+                           int nout) {
+  RGPass a = rg_lines(in, size, axis);
+  const size_t shared = (1 + nout) * rg_tile_bytes(axis == 0, a.ln);
+  if (shared > kRGMaxShared) {
+    if (nout == 2) {
+      const cudaError_t e = rg_pass(st, in, size, axis, out, 1);
+      return e != cudaSuccess ? e : rg_pass(st, in, size, axis, out + 1, 1);
+    }
+    a.out[0] = out[0];
+    k_rg_long<<<(unsigned)((a.lines + 127) / 128), 128, 0, st>>>(a);
+    return cudaGetLastError();
+  }
+  for (int k = 0; k < nout; ++k) a.out[k] = out[k];
+  if (axis == 0) return nout == 1 ? rg_launch<true, 1>(st, a, shared) : rg_launch<true, 2>(st, a, shared);
+  return nout == 1 ? rg_launch<false, 1>(st, a, shared) : rg_launch<false, 2>(st, a, shared);
 }
 
 // SmoothingRecursiveGaussianImageFilter: zero order along z, then x, then y.
@@ -218,29 +456,146 @@ int smooth_rg_device(cudaStream_t st, const float* in, float* out, float* t1, fl
   for (int p = 0; p < 3; ++p) {
     const int ax = order[p];
     if (rg_setup(sigma[ax], spacing[ax], 0, false, c) != GB_OK) return fail(GB_ERR_BAD_ARG, "sigma must be > 0");
-    cudaError_t e = rg_pass(st, src, dst[p], size, ax, c, 1.f);
+    const RGOut o{dst[p], 1.f, to_float(c)};
+    cudaError_t e = rg_pass(st, src, size, ax, &o, 1);
     if (e != cudaSuccess) return fail(GB_ERR_CUDA, std::string("smoothing pass: ") + cudaGetErrorString(e));
     src = dst[p];
   }
   return GB_OK;
 }
 
+// The direction matrix applied to a gradient.
+struct RGMatrix {
+  float m[9];
+  __device__ __forceinline__ float row(int r, float a, float b, float c) const {
+    return fmaf(m[3 * r], a, fmaf(m[3 * r + 1], b, m[3 * r + 2] * c));
+  }
+};
+
 // (value, D (gx, gy, gz)) per voxel, the gradient in physical units.
 __global__ void k_pack_gradient(const float* __restrict__ v, const float* __restrict__ gx,
-                                const float* __restrict__ gy, const float* __restrict__ gz, int64_t n, float d00,
-                                float d01, float d02, float d10, float d11, float d12, float d20, float d21,
-                                float d22, float4* __restrict__ out4, float* __restrict__ out3) {
+                                const float* __restrict__ gy, const float* __restrict__ gz, int64_t n, RGMatrix m,
+                                float4* __restrict__ out4, float* __restrict__ out3) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float a = gx[i], b = gy[i], c = gz[i];
-  const float px = fmaf(d00, a, fmaf(d01, b, d02 * c));
-  const float py = fmaf(d10, a, fmaf(d11, b, d12 * c));
-  const float pz = fmaf(d20, a, fmaf(d21, b, d22 * c));
-  if (out4) out4[i] = make_float4(v[i], px, py, pz);
-  if (out3) {
-    out3[3 * i] = px;
-    out3[3 * i + 1] = py;
-    out3[3 * i + 2] = pz;
+  if (out4) out4[i] = make_float4(v[i], m.row(0, a, b, c), m.row(1, a, b, c), m.row(2, a, b, c));
+  if (out3)
+    for (int r = 0; r < 3; ++r) out3[3 * i + r] = m.row(r, a, b, c);
+}
+
+// The gradient's last axis (z), its direction product and its packing in one kernel: the
+// three components' lines of a tile of kRGzLines lines, one warp per component (lanes
+// 0-15 the causal, 16-31 the anticausal recursion of the tile's lines), then float4
+// (value, gradient) or xyz triplets, each voxel's output written once.  Kept apart, the
+// three passes would write 12 and read 12 bytes a voxel more.  Element k from a line's
+// start lies in row 2k and element k from its end in row 2k + 1: both recursions walk
+// rows upwards to the middle and downwards past it by the same stride, in different banks.
+// 12 (with the value 16) bytes read and 12 or 16 written per voxel; bound as k_rg_pass is.
+// Measured at 256x256x200: 118 us (triplets), where three passes and the packing took 485.
+constexpr int kRGzLines = 16;
+struct RGGradZ {
+  const float* in[3];
+  const float* v;
+  RGOut out[3];  // p unused
+  RGMatrix m;
+  int64_t lines, step;
+  int ln;
+  int wide;  // lines in groups of four at 16-byte boundaries
+  float4* out4;
+  float* out3;
+};
+static size_t rgz_array(int ln) { return (size_t)kRGzLines * (size_t)ln; }
+
+__global__ void __launch_bounds__(96) k_rg_grad_z(RGGradZ a) {
+  extern __shared__ float tile[];
+  constexpr int kInc = 2 * kRGzLines;
+  const int ln = a.ln, lane = threadIdx.x & 31, comp = threadIdx.x >> 5;
+  const int line = lane & (kRGzLines - 1), back = lane >> 4;
+  const int size = kRGzLines * ln, half = ln / 2;
+  const int64_t l0 = (int64_t)blockIdx.x * kRGzLines;
+  const int64_t dir = back ? -a.step : a.step;                               // this lane's way along its line
+  const int64_t begin = l0 + line + (back ? (int64_t)(ln - 1) * a.step : 0);
+  const int mine = half + ((ln & 1) && !back ? 1 : 0);                       // rows of this parity
+  float* const xs = tile + 2 * comp * size + lane;
+  if (a.wide) {  // four lines at a time: a warp copies eight rows, the same way along each line
+    const int p = lane >> 2, w = 4 * (lane & 3);
+    const int64_t hop = (p & 1) ? -4 * a.step : 4 * a.step;
+    const int64_t from = l0 + w + ((p & 1) ? ln - 1 - (p >> 1) : p >> 1) * a.step;
+    if (l0 + w < a.lines && p < ln) {
+      copy_async_rows<true>(tile + 2 * comp * size + p * kRGzLines + w, 8 * kRGzLines, a.in[comp] + from, hop,
+                            (ln - p + 7) / 8);
+      if (a.out4 && p + 8 * comp < ln)
+        copy_async_rows<true>(tile + 6 * size + (p + 8 * comp) * kRGzLines + w, 24 * kRGzLines,
+                              a.v + from + comp * hop, 3 * hop, (ln - p - 8 * comp + 23) / 24);
+    }
+  } else if (l0 + line < a.lines) {
+    copy_async_rows<false>(xs, kInc, a.in[comp] + begin, dir, mine);
+    if (a.out4 && comp < mine)
+      copy_async_rows<false>(tile + 6 * size + lane + comp * kInc, 3 * kInc, a.v + begin + comp * dir, 3 * dir,
+                             (mine - comp + 2) / 3);
+  }
+  copy_async_wait();
+  __syncwarp();  // a warp's recursions read what the same warp has copied
+  RGTaps c;  // this lane's direction, by selection: no divergent copies
+#pragma unroll
+  for (int k = 0; k < 5; ++k) c.a[k] = back ? a.out[comp].c.dir[1].a[k] : a.out[comp].c.dir[0].a[k];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) c.d[k] = a.out[comp].c.dir[0].d[k];
+  c.edge = back ? a.out[comp].c.dir[1].edge : a.out[comp].c.dir[0].edge;
+  const float scale = a.out[comp].scale;
+  const float* x = xs;
+  RGLine s;
+  s.start(c, *x);
+  RGPark park{xs + size, kInc};
+  rg_run(s, c, x, kInc, half, park);
+  __syncwarp();
+  if (ln & 1) {  // the middle element, the last row, for both
+    float* m = xs - lane + size + (ln - 1) * kRGzLines + line;
+    const float v = s.step(c, xs[(ln - 1) * kRGzLines - lane + line]);
+    if (!back) *m = v;
+    __syncwarp();
+    if (back) *m = (*m + v) * scale;
+  }
+  // past the middle: the other recursion's rows, from the last one down
+  const int last = (half - 1) * kInc - lane + (lane ^ kRGzLines);
+  x = xs + last;
+  RGAdd add{xs + size + last, -kInc, scale};
+  rg_run(s, c, x, -kInc, half, add);
+  __syncthreads();
+  const float *g0 = tile + size, *g1 = tile + 3 * size, *g2 = tile + 5 * size, *v0 = tile + 6 * size;
+  constexpr int kOut = 8;  // rows read together
+  if (a.out4 && l0 + line < a.lines) {  // thread t: line t % 16 of every sixth row from t / 16
+    const int p = threadIdx.x >> 4;
+    const int64_t hop = (p & 1) ? -3 * a.step : 3 * a.step;
+    float4* dst = a.out4 + l0 + line + ((p & 1) ? ln - 1 - (p >> 1) : p >> 1) * a.step;
+    for (int q = threadIdx.x; q < size; q += 96 * kOut, dst += kOut * hop) {
+      float4 o[kOut];
+#pragma unroll
+      for (int u = 0; u < kOut; ++u)
+        if (q + 96 * u < size) o[u] = make_float4(v0[q + 96 * u], g0[q + 96 * u], g1[q + 96 * u], g2[q + 96 * u]);
+#pragma unroll
+      for (int u = 0; u < kOut; ++u)
+        if (q + 96 * u < size)
+          dst[u * hop] = make_float4(o[u].x, a.m.row(0, o[u].y, o[u].z, o[u].w), a.m.row(1, o[u].y, o[u].z, o[u].w),
+                                     a.m.row(2, o[u].y, o[u].z, o[u].w));
+    }
+  }
+  if (a.out3) {  // a row's 48 floats in order: thread t % 48 writes component t % 3 of line t / 3
+    const int p = threadIdx.x / (3 * kRGzLines), t = threadIdx.x % (3 * kRGzLines), r = t % 3, w = t / 3;
+    const float m0 = a.m.m[3 * r], m1 = a.m.m[3 * r + 1], m2 = a.m.m[3 * r + 2];
+    const int64_t hop = p ? -3 * a.step : 3 * a.step;
+    float* dst = a.out3 + 3 * (l0 + (p ? (int64_t)(ln - 1) * a.step : 0)) + t;
+    if (l0 + w < a.lines)
+      for (int q = p * kRGzLines + w; q < size; q += kInc * kOut, dst += kOut * hop) {
+        float o[kOut];
+#pragma unroll
+        for (int u = 0; u < kOut; ++u)
+          if (q + kInc * u < size) o[u] = fmaf(m0, g0[q + kInc * u], fmaf(m1, g1[q + kInc * u], m2 * g2[q + kInc * u]));
+#pragma unroll
+        for (int u = 0; u < kOut; ++u)
+          if (q + kInc * u < size) dst[u * hop] = o[u];
+      }
   }
 }
 
@@ -261,35 +616,61 @@ int gradient_rg_device(cudaStream_t st, const float* in, const int64_t size[3], 
   cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&buf), sizeof(float) * 5 * (size_t)n, st);
   if (e != cudaSuccess) return fail(GB_ERR_OUT_OF_MEMORY, "gradient filter scratch: out of device memory");
   float *A = buf, *B = buf + n, *C = buf + 2 * n, *D = buf + 3 * n, *E = buf + 4 * n;
-  RGCoef s[3], dv[3];
+  RGCoefF s[3], dv[3];
   int rc = GB_OK;
   for (int k = 0; k < 3 && rc == GB_OK; ++k) {
-    rc = rg_setup(sigma, spacing[k], 0, normalize_across_scale, s[k]);
-    if (rc == GB_OK) rc = rg_setup(sigma, spacing[k], 1, normalize_across_scale, dv[k]);
+    RGCoef c;
+    rc = rg_setup(sigma, spacing[k], 0, normalize_across_scale, c);
+    s[k] = to_float(c);
+    if (rc == GB_OK) rc = rg_setup(sigma, spacing[k], 1, normalize_across_scale, c);
+    dv[k] = to_float(c);
   }
   if (rc != GB_OK) {
     cudaFreeAsync(buf, st);
     return fail(GB_ERR_BAD_ARG, "sigma must be > 0");
   }
   const float inv[3] = {(float)(1.0 / spacing[0]), (float)(1.0 / spacing[1]), (float)(1.0 / spacing[2])};
+  RGMatrix m{{1, 0, 0, 0, 1, 0, 0, 0, 1}};
+  if (use_direction)
+    for (int k = 0; k < 9; ++k) m.m[k] = (float)direction[k];
   // x: A = Dx I, B = Sx I; y: C = Sy A, D = Dy B, E = Sy B;
-  // z: gx = Sz C / sx -> A, gy = Sz D / sy -> B, gz = Dz E / sz -> C
-  if (e == cudaSuccess) e = rg_pass(st, in, A, size, 0, dv[0], 1.f);
-  if (e == cudaSuccess) e = rg_pass(st, in, B, size, 0, s[0], 1.f);
-  if (e == cudaSuccess) e = rg_pass(st, A, C, size, 1, s[1], 1.f);
-  if (e == cudaSuccess) e = rg_pass(st, B, D, size, 1, dv[1], 1.f);
-  if (e == cudaSuccess) e = rg_pass(st, B, E, size, 1, s[1], 1.f);
-  if (e == cudaSuccess) e = rg_pass(st, C, A, size, 2, s[2], inv[0]);
-  if (e == cudaSuccess) e = rg_pass(st, D, B, size, 2, s[2], inv[1]);
-  if (e == cudaSuccess) e = rg_pass(st, E, C, size, 2, dv[2], inv[2]);
-  if (e == cudaSuccess) {
-    double m[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    if (use_direction) std::copy(direction, direction + 9, m);
-    k_pack_gradient<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(in, A, B, C, n, (float)m[0], (float)m[1],
-                                                                   (float)m[2], (float)m[3], (float)m[4],
-                                                                   (float)m[5], (float)m[6], (float)m[7],
-                                                                   (float)m[8], out4, out3);
-    e = cudaGetLastError();
+  // z: gx = Sz C / sx, gy = Sz D / sy, gz = Dz E / sz
+  const RGOut ox[2] = {{A, 1.f, dv[0]}, {B, 1.f, s[0]}};
+  const RGOut oy[3] = {{C, 1.f, s[1]}, {D, 1.f, dv[1]}, {E, 1.f, s[1]}};
+  e = rg_pass(st, in, size, 0, ox, 2);
+  if (e == cudaSuccess) e = rg_pass(st, A, size, 1, oy, 1);
+  if (e == cudaSuccess) e = rg_pass(st, B, size, 1, oy + 1, 2);
+  const size_t shared = sizeof(float) * rgz_array((int)size[2]) * (out4 ? 7 : 6);
+  if (shared <= kRGMaxShared) {
+    RGGradZ z;
+    memset(&z, 0, sizeof(z));
+    z.in[0] = C;
+    z.in[1] = D;
+    z.in[2] = E;
+    z.v = in;
+    for (int k = 0; k < 3; ++k) z.out[k] = RGOut{nullptr, inv[k], k < 2 ? s[2] : dv[2]};
+    z.m = m;
+    z.lines = size[0] * size[1];
+    z.step = z.lines;
+    z.ln = (int)size[2];
+    z.wide = n % 4 == 0 && z.lines % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0 ? 1 : 0;
+    z.out4 = out4;
+    z.out3 = out3;
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_rg_grad_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRGMaxShared);
+    if (e == cudaSuccess) {
+      k_rg_grad_z<<<(unsigned)((z.lines + kRGzLines - 1) / kRGzLines), 96, shared, st>>>(z);
+      e = cudaGetLastError();
+    }
+  } else {
+    const RGOut oz[3] = {{A, inv[0], s[2]}, {B, inv[1], s[2]}, {C, inv[2], dv[2]}};
+    const float* iz[3] = {C, D, E};  // C is read before it is written
+    for (int k = 0; k < 3; ++k)
+      if (e == cudaSuccess) e = rg_pass(st, iz[k], size, 2, oz + k, 1);
+    if (e == cudaSuccess) {
+      k_pack_gradient<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(in, A, B, C, n, m, out4, out3);
+      e = cudaGetLastError();
+    }
   }
   cudaFreeAsync(buf, st);
   if (e != cudaSuccess) return fail(GB_ERR_CUDA, std::string("gradient filter: ") + cudaGetErrorString(e));

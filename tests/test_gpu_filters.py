@@ -208,3 +208,26 @@ def test_gradient_filter_agrees_with_central_difference(degrees):
         if n1 > 0 and n2 > 0:
             total += (g @ truth) / (n1 * n2)
     assert total / 2.0 >= 0.96
+
+
+# tiles of 32 (z of the gradient: 16) lines and lines of both parities; lines too long for a
+# block's shared memory along each axis (above 907 and, for the gradient's z, 518 elements)
+@pytest.mark.parametrize("size", [(4, 4, 4), (5, 7, 9), (33, 31, 6), (64, 32, 40), (17, 6, 67), (1000, 5, 6), (6, 950, 5),
+                                  (5, 7, 601), (7, 4, 921)])
+def test_filters_match_oracle_at_tile_edges(size):
+    rng = np.random.default_rng(size[0] * 1000003 + size[1] * 1009 + size[2])
+    img = Image(rng.normal(0.0, 100.0, size=size[::-1]).astype(np.float32), spacing=(1.0, 1.25, 0.8),
+                direction=rotation(20))
+    f = SmoothingRecursiveGaussianImageFilter()
+    f.SetSigma(1.3)
+    f.SetInput(img)
+    f.Update()
+    want = O.smooth_recursive_gaussian(img.array, img.spacing, np.full(3, 1.3))
+    assert np.max(np.abs(f.GetOutput().array - want)) <= 2e-6 * np.max(np.abs(want))
+    g = GradientRecursiveGaussianImageFilter()
+    g.SetSigma(1.3)
+    g.SetNormalizeAcrossScale(True)
+    g.SetInput(img)
+    g.Update()
+    want = O.gradient_recursive_gaussian(img.array, img.spacing, img.direction, 1.3, True, True)
+    assert np.max(np.abs(g.GetOutput().array - want)) <= 2e-5 * np.max(np.abs(want))
