@@ -362,8 +362,8 @@ int gb_batch_run(gb_batch *b, int64_t max_iterations, int64_t *running);
  * the metric handle holds the final parameters, and the return value is the
  * registration's status (as gb_metric_optimize_regular_step returns it). */
 int gb_batch_result(gb_batch *b, int64_t slot, int *finished, gb_optimizer_report *report);
-/* Samples per block of the MeanSquares pass, Mattes pass 1 and Mattes pass 2
- * (default 8192 each); gb_batch_autotune picks them by timing the batch's
+/* Samples per block (at most) of the MeanSquares pass, Mattes pass 1 and Mattes pass 2
+ * (default 8192 each; small registrations are spread over more blocks); gb_batch_autotune picks them by timing the batch's
  * evaluations (no optimizer state changes) and leaves the fastest set. */
 int gb_batch_set_samples_per_block(gb_batch *b, const int64_t spb[3]);
 int gb_batch_get_samples_per_block(gb_batch *b, int64_t spb[3]);
