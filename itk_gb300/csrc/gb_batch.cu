@@ -6,8 +6,8 @@
 //   k_batch_clear    accumulators of every running registration
 //   k_batch_prepare  per-evaluation transform constants (22 FP64 entries each)
 //   k_batch_msq      MeanSquares value and derivative      } blocks of all
-//   k_batch_pass1    Mattes joint histogram, last block's   } registrations in
-//                    log(p / pm) table                      } one grid, each
+//   k_batch_pass1    Mattes joint histogram                 } registrations in
+//                                                           } one grid, each
 //   k_batch_pass2    Mattes value and derivative            } block one virtual
 //   k_batch_step     AdvanceOneStep (one block per registration)   block of one
 // captured once as a CUDA graph and relaunched per iteration.     registration
@@ -543,7 +543,7 @@ int rebuild_tables(gb_batch* b) {
     for (int v = 0; v < meta[(size_t)k].y; ++v) items.push_back(make_int4(kItP2, k, v, meta[(size_t)k].y));
   for (size_t k = 0; k < n; ++k) items.push_back(make_int4(kItStep, (int)k, 0, 0));
   b->per_iter = (unsigned)items.size();
-  b->smem1 = sizeof(unsigned long long) * (size_t)(maxbins * maxbins + maxbins) + sizeof(unsigned) * (size_t)maxbins;
+  b->smem1 = mattes_hist_bytes(maxbins);
   b->smem2 = mattes_pass2_smem(maxbins);
   if (maxbins > 0) {
     if (b->smem1 > 200 * 1024) return fail(GB_ERR_UNSUPPORTED, "histogram too large for shared memory (bins > 160)");

@@ -183,73 +183,74 @@ __global__ void __launch_bounds__(kBlock) k_msq_bspline(EvalArgs a) {
 // Dynamic shared memory of the B-spline Mattes pass 1: histogram, column sums,
 // fixed counts, then (16-byte aligned) the nodes.
 __host__ __device__ inline size_t mattes_bspline_node_offset(int B) {
-  return ((size_t)8 * (B * B + B) + 4 * (size_t)B + 15) / 16 * 16;
+  return (mattes_hist_bytes(B) + 15) / 16 * 16;
 }
 
 // Mattes pass 1, B-spline: as k_mattes_pass1_affine, caching (term, M^T g).
 template <int GRAD, bool SMEM>
 __global__ void __launch_bounds__(kBlock, SMEM ? 4 : 3) k_mattes_pass1_bspline(EvalArgs a) {
-  extern __shared__ unsigned long long smem_u64[];
+  extern __shared__ __align__(16) unsigned smem_hist[];
   const int B = a.bins;
-  unsigned long long* hist = smem_u64;
-  unsigned long long* cs = smem_u64 + B * B;
-  unsigned* fm = reinterpret_cast<unsigned*>(smem_u64 + B * B + B);
-  float4* nodes_sh = reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(smem_u64) + mattes_bspline_node_offset(B));
+  __shared__ unsigned long long warp_total[kBlock / 32];
+  const MattesHist h(smem_hist, warp_total, B);
+  float4* nodes_sh = reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(smem_hist) + mattes_bspline_node_offset(B));
   __shared__ EvalConsts K;
-  for (int k = threadIdx.x; k < B * B; k += blockDim.x) hist[k] = 0ull;
-  for (int k = threadIdx.x; k < B; k += blockDim.x) {
-    fm[k] = 0u;
-    cs[k] = 0ull;
-  }
+  mattes_hist_clear(h, B);
   griddep_wait();
   if (halted(a)) return;
   griddep_launch_dependents();
   load_consts(a.consts, K);
   const float4* nodes = stage_nodes<SMEM>(a, nodes_sh);
   __syncthreads();
-  unsigned nv = 0;
-  const int lane = threadIdx.x & 31;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  // 32-bit sample indices (a handle holds at most 2^31 - 1)
+  const unsigned n = (unsigned)a.n, stride = (unsigned)(gridDim.x * kBlock);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
+  unsigned base = (unsigned)(blockIdx.x * kBlock);  // the block's samples: base + thread
   // the next iteration's record and support travel while this one is evaluated
-  float4 s_next = base + lane < a.n ? __ldcs(a.samples + base + lane) : zero;
-  float4 su_next = base + lane < a.n ? __ldcs(a.sup + base + lane) : zero;
-  for (; base < a.n; base += stride) {
-    const int64_t i = base + lane;
-    const bool live = i < a.n;
-    const float4 s = s_next, su = su_next;
-    s_next = i + stride < a.n ? __ldcs(a.samples + i + stride) : zero;
-    su_next = i + stride < a.n ? __ldcs(a.sup + i + stride) : zero;
-    float m = 0.f;
-    float3 g = make_float3(0.f, 0.f, 0.f);
-    bool ok = false, has_jac = false;
-    if (live) {
-      const DFPos p = bspline_position(K, nodes, a, s, su, has_jac);
-      ok = eval_moving<GRAD>(a, p, a.with_derivative != 0 && has_jac, m, g);
-      ok = ok && !(m < a.mmin) && !(m > a.mmax);  // Mattes...Threader.hxx:238-245
-    }
-    const float term = fmaf(m - a.mmin, a.m_inv_bs, 2.f);
-    if (a.with_derivative && live) {
-      const float3 gm = has_jac ? grad_map(K, g) : make_float3(0.f, 0.f, 0.f);
-      __stcs(a.cache + i, ok ? make_float4(term, gm.x, gm.y, gm.z)
-                             : make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f));
-    }
-    int pdfm = 0;
-    unsigned q[4] = {0u, 0u, 0u, 0u};
-    const int fidx = __float_as_int(s.w);
-    if (ok) {
-      float t, w6[4];
-      parzen_window(term, B, pdfm, t);
-      parzen6(t, w6);
+  float4 s_next = base + threadIdx.x < n ? __ldcs(a.samples + base + threadIdx.x) : zero;
+  float4 su_next = base + threadIdx.x < n ? __ldcs(a.sup + base + threadIdx.x) : zero;
+  for (;;) {
+    int left = kHistSamples / kBlock;
+    for (; left > 0 && base < n; base += stride, --left) {
+      const unsigned i = base + threadIdx.x;
+      const bool live = i < n;
+      const float4 s = s_next, su = su_next;
+      s_next = i + stride < n ? __ldcs(a.samples + i + stride) : zero;
+      su_next = i + stride < n ? __ldcs(a.sup + i + stride) : zero;
+      float m = 0.f;
+      float3 g = make_float3(0.f, 0.f, 0.f);
+      bool ok = false, has_jac = false;
+      if (live) {
+        const DFPos p = bspline_position(K, nodes, a, s, su, has_jac);
+        ok = eval_moving<GRAD>(a, p, a.with_derivative != 0 && has_jac, m, g);
+        ok = ok && !(m < a.mmin) && !(m > a.mmax);  // Mattes...Threader.hxx:238-245
+      }
+      const float term = fmaf(m - a.mmin, a.m_inv_bs, 2.f);
+      if (a.with_derivative && live) {
+        const float3 gm = has_jac ? grad_map(K, g) : make_float3(0.f, 0.f, 0.f);
+        __stcs(a.cache + i, ok ? make_float4(term, gm.x, gm.y, gm.z)
+                               : make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f));
+      }
+      int pdfm = 0;
+      unsigned q[4] = {0u, 0u, 0u, 0u};
+      const int fidx = __float_as_int(s.w);
+      if (ok) {
+        float t, w6[4];
+        parzen_window(term, B, pdfm, t);
+        parzen6(t, w6);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) q[k] = (__float2uint_rn(w6[k] * kQScale) + 3u) / 6u;
+        for (int k = 0; k < 4; ++k) q[k] = (__float2uint_rn(w6[k] * kQScale) + 3u) / 6u;
+      }
+      hist_add_aggregated(ok, fidx * B + pdfm, fidx, q, h.bins, h.fm);
     }
-    hist_add_aggregated(ok, fidx * B + pdfm, fidx, q, hist, fm);
-    nv += ok ? 1u : 0u;
+    __syncthreads();
+    mattes_hist_flush(a, h, hw_grid());
+    if (base >= n) break;
+    __syncthreads();
+    for (int k = threadIdx.x; k < 2 * B * B; k += blockDim.x) h.bins[k] = 0u;
+    __syncthreads();
   }
-  // the derivative's table is formed by k_mattes_table, not by the last block
-  mattes_pass1_epilogue(a, nv, hist, cs, fm, hw_grid(), false);
+  mattes_pass1_epilogue(a, h);
 }
 
 // One block per chunk of same-cell samples (at most kChunkLen = blockDim).
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(kChunkLen) k_bspline_chunks(EvalArgs a) {
   const int B = a.bins;
   const int t = threadIdx.x;
   if (MATTES) {
-    mattes_value_groups<true>(a);  // the value's group partials (blocks b, b + G, ...) and their sum
+    mattes_value_groups(a);  // the value's group partials (blocks b, b + G, ...) and their sum
     for (int k = t; k < B * B; k += blockDim.x) pr_sh[k] = __ldcg(a.pratio + k);
   }
   // this thread's inputs of one chunk: the run, the sample's support, cache and fixed bin

@@ -104,9 +104,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_mattes_pass1_field(EvalArgs a) {
   mattes_pass1_affine_body<GRAD, TK>(a, hw_grid());
 }
 
-// Mattes pass 2 under a displacement field, after k_mattes_finalize: each
-// sample's block from its cached Parzen term and gradient and the log(p / pm)
-// table.  Dynamic shared memory: the bins^2 table.
+// Mattes pass 2 under a displacement field, after k_mattes_table: each sample's block from
+// its cached Parzen term and gradient and the log(p / pm) table; the value's FP64 groups by
+// the last warps of the first blocks (a kernel of their own before this one cost 10 us, the
+// table's takes 5).  Dynamic shared memory: the bins^2 table.
 template <int TK>
 __global__ void __launch_bounds__(kBlock) k_mattes_pass2_field(EvalArgs a) {
   extern __shared__ float pr[];
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(kBlock) k_mattes_pass2_field(EvalArgs a) {
     const unsigned long long N = __ldcg(a.acc_n);
     coef = N > 0 ? (float)(-1.0 / (a.m_bs * (double)N)) : 0.f;  // -nFactor, Mattes...v4.hxx:415
   }
+  mattes_value_groups<true>(a);
   __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride) {

@@ -31,13 +31,12 @@ constexpr int kMaxBlocks = 2048;          // grid cap of the evaluation kernels
 constexpr int kTicketMain = 0;            // grid_sums of the MeanSquares kernel: [0, 128]
 constexpr int kTicketFinalize = 160;      // last_block of the Mattes finalize
 constexpr int kTicketPass2 = 192;         // grid_sums of Mattes pass 2: [192, 320]
-constexpr int kTicketPass1 = 176;         // last_block of Mattes pass 1
 constexpr int kTicketValue = 340;         // the Mattes derivative pass's value groups done
 constexpr int kTicketCount = 352;
 constexpr int kPartPass2 = 4096;          // offset of pass-2 partials (finalize blocks use [0, 4096))
 constexpr int kPartValue = kPartPass2 - 1;  // the Mattes derivative pass's value (sum of the groups)
 constexpr size_t kGroupOffset = kPartPass2 + (size_t)kMaxBlocks * 16;  // per-group partials: 128 groups x 16
-constexpr size_t kMargOffset = kGroupOffset + 2048;     // [T, 1/T, derivative scale]
+constexpr size_t kMargOffset = kGroupOffset + 2048;     // per-evaluation FP64 scalars (EvalArgs::marg)
 constexpr size_t kScratchDoubles = kMargOffset + 8;
 constexpr int kFinalizeThreads = 32;
 constexpr float kQScale = 67108864.f;  // 2^26 fixed point of histogram weights
@@ -156,6 +155,7 @@ struct EvalArgs {
   double m_bs;
   // accumulators (cleared per evaluation)
   unsigned long long* acc_n;
+  unsigned long long* acc_t;    // Mattes: the joint histogram's total, 2^26 fixed point
   unsigned* tickets;            // [kTicketCount]
   unsigned long long* hist;     // bins*bins, 2^26 fixed point
   unsigned long long* fmarg;    // bins
@@ -163,7 +163,7 @@ struct EvalArgs {
   // scratch (overwritten per evaluation)
   double* part;                 // per-block partials
   double* grp;                  // per-group partials
-  double* marg;                 // [fixed-point total T, 1 / T]
+  double* marg;                 // [2]: Mattes, B-spline: the derivative scale; correlation: [2] to [5]
   float4* cache;
   float* pratio;
   double* pdf_out;
@@ -927,23 +927,52 @@ __device__ __forceinline__ void parzen_window(float term, int B, int& pdfm, floa
   t = term - (float)midx;
 }
 
-// Adds one sample's four Parzen weights into the block histogram.  Lanes with
-// the same (fixed bin, first moving bin) key are summed with one redux per
-// weight, and only the group leader issues the shared atomics.
-__device__ __forceinline__ void hist_add_aggregated(bool ok, int key, int fidx, const unsigned q[4],
-                                                    unsigned long long* hist, unsigned* fm) {
+// The block histogram holds a bin as two 32-bit words: its weights' low kHalfBits bits and
+// the bits above them, summed apart.  Shared memory adds 32-bit words in hardware; a
+// 64-bit add is a loop around a compare-and-swap.  A sample adds less than 2^13 to either
+// word, so a word would hold 2^19 of them; a block flushes after kHistSamples.
+constexpr int kHalfBits = 13;
+constexpr int kHistSamples = 1 << 14;
+__device__ __forceinline__ void hist_add_bin(unsigned* bin, unsigned q) {
+  atomicAdd(bin, q & ((1u << kHalfBits) - 1u));
+  atomicAdd(bin + 1, q >> kHalfBits);
+}
+__device__ __forceinline__ unsigned long long hist_bin(const unsigned* bin) {
+  return (unsigned long long)bin[0] + ((unsigned long long)bin[1] << kHalfBits);
+}
+
+// Adds one sample's four Parzen weights into the block histogram.  Where a warp's samples
+// fall on few (fixed bin, first moving bin) keys -- an image's background -- the lanes of a
+// key are summed with one redux per weight and one lane adds them: alone, those lanes
+// would queue on the same words.  Spread over more than kFewKeys keys, every lane adds its
+// own: the groups run one after another, about 20 instructions each.  Pass 1, us:
+//                     256^2x200 random   61x67x53   B-spline 192^2x160   field 192^2x160
+//   all grouped               77             19.5            44                 198
+//   all alone                106             13.3            44                 185
+//   grouped up to 4 keys      75             13.4            38                 182
+//   grouped up to 10          75             15.5            40                 198
+// (with the 64-bit words: all grouped 79, 19.5, 44, 207; all alone 298, 25.6, 93, 497).
+constexpr int kFewKeys = 4;
+__device__ __forceinline__ void hist_add_aggregated(bool ok, int key, int fidx, const unsigned q[4], unsigned* hist,
+                                                    unsigned* fm) {
   const unsigned okmask = __ballot_sync(0xffffffffu, ok);
   if (!ok) return;
   const unsigned peers = __match_any_sync(okmask, key);
   const int leader = __ffs(peers) - 1;
   const int lane = threadIdx.x & 31;
+  unsigned* bin = hist + 2 * key;
+  if (__popc(__ballot_sync(okmask, lane == leader)) > kFewKeys) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) hist_add_bin(bin + 2 * k, q[k]);
+    atomicAdd(&fm[fidx], 1u);
+    return;
+  }
   unsigned s[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) s[k] = __reduce_add_sync(peers, q[k]);
   if (lane == leader) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (s[k]) atomicAdd(&hist[key + k], (unsigned long long)s[k]);
+    for (int k = 0; k < 4; ++k) hist_add_bin(bin + 2 * k, s[k]);
     atomicAdd(&fm[fidx], (unsigned)__popc(peers));
   }
 }
@@ -968,65 +997,79 @@ __device__ __forceinline__ PratioThresholds pratio_thresholds(double T, unsigned
   return t;
 }
 
-template <bool STREAMERS>
-static __device__ __noinline__ void mattes_pratio_build(const EvalArgs& a, double T, float* dst, float* colf,
-                                                        unsigned* fmask);
-
 // u64 count -> float from its two 32-bit halves, FP32 arithmetic only (two roundings,
 // relative error below 2^-23)
 __device__ __forceinline__ float u64_to_float(unsigned long long v) {
   return fmaf(__uint2float_rn((unsigned)(v >> 32)), 4294967296.f, __uint2float_rn((unsigned)v));
 }
 
-// End of Mattes pass 1 (any transform): flush the block histogram, marginals and
-// count; the last block forms the fixed-point total T and, with `table`, the
-// derivative's log(p / pm) table in global memory (the affine derivative pass
-// builds the table itself, in shared memory).
-__device__ __forceinline__ void mattes_pass1_epilogue(const EvalArgs& a, unsigned nv, unsigned long long* hist,
-                                                      unsigned long long* cs, unsigned* fm, VGrid vg = hw_grid(),
-                                                      bool table = true) {
+// Shared memory of Mattes pass 1: the joint histogram, the column sums (two words each:
+// the low kColBits bits of every bin's count, and those above) and the fixed-bin counts.
+constexpr int kColBits = 20;
+struct MattesHist {
+  unsigned *bins, *cols, *fm;
+  unsigned long long* warp_total;  // per warp: the weights it has flushed
+  __device__ __forceinline__ MattesHist(unsigned* shared, unsigned long long* warp_total, int B)
+      : bins(shared), cols(shared + 2 * B * B), fm(shared + 2 * B * B + 2 * B), warp_total(warp_total) {}
+};
+__host__ __device__ inline size_t mattes_hist_bytes(int B) { return 8 * ((size_t)B * B + B) + 4 * (size_t)B; }
+
+__device__ __forceinline__ void mattes_hist_clear(const MattesHist& h, int B) {
+  for (int k = threadIdx.x; k < 2 * B * B + 3 * B; k += blockDim.x) h.bins[k] = 0u;
+  if (threadIdx.x < kBlock / 32) h.warp_total[threadIdx.x] = 0ull;
+}
+
+// Flushes the block histogram's nonzero bins; the block's column sums ride along in shared
+// memory.  Each block starts at its own bin, so the blocks finishing together do not queue
+// on the same global addresses.  The caller has synchronized.
+__device__ __forceinline__ void mattes_hist_flush(const EvalArgs& a, const MattesHist& h, VGrid vg) {
   const int B = a.bins;
   const int BB = B * B;
-  __syncthreads();
-  // flush the nonzero bins; the block's column sums ride along as shared atomics.  Each
-  // block starts at its own bin, so the blocks finishing together do not queue on the
-  // same global addresses.
   const int rot = (int)(((long long)vg.b * 97) % BB);
+  unsigned long long t = 0ull;
   for (int k0 = threadIdx.x; k0 < BB; k0 += blockDim.x) {
     const int k = k0 + rot < BB ? k0 + rot : k0 + rot - BB;
-    const unsigned long long h = hist[k];
-    if (h) {
-      atomicAdd(&a.hist[k], h);
-      atomicAdd(&cs[k % B], h);
+    const unsigned long long v = hist_bin(h.bins + 2 * k);
+    if (v) {
+      atomicAdd(&a.hist[k], v);
+      const int m = k % B;
+      atomicAdd(h.cols + 2 * m, (unsigned)v & ((1u << kColBits) - 1u));
+      atomicAdd(h.cols + 2 * m + 1, (unsigned)(v >> kColBits));
+      t += v;
     }
   }
-  __syncthreads();
-  for (int k = threadIdx.x; k < B; k += blockDim.x) {
-    const unsigned c = fm[k];
-    if (c) atomicAdd(&a.fmarg[k], (unsigned long long)c);
-    if (cs[k]) atomicAdd(&a.colsum[k], cs[k]);
-  }
-  block_count(nv, a.acc_n);
-  if (!last_block(a.tickets + kTicketPass1, vg)) return;
-  // Last block: the fixed-point total T of the joint histogram (the value's
-  // normalization, JointPDFSum).  It is on the critical path, so it does no FP64
-  // transcendental work.
-  __shared__ unsigned long long tot_sh;
-  if (threadIdx.x == 0) tot_sh = 0ull;
-  __syncthreads();
-  unsigned long long t = 0ull;
-  for (int k = threadIdx.x; k < B; k += blockDim.x) t += __ldcg(&a.colsum[k]);
-  // one shared atomic per warp: a block's worth of same-address atomics would serialize
+#pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if ((threadIdx.x & 31) == 0 && t) atomicAdd(&tot_sh, t);
-  __syncthreads();
-  const double T = (double)tot_sh;
-  if (threadIdx.x == 0) {
-    a.marg[0] = T;                         // fixed-point total
-    a.marg[1] = T > 0.0 ? 1.0 / T : 0.0;   // normalization factor (of the fixed-point histogram)
-  }
-  if (table) mattes_pratio_build<false>(a, T, a.pratio, reinterpret_cast<float*>(cs), fm);
+  if ((threadIdx.x & 31) == 0) h.warp_total[threadIdx.x >> 5] += t;
 }
+
+// End of Mattes pass 1 (any transform), after the last flush: the marginals, the valid
+// count (every valid sample counts in one fixed bin) and the histogram's total (the value's
+// normalization, JointPDFSum).  Each is one integer atomic per block and entry, so the
+// following kernels read them as they stand: a last block forming the total cost a fence,
+// a ticket and a round of loads at the end of the pass.
+__device__ __forceinline__ void mattes_pass1_epilogue(const EvalArgs& a, const MattesHist& h) {
+  __syncthreads();
+  unsigned n = 0u;
+  for (int k = threadIdx.x; k < a.bins; k += blockDim.x) {
+    const unsigned f = h.fm[k];
+    if (f) atomicAdd(&a.fmarg[k], (unsigned long long)f);
+    n += f;
+    const unsigned long long c =
+        (unsigned long long)h.cols[2 * k] + ((unsigned long long)h.cols[2 * k + 1] << kColBits);
+    if (c) atomicAdd(&a.colsum[k], c);
+  }
+  n = warp_sum_u(n);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(a.acc_n, (unsigned long long)n);
+  if (threadIdx.x == blockDim.x - 1) {
+    unsigned long long t = 0ull;
+    for (int w = 0; w < kBlock / 32; ++w) t += h.warp_total[w];
+    if (t) atomicAdd(a.acc_t, t);
+  }
+}
+
+// The total of the finished joint histogram.
+__device__ __forceinline__ double mattes_total(const EvalArgs& a) { return (double)__ldcg(a.acc_t); }
 
 // The derivative's FP32 table log(p / pm) = log(h / colsum) (pRatio,
 // Mattes...v4.hxx:446-457), 0 where p, pm or pf is not above DBL_EPSILON:
@@ -1083,7 +1126,7 @@ static __device__ __noinline__ void mattes_pratio_build(const EvalArgs& a, doubl
 __device__ __forceinline__ int mattes_status(const EvalArgs& a) {
   const unsigned long long N = __ldcg(a.acc_n);
   if (N == 0) return GB_ERR_NO_VALID_POINTS;
-  return __ldcg(&a.marg[0]) * kQInv >= DBL_EPSILON ? GB_OK : GB_ERR_JOINT_PDF_SUM_ZERO;
+  return mattes_total(a) * kQInv >= DBL_EPSILON ? GB_OK : GB_ERR_JOINT_PDF_SUM_ZERO;
 }
 
 // One warp, bins [32 g, 32 g + 32) of the joint histogram: the FP64 terms
@@ -1095,8 +1138,8 @@ __device__ __forceinline__ int mattes_status(const EvalArgs& a) {
 // and GetValueAndDerivative give the same bits.
 __device__ __forceinline__ double mattes_group_partial(const EvalArgs& a, int g, int lane) {
   const int B = a.bins;
-  const double T = __ldcg(&a.marg[0]);
-  const double invT = __ldcg(&a.marg[1]);
+  const double T = mattes_total(a);
+  const double invT = T > 0.0 ? 1.0 / T : 0.0;
   const bool bad = (__ldcg(a.acc_n) == 0) || !(T * kQInv >= DBL_EPSILON);  // JointPDFSum
   const int bin = g * 32 + lane;
   double part = 0.0;
@@ -1139,11 +1182,12 @@ __device__ __forceinline__ double mattes_value_sum(const double* part, int ngrou
   return warp_sum_d(s);
 }
 
-// Group partials computed by the last warp of blocks b, b + gridDim.x, ... (all blocks participate).
 // After a warp has written the partial of one group: the warp that completes the last
 // group sums all of them into part[kPartValue] (the same order as mattes_value_sum at
 // the end of the pass), so the derivative pass's last block only reads the value.
 // It writes before its block takes its cross-block ticket, so the last block sees it.
+// WRITE: it writes the value, the count and the status itself (a pass without a last block).
+template <bool WRITE = false>
 __device__ __forceinline__ void mattes_value_group_done(const EvalArgs& a, int ng) {
   const int lane = threadIdx.x & 31;
   __threadfence();
@@ -1153,12 +1197,20 @@ __device__ __forceinline__ void mattes_value_group_done(const EvalArgs& a, int n
   if (t != (unsigned)(ng - 1)) return;
   __threadfence();
   const double s = mattes_value_sum(a.part, ng, lane);
-  if (lane == 0) a.part[kPartValue] = s;
+  if (lane != 0) return;
+  if (WRITE) {
+    const int st = mattes_status(a);
+    *a.status = st;
+    a.out[0] = st == GB_OK ? -1.0 * s : 0.0;  // metrics minimize: value = -MI
+    a.out[1] = (double)__ldcg(a.acc_n);
+  } else {
+    a.part[kPartValue] = s;
+  }
 }
 
-// SUM: the derivative pass's form, with the value summed by the warp completing the
-// last group (mattes_value_group_done).
-template <bool SUM = false>
+// The value's group partials, computed by the last warp of blocks b, b + gridDim.x, ...
+// (all blocks take part), and their sum.
+template <bool WRITE = false>
 __device__ __forceinline__ void mattes_value_groups(const EvalArgs& a, VGrid vg = hw_grid()) {
   if ((int)(threadIdx.x >> 5) != (int)(blockDim.x >> 5) - 1) return;
   const int lane = threadIdx.x & 31;
@@ -1166,16 +1218,16 @@ __device__ __forceinline__ void mattes_value_groups(const EvalArgs& a, VGrid vg 
   for (int g = vg.b; g < ng; g += vg.n) {
     const double s = mattes_group_partial(a, g, lane);
     if (lane == 0) a.part[g] = s;
-    if (SUM) mattes_value_group_done(a, ng);
+    mattes_value_group_done<WRITE>(a, ng);
   }
 }
 
 // One sample of Mattes pass 1 (affine and displacement-field maps): position, moving
 // value and gradient, range reject, cache write, Parzen weights into the block
-// histogram `hist` (warp-aggregated), valid count.  Called by all 32 lanes of a warp.
+// histogram.  Called by all 32 lanes of a warp.
 template <int GRAD, int TK>
 __device__ __forceinline__ void mattes_pass1_sample(const EvalArgs& a, const EvalConsts& K, const float4& s, int64_t i,
-                                                    bool live, unsigned long long* hist, unsigned* fm, unsigned& nv) {
+                                                    bool live, const MattesHist& h) {
   const int B = a.bins;
   float m = 0.f;
   float3 g = make_float3(0.f, 0.f, 0.f);
@@ -1202,44 +1254,42 @@ __device__ __forceinline__ void mattes_pass1_sample(const EvalArgs& a, const Eva
 #pragma unroll
     for (int k = 0; k < 4; ++k) q[k] = (__float2uint_rn(w6[k] * kQScale) + 3u) / 6u;  // unbiased 1/6
   }
-  hist_add_aggregated(ok, fidx * B + pdfm, fidx, q, hist, fm);
-  nv += ok ? 1u : 0u;
+  hist_add_aggregated(ok, fidx * B + pdfm, fidx, q, h.bins, h.fm);
 }
 
 template <int GRAD, int TK = kMapAffine>
 __device__ __forceinline__ void mattes_pass1_affine_body(const EvalArgs& a, VGrid vg) {
-  extern __shared__ unsigned long long smem_u64[];
-  const int B = a.bins;
-  unsigned long long* hist = smem_u64;
-  unsigned long long* cs = smem_u64 + B * B;
-  unsigned* fm = reinterpret_cast<unsigned*>(smem_u64 + B * B + B);
+  extern __shared__ unsigned smem_hist[];
   __shared__ EvalConsts K;
-  for (int k = threadIdx.x; k < B * B; k += blockDim.x) hist[k] = 0ull;
-  for (int k = threadIdx.x; k < B; k += blockDim.x) {
-    fm[k] = 0u;
-    cs[k] = 0ull;
-  }
+  __shared__ unsigned long long warp_total[kBlock / 32];
+  const MattesHist h(smem_hist, warp_total, a.bins);
+  mattes_hist_clear(h, a.bins);
   griddep_wait();
   if (halted(a)) return;
   griddep_launch_dependents();
   load_consts(a.consts, K);
   __syncthreads();
-  unsigned nv = 0;
-  const int lane = threadIdx.x & 31;
-  const int64_t stride = (int64_t)vg.n * blockDim.x;
-  // the affine derivative pass builds the log(p / pm) table itself
-  constexpr bool kOwnTable = TK == kMapAffine;
-  int64_t base = (int64_t)vg.b * blockDim.x + (threadIdx.x & ~31);
-  float4 s_next = base + lane < a.n ? __ldcs(a.samples + base + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-  for (; base < a.n; base += stride) {
-    const int64_t i = base + lane;
-    const bool live = i < a.n;
-    const float4 s = s_next;
-    // prefetch the next record so its latency overlaps this iteration's gathers
-    s_next = i + stride < a.n ? __ldcs(a.samples + i + stride) : make_float4(0.f, 0.f, 0.f, 0.f);
-    mattes_pass1_sample<GRAD, TK>(a, K, s, i, live, hist, fm, nv);
+  // 32-bit sample indices (a handle holds at most 2^31 - 1)
+  const unsigned n = (unsigned)a.n, stride = (unsigned)(vg.n * kBlock);
+  unsigned base = (unsigned)(vg.b * kBlock);  // the block's samples: base + thread
+  float4 s_next = base + threadIdx.x < n ? __ldcs(a.samples + base + threadIdx.x) : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (;;) {
+    int left = kHistSamples / kBlock;
+    for (; left > 0 && base < n; base += stride, --left) {
+      const unsigned i = base + threadIdx.x;
+      const float4 s = s_next;
+      // prefetch the next record so its latency overlaps this iteration's gathers
+      s_next = i + stride < n ? __ldcs(a.samples + i + stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+      mattes_pass1_sample<GRAD, TK>(a, K, s, i, i < n, h);
+    }
+    __syncthreads();
+    mattes_hist_flush(a, h, vg);
+    if (base >= n) break;
+    __syncthreads();
+    for (int k = threadIdx.x; k < 2 * a.bins * a.bins; k += blockDim.x) h.bins[k] = 0u;
+    __syncthreads();
   }
-  mattes_pass1_epilogue(a, nv, hist, cs, fm, vg, !kOwnTable);
+  mattes_pass1_epilogue(a, h);
 }
 
 template <int GRAD>
@@ -1250,7 +1300,7 @@ __global__ void __launch_bounds__(kBlock, GRAD == kGradImage ? 5 : 4) k_mattes_p
 #ifndef GB_KERNELS_HELPERS_ONLY
 // The derivative's log(p / pm) table in global memory, one entry per thread (the
 // same arithmetic as mattes_pratio_build), for the derivative kernels that read it
-// from global memory (B-spline chunk sums).  A few blocks launched after pass 1,
+// from global memory (B-spline chunk sums, displacement fields).  A few blocks launched after pass 1,
 // instead of pass 1's last block forming all bins^2 entries alone on one SM.
 __global__ void __launch_bounds__(kBlock) k_mattes_table(EvalArgs a) {
   griddep_wait();
@@ -1259,7 +1309,7 @@ __global__ void __launch_bounds__(kBlock) k_mattes_table(EvalArgs a) {
   const int B = a.bins;
   __shared__ PratioThresholds th_s;
   if (threadIdx.x == 0) {
-    const double T = __ldcg(&a.marg[0]);
+    const double T = mattes_total(a);
     const unsigned long long N = __ldcg(a.acc_n);
     th_s = pratio_thresholds(T, N);  // FP64: once per block
     // the derivative scale for the parameter gather: nFactor = -1 / (MovingImageBinSize
@@ -1282,7 +1332,7 @@ __global__ void __launch_bounds__(kBlock) k_mattes_table(EvalArgs a) {
 // Mattes value without the derivative: one warp per group of 32 joint-histogram
 // bins (mattes_group_partial), the last block adds the group partials.  With the
 // derivative the same groups are formed by spare warps of the derivative pass
-// (k_mattes_pass2_affine, k_bspline_chunks) and summed at its end.
+// (k_mattes_pass2_affine, k_bspline_chunks, k_mattes_pass2_field) and summed at its end.
 __global__ void __launch_bounds__(kFinalizeThreads) k_mattes_finalize(EvalArgs a) {
   griddep_wait();
   if (halted(a)) return;
@@ -1439,7 +1489,7 @@ __device__ __forceinline__ void mattes_pass2_affine_body(const EvalArgs& a, VGri
   constexpr int kConstWords = (int)(sizeof(EvalConsts) / 4);
   const int cw = (int)threadIdx.x;
   const float cword = cw < kConstWords ? __ldcg(reinterpret_cast<const float*>(a.consts) + cw) : 0.f;
-  const double T = streamer ? __ldcg(&a.marg[0]) : 0.0;
+  const double T = streamer ? mattes_total(a) : 0.0;
   const unsigned long long N = streamer ? __ldcg(a.acc_n) : 0ull;
   // nFactor = -1 / (MovingImageBinSize * N), Mattes...Threader.hxx:446-457: formed now,
   // off the last block's tail (FP64 division)
@@ -1462,7 +1512,7 @@ __device__ __forceinline__ void mattes_pass2_affine_body(const EvalArgs& a, VGri
   if (!GROUP_WARP) {
     if (threadIdx.x == 0) nfac_s = -1.0 / (a.m_bs * (double)N);
     mattes_pratio_build<false>(a, T, pr, colf, fmask);
-    mattes_value_groups<true>(a, vg);  // the value's FP64 group partials and sum, last warp
+    mattes_value_groups(a, vg);  // the value's FP64 group partials and sum, last warp
     __syncthreads();
   } else if (streamer) {
     if (threadIdx.x == 0) nfac_s = -1.0 / (a.m_bs * (double)N);

@@ -550,11 +550,13 @@ extern "C" int gb_metric_get_number_of_parameters(gb_metric* m, int64_t* nparams
 // Initialize
 
 // Accumulators cleared before every evaluation:
-// acc_n u64 | tickets kTicketCount u32 | hist B*B u64 | fmarg B u64 | colsum B u64 | 16 bytes
+// acc_n u64 | tickets kTicketCount u32 | acc_t u64 | hist B*B u64 | fmarg B u64 | colsum B u64 | 16 bytes
 // The histogram starts at a 16-byte boundary and the padding covers the Mattes
 // derivative pass's bulk copy of hist..colsum rounded up to 16 bytes.
 static size_t acc_offset_tickets() { return 8; }
-static size_t acc_offset_hist() { return (8 + sizeof(unsigned) * kTicketCount + 15) / 16 * 16; }
+static size_t acc_offset_total() { return 8 + sizeof(unsigned) * kTicketCount; }
+static size_t acc_offset_hist() { return (acc_offset_total() + 8 + 15) / 16 * 16; }
+static_assert(kTicketCount % 2 == 0, "the total is an aligned 64-bit word");
 static size_t acc_offset_fmarg(int64_t B) { return acc_offset_hist() + 8 * (size_t)(B * B); }
 static size_t acc_offset_colsum(int64_t B) { return acc_offset_fmarg(B) + 8 * (size_t)B; }
 static size_t acc_layout_bytes(const gb_metric* m) {
@@ -1016,6 +1018,7 @@ static void fill_eval_args(gb_metric* m, EvalArgs& a, const double* d_params, do
   a.m_inv_bs = (float)(1.0 / m->mstate[5]);
   unsigned char* base = m->d_acc.p;
   a.acc_n = reinterpret_cast<unsigned long long*>(base);
+  a.acc_t = reinterpret_cast<unsigned long long*>(base + acc_offset_total());
   a.tickets = reinterpret_cast<unsigned*>(base + acc_offset_tickets());
   a.acc = reinterpret_cast<uint4*>(base);
   a.acc_words = (int)(m->acc_bytes / 16);
@@ -1193,8 +1196,8 @@ static int enqueue_eval_bspline(gb_metric* m, const EvalArgs& a, bool cd, bool d
   return GB_OK;
 }
 
-// Displacement-field evaluation: MeanSquares in one pass; Mattes pass 1, the
-// value, then the per-sample derivative blocks.  The derivative field is
+// Displacement-field evaluation: MeanSquares in one pass; Mattes pass 1, the log(p / pm)
+// table, then the per-sample derivative blocks and the value.  The derivative field is
 // cleared first unless every virtual voxel holds a sample (each then stores its
 // own block, zeros when invalid).
 static int enqueue_eval_field(gb_metric* m, const EvalArgs& a, bool cd, bool deriv) {
@@ -1212,7 +1215,7 @@ static int enqueue_eval_field(gb_metric* m, const EvalArgs& a, bool cd, bool der
     return GB_OK;
   }
   const int B = (int)m->bins;
-  const size_t sh1 = sizeof(unsigned long long) * (B * B + B) + sizeof(unsigned) * B;
+  const size_t sh1 = mattes_hist_bytes(B);
   if (sh1 > 200 * 1024) return fail(GB_ERR_UNSUPPORTED, "histogram too large for shared memory (bins > 160)");
   cudaError_t e;
   if (pts) e = cd ? launch_wave(m, k_mattes_pass1_field<kGradCentralDifference, kMapFieldPoints>, sh1, a)
@@ -1221,9 +1224,12 @@ static int enqueue_eval_field(gb_metric* m, const EvalArgs& a, bool cd, bool der
               : launch_wave(m, k_mattes_pass1_field<kGradImage, kMapFieldDense>, sh1, a);
   GB_CUDA(e);
   m->mark();
-  GB_CUDA(launch_chain(m, k_mattes_finalize, (unsigned)mattes_groups(B), kFinalizeThreads, 0, a));
-  m->mark();
-  if (deriv) {
+  if (!deriv) {  // with the derivative the value is formed in pass 2
+    GB_CUDA(launch_chain(m, k_mattes_finalize, (unsigned)mattes_groups(B), kFinalizeThreads, 0, a));
+    m->mark();
+  } else {
+    GB_CUDA(launch_chain(m, k_mattes_table, (unsigned)((B * B + kBlock - 1) / kBlock), kBlock, 0, a));
+    m->mark();
     const size_t sh2 = sizeof(float) * B * B;
     GB_CUDA(pts ? launch_wave(m, k_mattes_pass2_field<kMapFieldPoints>, sh2, a)
                 : launch_wave(m, k_mattes_pass2_field<kMapFieldDense>, sh2, a));
@@ -1409,7 +1415,7 @@ int gb::enqueue_eval(gb_metric* m, const double* d_params, double* d_out, bool d
   }
   // Mattes: pass 1, finalize, pass 2
   const int B = (int)m->bins;
-  const size_t sh1 = sizeof(unsigned long long) * (B * B + B) + sizeof(unsigned) * B;
+  const size_t sh1 = mattes_hist_bytes(B);
   if (sh1 > 200 * 1024) return fail(GB_ERR_UNSUPPORTED, "histogram too large for shared memory (bins > 160)");
   GB_CUDA(cd ? launch_wave(m, k_mattes_pass1_affine<kGradCentralDifference>, sh1, a)
              : launch_wave(m, k_mattes_pass1_affine<kGradImage>, sh1, a));

@@ -12,7 +12,7 @@ import pytest
 
 from cases import mattes_2d_case, mattes_2d_sample_points, perturbed, run_oracle, small_pair
 from conftest import MATTES_VALUE_ATOL, assert_deriv_close, assert_value_close
-from itk_gb300 import (AffineTransform, ExceptionObject, MattesMutualInformationImageToImageMetricv4,
+from itk_gb300 import (AffineTransform, ExceptionObject, Image, MattesMutualInformationImageToImageMetricv4,
                        MeanSquaresImageToImageMetricv4, data)
 from itk_gb300 import _capi
 
@@ -244,3 +244,33 @@ def test_floating_point_correction(resolution):
     assert_deriv_close(out[1][1], rd)
     if resolution == 10.0:
         assert np.max(np.abs(out[1][1] - out[0][1])) > 1e-3 / nv
+
+
+@pytest.mark.parametrize("levels", [2, 3, 6, 1000])
+@pytest.mark.parametrize("n", [31, 4099])
+def test_mattes_histogram_with_few_and_many_keys(levels, n):
+    """Samples of a warp in one, a few (summed together) and many (added one by one) joint bins."""
+    rng = np.random.default_rng(levels)
+    size = (24, 20, 18)
+    fixed = Image(rng.integers(0, levels, size=size[::-1]).astype(np.float32))
+    moving = Image(rng.integers(0, levels, size=size[::-1]).astype(np.float32))
+    T = AffineTransform()
+    T.SetTranslation((0.25, -0.5, 0.0))
+    pts = rng.uniform(0.0, 17.0, size=(n, 3)).astype(np.float32)
+    pts[: n // 2] = np.round(pts[: n // 2])  # half of them on voxels: exactly quantized fixed values
+    grad = data.gradient_image(moving)
+    m = MattesMutualInformationImageToImageMetricv4()
+    m.SetNumberOfHistogramBins(20)
+    m.SetFixedImage(fixed)
+    m.SetMovingImage(moving)
+    m.SetMovingTransform(T)
+    m.SetMovingImageGradientImage(grad)
+    m.SetVirtualSampledPointSet(pts)
+    m.SetUseSampledPointSet(True)
+    m.Initialize()
+    v, d = m.GetValueAndDerivative()
+    r = run_oracle("mattes", fixed, moving, T, gradient=grad, points=pts, bins=20)
+    assert m.GetNumberOfValidPoints() == r["nvalid"]
+    assert_value_close(v, r["value"], atol=MATTES_VALUE_ATOL)
+    assert_deriv_close(d, r["derivative"])
+    assert m.GetValue() == v

@@ -269,3 +269,24 @@ def test_first_iteration_matches_oracle(pairs):
         assert_value_close(o.GetValue(), v, atol=MATTES_VALUE_ATOL if kind == "mattes" else 0.0)
         d_batch = (U.GetParameters() - p0) * SCALES * (o.GetGradientMagnitude() / lr)
         assert_deriv_close(d_batch, d)
+
+
+def test_pass1_flushes_a_full_block_histogram():
+    """1.4 M dense samples in 80 blocks: each block flushes its histogram once on the way
+    (every 16384 samples).  The joint PDF is of integer counts: the same bits as the
+    single-registration loop's, whose blocks do not reach the limit."""
+    pair = small_pair((112, 112, 112), config=1, multimodal=True)
+    got = []
+    for batched in (True, False):
+        U, o = make([pair], 0, "mattes", iters=1)
+        if batched:
+            b = RegistrationBatch()
+            b.SetSamplesPerBlock(32768, 32768, 32768)
+            b.Add(o)
+            assert b.Run() == 0
+        else:
+            o.StartOptimization()
+        got.append((o.GetMetric().GetJointPDF(), o.GetValue(), U.GetParameters()))
+    assert np.array_equal(got[0][0], got[1][0])
+    assert got[0][1] == got[1][1]
+    assert np.max(np.abs(got[0][2] - got[1][2])) <= 1e-5
