@@ -115,11 +115,9 @@ struct CIdx {
 // (Core/ImageFunction/include/itkImageFunction.h:157-169).  With b the
 // round-half-up index, cidx >= -0.5 <=> b >= 0 and cidx < n - 0.5 <=> b <= n - 1.
 __device__ __forceinline__ bool ci_inside(const CIdx& c, int nx, int ny, int nz) {
-  const int n[3] = {nx, ny, nz};
-  bool in = true;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) in = in && (c.f[k] == c.f[k]) && c.b[k] >= 0 && c.b[k] <= n[k] - 1;
-  return in;
+  const float any = __fadd_rn(__fadd_rn(c.f[0], c.f[1]), c.f[2]);  // NaN if one is (|f| <= 1/2 otherwise)
+  return any == any && (unsigned)c.b[0] < (unsigned)nx && (unsigned)c.b[1] < (unsigned)ny &&
+         (unsigned)c.b[2] < (unsigned)nz;
 }
 
 // Corner indices and weights of LinearInterpolateImageFunction's 3-D path
@@ -150,9 +148,60 @@ __device__ __forceinline__ Stencil make_stencil(const CIdx& c, int nx, int ny, i
 
 __device__ __forceinline__ float lerp(float a, float b, float t) { return fmaf(b - a, t, a); }
 
-__device__ __forceinline__ float4 lerp4(float4 a, float4 b, float t) {
-  return make_float4(lerp(a.x, b.x, t), lerp(a.y, b.y, t), lerp(a.z, b.z, t), lerp(a.w, b.w, t));
+// Two FP32 values in a register pair, and one instruction on both (each rounded as its
+// scalar form, so results do not depend on which form computed them).  The FP32 units take
+// two cycles for a pair, but the warp issues one instruction instead of two: the per-sample
+// loops are bound by issue (430 to 870 instructions a sample at the start, a third to half
+// of them FP32), and the slots go to their integer and memory instructions.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
+__device__ __forceinline__ f32x2 pair(float a) { return pair(a, a); }
+__device__ __forceinline__ void unpair(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 lerp2(f32x2 a, f32x2 b, f32x2 t) { return fma2(sub2(b, a), t, a); }
+// lerp of four values held as two pairs
+__device__ __forceinline__ ulonglong2 lerp4(ulonglong2 a, ulonglong2 b, f32x2 t) {
+  return make_ulonglong2(lerp2(a.x, b.x, t), lerp2(a.y, b.y, t));
+}
+
+// KahanF on a pair of sums.
+struct KahanF2 {
+  f32x2 s, c;
+  __device__ __forceinline__ void zero() { s = c = 0ull; }
+  __device__ __forceinline__ void add(f32x2 x) {
+    const f32x2 y = sub2(x, c);
+    const f32x2 t = add2(s, y);
+    c = sub2(sub2(t, s), y);
+    s = t;
+  }
+  __device__ __forceinline__ void split(KahanF& a, KahanF& b) const {
+    unpair(s, a.s, b.s);
+    unpair(c, a.c, b.c);
+  }
+};
 
 // Trilinear gather of the packed (value, gx, gy, gz) moving image.
 __device__ __forceinline__ float4 gather4(const float4* __restrict__ img, const Stencil& s, int nx, int ny) {
@@ -160,14 +209,20 @@ __device__ __forceinline__ float4 gather4(const float4* __restrict__ img, const 
   const unsigned sy = (unsigned)nx, sz = (unsigned)nx * (unsigned)ny;
   const unsigned r00 = s.z0 * sz + s.y0 * sy, r10 = s.z0 * sz + s.y1 * sy;
   const unsigned r01 = s.z1 * sz + s.y0 * sy, r11 = s.z1 * sz + s.y1 * sy;
-  const float4 v000 = __ldg(img + r00 + s.x0), v100 = __ldg(img + r00 + s.x1);
-  const float4 v010 = __ldg(img + r10 + s.x0), v110 = __ldg(img + r10 + s.x1);
-  const float4 v001 = __ldg(img + r01 + s.x0), v101 = __ldg(img + r01 + s.x1);
-  const float4 v011 = __ldg(img + r11 + s.x0), v111 = __ldg(img + r11 + s.x1);
-  const float4 x00 = lerp4(v000, v100, s.dx), x10 = lerp4(v010, v110, s.dx);
-  const float4 x01 = lerp4(v001, v101, s.dx), x11 = lerp4(v011, v111, s.dx);
-  const float4 xx0 = lerp4(x00, x10, s.dy), xx1 = lerp4(x01, x11, s.dy);
-  return lerp4(xx0, xx1, s.dz);
+  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(img);  // (value, gx), (gy, gz)
+  const ulonglong2 v000 = __ldg(q + r00 + s.x0), v100 = __ldg(q + r00 + s.x1);
+  const ulonglong2 v010 = __ldg(q + r10 + s.x0), v110 = __ldg(q + r10 + s.x1);
+  const ulonglong2 v001 = __ldg(q + r01 + s.x0), v101 = __ldg(q + r01 + s.x1);
+  const ulonglong2 v011 = __ldg(q + r11 + s.x0), v111 = __ldg(q + r11 + s.x1);
+  const f32x2 dx = pair(s.dx), dy = pair(s.dy), dz = pair(s.dz);
+  const ulonglong2 x00 = lerp4(v000, v100, dx), x10 = lerp4(v010, v110, dx);
+  const ulonglong2 x01 = lerp4(v001, v101, dx), x11 = lerp4(v011, v111, dx);
+  const ulonglong2 xx0 = lerp4(x00, x10, dy), xx1 = lerp4(x01, x11, dy);
+  const ulonglong2 r = lerp4(xx0, xx1, dz);
+  float4 o;
+  unpair(r.x, o.x, o.y);
+  unpair(r.y, o.z, o.w);
+  return o;
 }
 
 // Trilinear gather of a scalar image.
@@ -200,60 +255,82 @@ struct DFPos {
 };
 
 // Affine map virtual point -> moving continuous index, as FP32 hi/lo pairs:
-// cidx_k = sum_j (Ahi + Alo)[k][j] x_j + (bhi + blo)[k].
+// cidx_k = sum_j (hi + lo)(k, j) x_j + (bhi + blo)(k).  Rows 0 and 1 lie in pairs, six
+// 16-byte words in all: (hi0j, hi1j, lo0j, lo1j) for j = 0..2, (bhi0, bhi1, blo0, blo1),
+// (hi20, lo20, hi21, lo21), (hi22, lo22, bhi2, blo2).
 struct __align__(16) AffineDF {
-  float Ahi[9], Alo[9], bhi[3], blo[3];
+  float v[24];
+  static constexpr int kHi(int k, int j) { return k < 2 ? 4 * j + k : 16 + 2 * j; }
+  static constexpr int kLo(int k, int j) { return k < 2 ? 4 * j + 2 + k : 17 + 2 * j; }
+  static constexpr int kBhi(int k) { return k < 2 ? 12 + k : 22; }
+  static constexpr int kBlo(int k) { return k < 2 ? 14 + k : 23; }
+  __host__ __device__ float& hi(int k, int j) { return v[kHi(k, j)]; }
+  __host__ __device__ float& lo(int k, int j) { return v[kLo(k, j)]; }
+  __host__ __device__ float& bhi(int k) { return v[kBhi(k)]; }
+  __host__ __device__ float& blo(int k) { return v[kBlo(k)]; }
+  __host__ __device__ float hi(int k, int j) const { return v[kHi(k, j)]; }
+  __host__ __device__ float lo(int k, int j) const { return v[kLo(k, j)]; }
+  __host__ __device__ float bhi(int k) const { return v[kBhi(k)]; }
+  __host__ __device__ float blo(int k) const { return v[kBlo(k)]; }
 };
 
-// A copy of a shared-memory map in six 16-byte loads (the per-sample loops read
-// the map once per sample; narrower loads cost more shared-memory wavefronts).
-__device__ __forceinline__ AffineDF load_map(const AffineDF& s) {
-  static_assert(sizeof(AffineDF) == 96, "six float4");
-  AffineDF r;
-  const float4* v = reinterpret_cast<const float4*>(&s);
-  float4* o = reinterpret_cast<float4*>(&r);
-#pragma unroll
-  for (int k = 0; k < 6; ++k) o[k] = v[k];
+__device__ __forceinline__ void two_sum2(f32x2 a, f32x2 b, f32x2& s, f32x2& e) {
+  s = add2(a, b);
+  const f32x2 bb = sub2(s, a);
+  e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+
+// Unevaluated sums s + err per axis, renormalized.
+__device__ __forceinline__ DFPos df_renorm(f32x2 s01, f32x2 e01, float s2, float e2) {
+  DFPos r;
+  const f32x2 hi = add2(s01, e01);
+  unpair(hi, r.hi[0], r.hi[1]);
+  unpair(sub2(e01, sub2(hi, s01)), r.lo[0], r.lo[1]);
+  r.hi[2] = __fadd_rn(s2, e2);
+  r.lo[2] = __fsub_rn(e2, __fsub_rn(r.hi[2], s2));
   return r;
 }
 
 // Continuous index of one float point to ~1e-12 voxel: products by FMA error
-// terms, sums by two-sum.
+// terms, sums by two-sum.  K in shared memory.
 __device__ __forceinline__ DFPos map_pos(const AffineDF& K, float x, float y, float z) {
+  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(K.v);
+  const float4* w = reinterpret_cast<const float4*>(K.v);
   const float xs[3] = {x, y, z};
-  DFPos r;
+  const ulonglong2 b01 = q[3];
+  const float4 r0 = w[4], r1 = w[5];
+  const float hi2[3] = {r0.x, r0.z, r1.x}, lo2[3] = {r0.y, r0.w, r1.y};
+  f32x2 s01 = b01.x, e01 = b01.y;
+  float s2 = r1.z, e2 = r1.w;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float s = K.bhi[k], err = K.blo[k];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const float a = K.Ahi[3 * k + j];
-      const float p = __fmul_rn(a, xs[j]);
-      const float pe = __fmaf_rn(a, xs[j], -p);  // exact product error
-      float t, e;
-      two_sum(s, p, t, e);
-      s = t;
-      err = __fadd_rn(err, __fadd_rn(e, __fmaf_rn(K.Alo[3 * k + j], xs[j], pe)));
-    }
-    r.hi[k] = __fadd_rn(s, err);
-    r.lo[k] = __fsub_rn(err, __fsub_rn(r.hi[k], s));
+  for (int j = 0; j < 3; ++j) {
+    const ulonglong2 A = q[j];
+    const f32x2 X = pair(xs[j]), nX = pair(-xs[j]);
+    const f32x2 p = mul2(A.x, X);
+    const f32x2 npe = fma2(A.x, nX, p);  // exact product error, negated
+    f32x2 t, e;
+    two_sum2(s01, p, t, e);
+    s01 = t;
+    e01 = add2(e01, sub2(e, fma2(A.y, nX, npe)));
+    const float p2 = __fmul_rn(hi2[j], xs[j]);
+    const float pe2 = __fmaf_rn(hi2[j], xs[j], -p2);
+    float t2, u2;
+    two_sum(s2, p2, t2, u2);
+    s2 = t2;
+    e2 = __fadd_rn(e2, __fadd_rn(u2, __fmaf_rn(lo2[j], xs[j], pe2)));
   }
-  return r;
+  return df_renorm(s01, e01, s2, e2);
 }
 
-// Nearest integer b = floor(hi + lo + 0.5) and the remainder hi + lo - b.
+// Nearest integer b = floor(hi + lo + 0.5) and the remainder hi + lo - b.  hi - rint(hi)
+// is exact; lo, at most half an ulp of hi, decides the ties and the crossings next to them
+// (the differences from 1/2 are exact there).
 __device__ __forceinline__ void split_nearest(float hi, float lo, int& b, float& f) {
-  float s, e;
-  two_sum(hi, 0.5f, s, e);
-  const float e2 = __fadd_rn(e, lo);
-  float fl = floorf(s);
-  if (s == fl) {
-    if (e2 < 0.f) fl -= 1.f;
-  } else if (e2 >= __fsub_rn(fl + 1.f, s)) {
-    fl += 1.f;
-  }
-  b = (int)fl;  // saturates for huge values: outside any buffer
-  f = __fadd_rn(__fsub_rn(hi, fl), lo);
+  const float r = rintf(hi);
+  const float d = __fsub_rn(hi, r);
+  const float adj = lo >= __fsub_rn(0.5f, d) ? 1.f : (lo < __fsub_rn(-0.5f, d) ? -1.f : 0.f);
+  b = (int)__fadd_rn(r, adj);  // saturates for huge values: outside any buffer
+  f = __fadd_rn(__fsub_rn(d, adj), lo);
 }
 
 __device__ __forceinline__ CIdx to_cidx(const DFPos& p) {
@@ -304,28 +381,35 @@ __device__ __forceinline__ void split_double_bits(double x, float& hi, float& lo
   lo = e < 949 ? 0.f : __uint2float_rn(w0 & 0x1fffffffu) * __uint_as_float(sign | ((unsigned)(e - 948) << 23));
 }
 
-// p + A u for a double-float matrix A and a double-float vector u (products with
-// FMA error terms, sums by two-sum), renormalized.
-__device__ __forceinline__ DFPos df_add_matvec(const DFPos& p, const AffineDF& A, const float uhi[3],
+// p + A u for a double-float matrix A (in shared memory) and a double-float vector u
+// (products with FMA error terms, sums by two-sum), renormalized.
+__device__ __forceinline__ DFPos df_add_matvec(const DFPos& p, const AffineDF& K, const float uhi[3],
                                                const float ulo[3]) {
-  DFPos r;
+  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(K.v);
+  const float4* w = reinterpret_cast<const float4*>(K.v);
+  const float4 r0 = w[4];
+  const float2 r1 = *reinterpret_cast<const float2*>(K.v + 20);
+  const float hi2[3] = {r0.x, r0.z, r1.x}, lo2[3] = {r0.y, r0.w, r1.y};
+  f32x2 s01 = pair(p.hi[0], p.hi[1]), e01 = pair(p.lo[0], p.lo[1]);
+  float s2 = p.hi[2], e2 = p.lo[2];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float s = p.hi[k], err = p.lo[k];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const float a = A.Ahi[3 * k + j];
-      const float q = __fmul_rn(a, uhi[j]);
-      const float qe = __fmaf_rn(a, uhi[j], -q);  // exact product error
-      float t, e;
-      two_sum(s, q, t, e);
-      s = t;
-      err = __fadd_rn(err, __fadd_rn(e, __fadd_rn(qe, __fmaf_rn(A.Alo[3 * k + j], uhi[j], __fmul_rn(a, ulo[j])))));
-    }
-    r.hi[k] = __fadd_rn(s, err);
-    r.lo[k] = __fsub_rn(err, __fsub_rn(r.hi[k], s));
+  for (int j = 0; j < 3; ++j) {
+    const ulonglong2 A = q[j];
+    const f32x2 U = pair(uhi[j]), nU = pair(-uhi[j]), nL = pair(-ulo[j]);
+    const f32x2 v = mul2(A.x, U);
+    const f32x2 nve = fma2(A.x, nU, v);  // exact product error, negated
+    f32x2 t, e;
+    two_sum2(s01, v, t, e);
+    s01 = t;
+    e01 = add2(e01, sub2(e, add2(nve, fma2(A.y, nU, mul2(A.x, nL)))));
+    const float v2 = __fmul_rn(hi2[j], uhi[j]);
+    const float ve2 = __fmaf_rn(hi2[j], uhi[j], -v2);
+    float t2, u2;
+    two_sum(s2, v2, t2, u2);
+    s2 = t2;
+    e2 = __fadd_rn(e2, __fadd_rn(u2, __fadd_rn(ve2, __fmaf_rn(lo2[j], uhi[j], __fmul_rn(hi2[j], ulo[j])))));
   }
-  return r;
+  return df_renorm(s01, e01, s2, e2);
 }
 
 // ---------------------------------------------------------------------------

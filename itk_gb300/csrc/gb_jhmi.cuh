@@ -112,7 +112,7 @@ __device__ __forceinline__ void jhmi_pass1_body(const EvalArgs& a, const JhmiCon
 }
 
 template <int GRAD>
-__global__ void __launch_bounds__(kBlock) k_jhmi_pass1(EvalArgs a, const JhmiConsts* C) {
+__global__ void __launch_bounds__(kBlock, GRAD == kGradImage ? 5 : 4) k_jhmi_pass1(EvalArgs a, const JhmiConsts* C) {
   jhmi_pass1_body<GRAD>(a, C, hw_grid());
 }
 
@@ -320,9 +320,8 @@ __device__ __forceinline__ void jhmi_pass2_body(const EvalArgs& a, const JhmiCon
   const float* mm = tab + B * B;
   float max_slope, inv_scale, mlo, mhi;
   jhmi_pass2_scalars(C, max_slope, inv_scale, mlo, mhi);
-  float acc[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) acc[k] = 0.f;
+  JacSums acc;
+  acc.zero();
   unsigned nv = 0;
   const int64_t stride = (int64_t)vg.n * blockDim.x;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -338,19 +337,10 @@ __device__ __forceinline__ void jhmi_pass2_body(const EvalArgs& a, const JhmiCon
     float sf;
     if (!jhmi_scaling(C, pdf, mm, B, s.w, cc.x, mlo, mhi, max_slope, inv_scale, sf)) continue;
     ++nv;
-    const float3 v = jac_vec(K, s.x, s.y, s.z);
-    const float t0 = sf * cc.y, t1 = sf * cc.z, t2 = sf * cc.w;
-    acc[0] = fmaf(t0, v.x, acc[0]); acc[1] = fmaf(t0, v.y, acc[1]); acc[2] = fmaf(t0, v.z, acc[2]);
-    acc[3] = fmaf(t1, v.x, acc[3]); acc[4] = fmaf(t1, v.y, acc[4]); acc[5] = fmaf(t1, v.z, acc[5]);
-    acc[6] = fmaf(t2, v.x, acc[6]); acc[7] = fmaf(t2, v.y, acc[7]); acc[8] = fmaf(t2, v.z, acc[8]);
-    acc[9] += t0; acc[10] += t1; acc[11] += t2;
+    acc.add(make_float3(sf * cc.y, sf * cc.z, sf * cc.w), jac_pair(K, s.x, s.y, s.z));
   }
   KahanF kacc[13];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    kacc[k].s = acc[k];
-    kacc[k].c = 0.f;
-  }
+  acc.split(kacc);
   // the valid count rides along as the 13th sum (exact in FP32 per thread, FP64 across blocks)
   kacc[12].s = (float)nv;
   kacc[12].c = 0.f;

@@ -46,12 +46,12 @@ constexpr double kQInv = 1.0 / 67108864.0;
 // stored as FP32 / double-float).  Sample records hold "domain coordinates":
 // the physical point for a sampled point set, the integer grid index for the
 // dense virtual domain (so dense points are exact).  `map` takes domain
-// coordinates to the moving continuous index; U, joff give the affine
-// Jacobian's x - c = U u + joff.
+// coordinates to the moving continuous index.
 struct EvalConsts {
   AffineDF map;
-  float U[9];
-  float joff[3];
+  // the affine Jacobian's x - c = U u + joff, rows 0 and 1 in pairs: (U0j, U1j) for
+  // j = 0..2, (joff0, joff1), then (U20, U21, U22, joff2)
+  float jac[12];
   float Mg[9];  // B-spline paths: gradient -> (M^T g), M the initial affine of a composite (identity otherwise)
   float Pm[9];  // B-spline paths: physical displacement -> moving index offset, P2I M
   // displacement-field paths (map = the identity transform's map):
@@ -61,11 +61,82 @@ struct EvalConsts {
                   // position takes one product per axis (bitwise the same result)
 };
 
-__device__ __forceinline__ float3 jac_vec(const EvalConsts& K, float x, float y, float z) {
-  return make_float3(fmaf(K.U[0], x, fmaf(K.U[1], y, fmaf(K.U[2], z, K.joff[0]))),
-                     fmaf(K.U[3], x, fmaf(K.U[4], y, fmaf(K.U[5], z, K.joff[1]))),
-                     fmaf(K.U[6], x, fmaf(K.U[7], y, fmaf(K.U[8], z, K.joff[2]))));
+// x - c of a sample: rows 0 and 1 as a pair, row 2.  K in shared memory.
+struct JacVec {
+  f32x2 xy;
+  float z;
+};
+__device__ __forceinline__ JacVec jac_pair(const EvalConsts& K, float x, float y, float z) {
+  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(K.jac);
+  const float4 r = *reinterpret_cast<const float4*>(K.jac + 8);
+  const ulonglong2 a = q[0], b = q[1];
+  JacVec v;
+  v.xy = fma2(a.x, pair(x), fma2(a.y, pair(y), fma2(b.x, pair(z), b.y)));
+  v.z = fmaf(r.x, x, fmaf(r.y, y, fmaf(r.z, z, r.w)));
+  return v;
 }
+__device__ __forceinline__ float3 jac_vec(const EvalConsts& K, float x, float y, float z) {
+  const JacVec v = jac_pair(K, x, y, z);
+  float3 r;
+  unpair(v.xy, r.x, r.y);
+  r.z = v.z;
+  return r;
+}
+
+// Sums of t_r (x - c)_c and t_r over a thread's samples, as pairs: (r0, r1) and (r2, the
+// translation's) of each row r; plain FP32 (JacSums) or compensated (JacKahan).  The twelve
+// derivative entries: 3 r + c, then 9 + r.
+struct JacSums {
+  f32x2 xy[3], zt[3];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int r = 0; r < 3; ++r) xy[r] = zt[r] = 0ull;
+  }
+  __device__ __forceinline__ void add(const float3& t, const JacVec& v) {
+    const float tt[3] = {t.x, t.y, t.z};
+    const f32x2 z1 = pair(v.z, 1.f);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      xy[r] = fma2(pair(tt[r]), v.xy, xy[r]);
+      zt[r] = fma2(pair(tt[r]), z1, zt[r]);
+    }
+  }
+  __device__ __forceinline__ void split(KahanF* d) const {  // d[0, 12)
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      unpair(xy[r], d[3 * r].s, d[3 * r + 1].s);
+      unpair(zt[r], d[3 * r + 2].s, d[9 + r].s);
+    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) d[k].c = 0.f;
+  }
+};
+struct JacKahan {
+  KahanF2 xy[3], zt[3];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      xy[r].zero();
+      zt[r].zero();
+    }
+  }
+  __device__ __forceinline__ void add(const float3& t, const JacVec& v) {
+    const float tt[3] = {t.x, t.y, t.z};
+    const f32x2 z1 = pair(v.z, 1.f);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      xy[r].add(mul2(pair(tt[r]), v.xy));
+      zt[r].add(mul2(pair(tt[r]), z1));
+    }
+  }
+  __device__ __forceinline__ void split(KahanF* d) const {  // d[0, 12)
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      xy[r].split(d[3 * r], d[3 * r + 1]);
+      zt[r].split(d[3 * r + 2], d[9 + r]);
+    }
+  }
+};
 
 // MatrixOffsetTransformBase::ComputeOffset (itkMatrixOffsetTransformBase.hxx:612-631)
 // composed with ImageBase::TransformPhysicalPointToContinuousIndex (itkImageBase.h:515-531).
@@ -88,8 +159,14 @@ __host__ __device__ inline void affine_const_entry(int e, const double* p, const
   const double* U = dom2phys ? dom2phys : I;
   const double* u0 = dom2phys ? dom_origin : Z;
   if (e == 12) {
-    for (int i = 0; i < 9; ++i) K.U[i] = (float)U[i];
-    for (int i = 0; i < 3; ++i) K.joff[i] = (float)(u0[i] - center[i]);
+    for (int j = 0; j < 3; ++j) {
+      K.jac[2 * j] = (float)U[j];
+      K.jac[2 * j + 1] = (float)U[3 + j];
+      K.jac[8 + j] = (float)U[6 + j];
+    }
+    K.jac[6] = (float)(u0[0] - center[0]);
+    K.jac[7] = (float)(u0[1] - center[1]);
+    K.jac[11] = (float)(u0[2] - center[2]);
     for (int r = 0; r < 3; ++r)
       for (int c = 0; c < 3; ++c) K.Mg[r * 3 + c] = (float)p[c * 3 + r];  // M^T
     return;
@@ -112,7 +189,7 @@ __host__ __device__ inline void affine_const_entry(int e, const double* p, const
     const int c = e % 3;
     double s = 0.0;
     for (int k = 0; k < 3; ++k) s = dadd(s, dmul(Ar[k], U[k * 3 + c]));
-    split_df(s, K.map.Ahi[e], K.map.Alo[e]);
+    split_df(s, K.map.hi(r, c), K.map.lo(r, c));
     return;
   }
   double br = 0.0;
@@ -122,7 +199,7 @@ __host__ __device__ inline void affine_const_entry(int e, const double* p, const
     br = dadd(br, dmul(m_p2i[r * 3 + k], dadd(o, -m_origin[k])));
   }
   for (int k = 0; k < 3; ++k) br = dadd(br, dmul(Ar[k], u0[k]));
-  split_df(br, K.map.bhi[r], K.map.blo[r]);
+  split_df(br, K.map.bhi(r), K.map.blo(r));
 }
 
 __host__ __device__ inline void affine_consts(const double* p, const double center[3], const double m_p2i[9],
@@ -589,29 +666,31 @@ __device__ __forceinline__ void msq_affine_body(const EvalArgs& a, VGrid vg) {
   griddep_launch_dependents();
   load_consts(a.consts, K);
   __syncthreads();
-  KahanF acc[13];
-#pragma unroll
-  for (int k = 0; k < 13; ++k) acc[k].zero();
+  KahanF sq;
+  sq.zero();
+  JacKahan jac;
+  jac.zero();
   unsigned nv = 0;
-  const int64_t stride = (int64_t)vg.n * blockDim.x;
-  int64_t i = (int64_t)vg.b * blockDim.x + threadIdx.x;
-  float4 s_next = i < a.n ? __ldcs(a.samples + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-  for (; i < a.n; i += stride) {
+  // 32-bit sample indices (a handle holds at most 2^31 - 1)
+  const unsigned n = (unsigned)a.n, stride = (unsigned)(vg.n * kBlock);
+  unsigned i = (unsigned)(vg.b * kBlock) + threadIdx.x;
+  float4 s_next = i < n ? __ldcs(a.samples + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (; i < n; i += stride) {
     const float4 s = s_next;
-    s_next = i + stride < a.n ? __ldcs(a.samples + i + stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+    s_next = i + stride < n ? __ldcs(a.samples + i + stride) : make_float4(0.f, 0.f, 0.f, 0.f);
     float m;
     float3 g;
-    const DFPos p = map_pos(load_map(K.map), s.x, s.y, s.z);
+    const DFPos p = map_pos(K.map, s.x, s.y, s.z);
     if (!eval_moving<GRAD>(a, p, a.with_derivative != 0, m, g)) continue;
     const float diff = s.w - m;  // FixedImagePixelType diff, MeanSquares...Threader.hxx:46
-    acc[0].add(diff * diff);
+    sq.add(diff * diff);
     ++nv;
     if (a.with_derivative) {
       const float t = 2.f * diff;
-      const float3 v = jac_vec(K, s.x, s.y, s.z);
-      const float vx = v.x, vy = v.y, vz = v.z;
-      const float t0 = t * g.x, t1 = t * g.y, t2 = t * g.z;
       if (FPC) {
+        const float3 v = jac_vec(K, s.x, s.y, s.z);
+        const float vx = v.x, vy = v.y, vz = v.z;
+        const float t0 = t * g.x, t1 = t * g.y, t2 = t * g.z;
         // StorePointDerivativeResult with UseFloatingPointCorrection
         // (ThreaderBase.hxx:284-294): static_cast<intmax_t>(d * r) / r per parameter
         const float ld[12] = {t0 * vx, t0 * vy, t0 * vz, t1 * vx, t1 * vy, t1 * vz,
@@ -620,14 +699,14 @@ __device__ __forceinline__ void msq_affine_body(const EvalArgs& a, VGrid vg) {
         for (int k = 0; k < (FPC ? 12 : 1); ++k)
           dacc[k] += (double)(long long)((double)ld[k] * a.fp_res) / a.fp_res;
       } else {
-        acc[1].add(t0 * vx); acc[2].add(t0 * vy); acc[3].add(t0 * vz);
-        acc[4].add(t1 * vx); acc[5].add(t1 * vy); acc[6].add(t1 * vz);
-        acc[7].add(t2 * vx); acc[8].add(t2 * vy); acc[9].add(t2 * vz);
-        acc[10].add(t0); acc[11].add(t1); acc[12].add(t2);
+        jac.add(make_float3(t * g.x, t * g.y, t * g.z), jac_pair(K, s.x, s.y, s.z));
       }
     }
   }
   block_count(nv, a.acc_n);
+  KahanF acc[13];
+  acc[0] = sq;
+  jac.split(acc + 1);
   block_sums<13>(acc, red, blk);
   if (FPC) {
     // the truncated derivatives: FP64 warp trees, warps in order
@@ -661,8 +740,10 @@ __device__ __forceinline__ void msq_affine_body(const EvalArgs& a, VGrid vg) {
   }
 }
 
+// Four blocks per SM where 64 registers hold a sample (256x256x200 dense: 195 us with the
+// three that 70 registers leave, 181 with four).
 template <int GRAD, bool FPC = false>
-__global__ void __launch_bounds__(kBlock) k_msq_affine(EvalArgs a) {
+__global__ void __launch_bounds__(kBlock, GRAD == kGradImage && !FPC ? 4 : (FPC ? 3 : 2)) k_msq_affine(EvalArgs a) {
   msq_affine_body<GRAD, FPC>(a, hw_grid());
 }
 
@@ -844,14 +925,14 @@ __device__ __forceinline__ DFPos field_pos_diag(const EvalConsts& K, float x, fl
   DFPos r;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    float s = K.map.bhi[k], err = K.map.blo[k];
-    const float a = K.map.Ahi[4 * k];
+    float s = K.map.bhi(k), err = K.map.blo(k);
+    const float a = K.map.hi(k, k);
     const float p = __fmul_rn(a, xs[k]);
     const float pe = __fmaf_rn(a, xs[k], -p);
     float t, e;
     two_sum(s, p, t, e);
     s = t;
-    err = __fadd_rn(err, __fadd_rn(e, __fmaf_rn(K.map.Alo[4 * k], xs[k], pe)));
+    err = __fadd_rn(err, __fadd_rn(e, __fmaf_rn(K.map.lo(k, k), xs[k], pe)));
     r.hi[k] = __fadd_rn(s, err);
     r.lo[k] = __fsub_rn(err, __fsub_rn(r.hi[k], s));
   }
@@ -859,13 +940,13 @@ __device__ __forceinline__ DFPos field_pos_diag(const EvalConsts& K, float x, fl
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     float s = r.hi[k], err = r.lo[k];
-    const float a = K.umap.Ahi[4 * k];
+    const float a = K.umap.hi(k, k);
     const float p = __fmul_rn(a, uhi[k]);
     const float pe = __fmaf_rn(a, uhi[k], -p);
     float t, e;
     two_sum(s, p, t, e);
     s = t;
-    err = __fadd_rn(err, __fadd_rn(e, __fadd_rn(pe, __fmaf_rn(K.umap.Alo[4 * k], uhi[k], __fmul_rn(a, ulo[k])))));
+    err = __fadd_rn(err, __fadd_rn(e, __fadd_rn(pe, __fmaf_rn(K.umap.lo(k, k), uhi[k], __fmul_rn(a, ulo[k])))));
     q.hi[k] = __fadd_rn(s, err);
     q.lo[k] = __fsub_rn(err, __fsub_rn(q.hi[k], s));
   }
@@ -891,7 +972,7 @@ __device__ __forceinline__ DFPos sample_pos(const EvalArgs& a, const EvalConsts&
     for (int k = 0; k < 3; ++k) split_double_bits(__ldg(q + k), uhi[k], ulo[k]);
     return field_pos_diag(K, s.x, s.y, s.z, uhi, ulo);
   }
-  const DFPos p = map_pos(load_map(K.map), s.x, s.y, s.z);
+  const DFPos p = map_pos(K.map, s.x, s.y, s.z);
   if (TK == kMapAffine) return p;
   float uhi[3], ulo[3];
   if (TK == kMapFieldDense) {
@@ -1506,9 +1587,8 @@ __device__ __forceinline__ void mattes_pass2_affine_body(const EvalArgs& a, VGri
   for (int k = cw; k < kConstWords; k += blockDim.x)
     reinterpret_cast<float*>(&K)[k] = k == cw ? cword : __ldcg(reinterpret_cast<const float*>(a.consts) + k);
   __syncthreads();  // the barriers' initialization and the constants
-  float acc[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) acc[k] = 0.f;
+  JacSums acc;
+  acc.zero();
   if (!GROUP_WARP) {
     if (threadIdx.x == 0) nfac_s = -1.0 / (a.m_bs * (double)N);
     mattes_pratio_build<false>(a, T, pr, colf, fmask);
@@ -1556,12 +1636,7 @@ __device__ __forceinline__ void mattes_pass2_affine_body(const EvalArgs& a, VGri
         parzen_deriv(tt, d);
         const float* row = pr + __float_as_int(s.w) * B + pdfm;
         const float w = row[0] * d[0] + row[1] * d[1] + row[2] * d[2] + row[3] * d[3];
-        const float3 v = jac_vec(K, s.x, s.y, s.z);
-        const float t0 = w * cc.y, t1 = w * cc.z, t2 = w * cc.w;
-        acc[0] = fmaf(t0, v.x, acc[0]); acc[1] = fmaf(t0, v.y, acc[1]); acc[2] = fmaf(t0, v.z, acc[2]);
-        acc[3] = fmaf(t1, v.x, acc[3]); acc[4] = fmaf(t1, v.y, acc[4]); acc[5] = fmaf(t1, v.z, acc[5]);
-        acc[6] = fmaf(t2, v.x, acc[6]); acc[7] = fmaf(t2, v.y, acc[7]); acc[8] = fmaf(t2, v.z, acc[8]);
-        acc[9] += t0; acc[10] += t1; acc[11] += t2;
+        acc.add(make_float3(w * cc.y, w * cc.z, w * cc.w), jac_pair(K, s.x, s.y, s.z));
       }
       // stage st consumed by every streaming thread; `failed` seen by all of them
       if (GROUP_WARP) stream_barrier();
@@ -1585,11 +1660,7 @@ __device__ __forceinline__ void mattes_pass2_affine_body(const EvalArgs& a, VGri
     return;
   }
   KahanF kacc[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    kacc[k].s = acc[k];
-    kacc[k].c = 0.f;
-  }
+  acc.split(kacc);
   block_sums_df<12>(kacc, red, blk);
   DFloat* part = reinterpret_cast<DFloat*>(a.part + kPartPass2);
   // staged form: the last block requests every block partial at once into the (now idle)

@@ -123,6 +123,15 @@ static int full_wave(const gb_metric* m, K kernel, size_t smem, int64_t n) {
   return grid_for(m, n, per_sm);
 }
 
+// The same with the blocks evened out: every block runs the same number of iterations
+// (64^3 dense: 512 blocks of two 256-sample iterations, not 608 of one or two; 20 -> 17 us).
+template <typename K>
+static int even_wave(const gb_metric* m, K kernel, size_t smem, int64_t n) {
+  const int64_t tiles = std::max<int64_t>(1, (n + kBlock - 1) / kBlock), cap = full_wave(m, kernel, smem, n);
+  const int64_t each = (tiles + cap - 1) / cap;
+  return (int)((tiles + each - 1) / each);
+}
+
 static bool is_bspline(const gb_metric* m) {
   return m->tkind == GB_TRANSFORM_BSPLINE || m->tkind == GB_TRANSFORM_COMPOSITE;
 }
@@ -959,23 +968,23 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
       for (int cc = 0; cc < 3; ++cc) {
         double s = 0.0;
         for (int k = 0; k < 3; ++k) s = gb::dadd(s, gb::dmul(m->moving.p2i[3 * r + k], p[3 * k + cc]));
-        split_df(s, K.umap.Ahi[3 * r + cc], K.umap.Alo[3 * r + cc]);
+        split_df(s, K.umap.hi(r, cc), K.umap.lo(r, cc));
       }
     for (int r = 0; r < 3; ++r) {
-      K.umap.bhi[r] = K.umap.blo[r] = 0.f;
+      K.umap.bhi(r) = K.umap.blo(r) = 0.f;
       double b = 0.0;
       for (int k = 0; k < 3; ++k) {
-        split_df(m->virt.p2i[3 * r + k], K.fmap.Ahi[3 * r + k], K.fmap.Alo[3 * r + k]);
+        split_df(m->virt.p2i[3 * r + k], K.fmap.hi(r, k), K.fmap.lo(r, k));
         b = gb::dadd(b, -gb::dmul(m->virt.p2i[3 * r + k], m->virt.origin[k]));
       }
-      split_df(b, K.fmap.bhi[r], K.fmap.blo[r]);
+      split_df(b, K.fmap.bhi(r), K.fmap.blo(r));
     }
     bool diag = true;
     for (int r = 0; r < 3; ++r)
       for (int c = 0; c < 3; ++c)
         if (r != c)
-          diag = diag && K.map.Ahi[3 * r + c] == 0.f && K.map.Alo[3 * r + c] == 0.f && K.umap.Ahi[3 * r + c] == 0.f &&
-                 K.umap.Alo[3 * r + c] == 0.f;
+          diag = diag && K.map.hi(r, c) == 0.f && K.map.lo(r, c) == 0.f && K.umap.hi(r, c) == 0.f &&
+                 K.umap.lo(r, c) == 0.f;
     K.fdiag = diag ? 1.f : 0.f;
     GB_CUDA(cudaMemcpyAsync(m->d_consts.p, m->h_consts, sizeof(EvalConsts), cudaMemcpyHostToDevice, st));
   }
@@ -1404,12 +1413,9 @@ int gb::enqueue_eval(gb_metric* m, const double* d_params, double* d_out, bool d
     return GB_OK;
   }
   if (m->kind == GB_METRIC_MEAN_SQUARES) {
-    if (a.fp_res > 0.0)
-      GB_CUDA(cd ? launch_wave(m, k_msq_affine<kGradCentralDifference, true>, 0, a)
-                 : launch_wave(m, k_msq_affine<kGradImage, true>, 0, a));
-    else
-      GB_CUDA(cd ? launch_wave(m, k_msq_affine<kGradCentralDifference>, 0, a)
-                 : launch_wave(m, k_msq_affine<kGradImage>, 0, a));
+    auto kernel = a.fp_res > 0.0 ? (cd ? k_msq_affine<kGradCentralDifference, true> : k_msq_affine<kGradImage, true>)
+                                 : (cd ? k_msq_affine<kGradCentralDifference> : k_msq_affine<kGradImage>);
+    GB_CUDA(launch_chain(m, kernel, (unsigned)even_wave(m, kernel, 0, m->nsamples), kBlock, 0, a));
     m->mark();
     return GB_OK;
   }

@@ -76,9 +76,10 @@ __global__ void __launch_bounds__(kBlock) k_msq_affine_noalloc(NoAllocArgs na) {
   unsigned* tickets = reinterpret_cast<unsigned*>(na.scratch + 8);
   double* part = reinterpret_cast<double*>(na.scratch + kNoAllocPartOffset);
   double* grp = reinterpret_cast<double*>(na.scratch + kNoAllocGroupOffset);
-  KahanF acc[kNoAllocValues];
-#pragma unroll
-  for (int k = 0; k < kNoAllocValues; ++k) acc[k].zero();
+  KahanF sq;
+  sq.zero();
+  JacKahan jac;
+  jac.zero();
   unsigned nv = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < na.n; i += stride) {
@@ -87,16 +88,14 @@ __global__ void __launch_bounds__(kBlock) k_msq_affine_noalloc(NoAllocArgs na) {
     if (!ci_inside(c, na.nx, na.ny, na.nz)) continue;
     const float4 v = gather4(na.mov4, make_stencil(c, na.nx, na.ny, na.nz), na.nx, na.ny);
     const float diff = s.w - v.x;
-    acc[0].add(diff * diff);
+    sq.add(diff * diff);
     ++nv;
     const float t = 2.f * diff;
-    const float3 q = jac_vec(K, s.x, s.y, s.z);
-    const float t0 = t * v.y, t1 = t * v.z, t2 = t * v.w;
-    acc[1].add(t0 * q.x); acc[2].add(t0 * q.y); acc[3].add(t0 * q.z);
-    acc[4].add(t1 * q.x); acc[5].add(t1 * q.y); acc[6].add(t1 * q.z);
-    acc[7].add(t2 * q.x); acc[8].add(t2 * q.y); acc[9].add(t2 * q.z);
-    acc[10].add(t0); acc[11].add(t1); acc[12].add(t2);
+    jac.add(make_float3(t * v.y, t * v.z, t * v.w), jac_pair(K, s.x, s.y, s.z));
   }
+  KahanF acc[kNoAllocValues];
+  acc[0] = sq;
+  jac.split(acc + 1);
   block_count(nv, acc_n);
   block_sums<kNoAllocValues>(acc, red, blk);
   if (!grid_sums<kNoAllocValues>(blk, part, grp, tickets, fin)) return;
