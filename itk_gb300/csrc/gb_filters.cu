@@ -70,9 +70,6 @@ static int rg_setup(double sigma, double spacing, int order, bool normalize_acro
   c.d[1] = 4 * cos2 * cos1 * e1 * e2;
   c.d[1] += e1 * e1 + e2 * e2;
   c.d[0] = -2 * (e2 * cos2 + e1 * cos1);
-  // the recursion runs with FP32 coefficients: the normalization below is that of the rounded
-  // poles, so that their rounding (of the order of the gain over a wide kernel) drops out
-  for (int k = 0; k < 4; ++k) c.d[k] = (double)(float)c.d[k];
   const double SD = 1.0 + c.d[0] + c.d[1] + c.d[2] + c.d[3];
   const double DD = c.d[0] + 2 * c.d[1] + 3 * c.d[2] + 4 * c.d[3];
   // numerator of the causal part
@@ -114,13 +111,9 @@ static int rg_setup(double sigma, double spacing, int order, bool normalize_acro
 
 static RGCoefF to_float(const RGCoef& c) {
   RGCoefF f;
-  // the last (smallest) tap takes up the others' roundings, which keeps the taps' sum
-  double rn = 0.0, rm = 0.0;
   for (int k = 0; k < 4; ++k) {
-    f.dir[0].a[k] = (float)(c.n[k] + (k == 3 ? rn : 0.0));
-    f.dir[1].a[k + 1] = (float)(c.m[k] + (k == 3 ? rm : 0.0));
-    rn += c.n[k] - (double)f.dir[0].a[k];
-    rm += c.m[k] - (double)f.dir[1].a[k + 1];
+    f.dir[0].a[k] = (float)c.n[k];
+    f.dir[1].a[k + 1] = (float)c.m[k];
     f.dir[0].d[k] = f.dir[1].d[k] = (float)c.d[k];
   }
   f.dir[0].a[4] = f.dir[1].a[0] = 0.f;
