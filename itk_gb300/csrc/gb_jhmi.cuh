@@ -15,7 +15,7 @@
 //                   histogram, flushed with 64-bit atomics (order-free, so exact);
 //   k_jhmi_finalize a few blocks: the normalized PDF, the discrete-Gaussian smoothing
 //                   (separable, zero-flux border, moving axis first), the marginals
-//                   and the value (fixed-order trees); FP32 tables for pass 2;
+//                   and the value (fixed order); FP32 tables for pass 2;
 //   k_jhmi_pass2    per sample: bilinear PDF value and moving-axis slope, the
 //                   marginal and its slope, the clamped log-slope difference times
 //                   J^T g, fixed-order sums; the last block divides by the count.
@@ -25,14 +25,15 @@
 // reference's bin.
 #pragma once
 
+#include <cstddef>
+
 #include "gb_bspline.cuh"
 #include "gb_field.cuh"
 #include "gb_kernels.cuh"
 
 namespace gb {
 
-constexpr int kJhmiMaxBins = 64;  // the finalize blocks keep two bins^2 FP64 planes in shared memory
-constexpr int kJhmiFinalizeBlocks = 8;
+constexpr int kJhmiMaxBins = 64;
 
 // Joint-PDF constants (host-computed in FP64 at Initialize).
 struct JhmiConsts {
@@ -42,8 +43,18 @@ struct JhmiConsts {
   float fmin_f, finv_f, mmin_f, minv_f;  // FP32 twins: min, 1 / (max - min)
   float origin_f, inv_spacing_f, spacing_f;
   int radius;                            // discrete Gaussian radius (0: no smoothing)
-  double kernel[65];                     // 2 radius + 1 coefficients
+  // the finalize kernel's: the 2 radius + 1 coefficients, and what a bin adds to the sum of
+  // its smoothed line (1 but near the ends, where the border repeats the end bins)
+  double kernel[65];
+  double share[kJhmiMaxBins];
 };
+
+// The sample passes' part of the constants (all but the smoothing) into shared memory.
+__device__ __forceinline__ void load_jhmi(const JhmiConsts* __restrict__ gC, JhmiConsts& C) {
+  const unsigned* src = reinterpret_cast<const unsigned*>(gC);
+  unsigned* dst = reinterpret_cast<unsigned*>(&C);
+  for (int k = threadIdx.x; k < (int)(offsetof(JhmiConsts, kernel) / 4); k += blockDim.x) dst[k] = __ldg(src + k);
+}
 
 // Joint bin along one axis: TransformPhysicalPointToIndex (round half up) of the
 // joint-PDF point; -1 outside [0, bins).
@@ -74,11 +85,7 @@ __device__ __forceinline__ void jhmi_pass1_body(const EvalArgs& a, const JhmiCon
   if (halted(a)) return;
   griddep_launch_dependents();
   load_consts(a.consts, K);
-  {
-    const unsigned* src = reinterpret_cast<const unsigned*>(gC);
-    unsigned* dst = reinterpret_cast<unsigned*>(&C);
-    for (int k = threadIdx.x; k < (int)(sizeof(JhmiConsts) / 4); k += blockDim.x) dst[k] = __ldg(src + k);
-  }
+  load_jhmi(gC, C);
   __syncthreads();
   unsigned nv = 0;
   const int64_t stride = (int64_t)vg.n * blockDim.x;
@@ -116,28 +123,34 @@ __global__ void __launch_bounds__(kBlock, GRAD == kGradImage ? 5 : 4) k_jhmi_pas
   jhmi_pass1_body<GRAD>(a, C, hw_grid());
 }
 
-// One thread per output: out[x] = sum_k c[k] in[clamp(x + k - r)] along `dir`
-// (0: the fixed index, contiguous; 1: the moving index), ZeroFluxNeumann border.
-__device__ __forceinline__ void jhmi_gauss_pass(const double* in, double* out, int B, int dir, const JhmiConsts& C) {
+// Blocks of k_jhmi_finalize: about 64 bins each (two warps of FP64 logarithms).
+__host__ __device__ inline int jhmi_finalize_blocks(int B) { return (B * B + 63) / 64; }
+
+// sum_k c[k] in[clamp(x + k - r) * step] (DiscreteGaussianImageFilter, ZeroFluxNeumann border).
+__device__ __forceinline__ double jhmi_smooth(const double* in, int step, int x, int B, const JhmiConsts& C) {
   const int r = C.radius;
-  for (int q = threadIdx.x; q < B * B; q += blockDim.x) {
-    const int i = q % B, j = q / B;
-    double s = 0.0;
-    for (int k = 0; k <= 2 * r; ++k) {
-      int t = (dir == 0 ? i : j) + k - r;
-      t = t < 0 ? 0 : (t > B - 1 ? B - 1 : t);
-      s += C.kernel[k] * (dir == 0 ? in[t + B * j] : in[i + B * t]);
-    }
-    out[q] = s;
+  double s = 0.0;
+  for (int k = 0; k <= 2 * r; ++k) {
+    int t = x + k - r;
+    t = t < 0 ? 0 : (t > B - 1 ? B - 1 : t);
+    s += C.kernel[k] * in[t * step];
   }
+  return s;
 }
 
-// k_jhmi_finalize (kJhmiFinalizeBlocks blocks).  Writes the smoothed PDF (FP64, pdf_out; FP32 and the
-// FP32 moving marginal into the pratio table), the value, the count and the status.
+// k_jhmi_finalize (jhmi_finalize_blocks blocks).  Writes the smoothed PDF (FP64, pdf_out; FP32 and
+// the FP32 moving marginal into the pratio table), the value, the count and the status.  Each block
+// forms its own bins: the marginals (the smoothing is linear, so the marginals
+// of the smoothed PDF are smoothed sums of the counts), the smoothed PDF of its rows, moving axis
+// first, and its terms of the value.  Bound by FP64 (about 1.7 operations per SM and clock): with
+// every block smoothing the whole PDF and summing it to marginals by warp trees it took 16 to 18 us
+// for 20 bins.  Dynamic shared memory: 2 B^2 + 4 B doubles.
+__host__ __device__ inline size_t jhmi_finalize_shared(int B) { return sizeof(double) * (2 * (size_t)B * B + 4 * (size_t)B); }
+
 __global__ void __launch_bounds__(kBlock) k_jhmi_finalize(EvalArgs a, const JhmiConsts* gC) {
-  extern __shared__ double plane[];  // 2 B^2 doubles, then 2 B (marginals)
+  extern __shared__ double plane[];
   __shared__ JhmiConsts C;
-  __shared__ double red[kBlock / 32];
+  __shared__ double red[kBlock / 32], inv_s;
   griddep_wait();
   if (halted(a)) return;
   griddep_launch_dependents();
@@ -147,48 +160,48 @@ __global__ void __launch_bounds__(kBlock) k_jhmi_finalize(EvalArgs a, const Jhmi
     unsigned* dst = reinterpret_cast<unsigned*>(&C);
     for (int k = threadIdx.x; k < (int)(sizeof(JhmiConsts) / 4); k += blockDim.x) dst[k] = __ldg(src + k);
   }
-  double* p0 = plane;
-  double* p1 = plane + B * B;
-  double* fm = plane + 2 * B * B;
+  double* p0 = plane;           // the counts; sums of them are normalized last
+  double* p1 = p0 + B * B;      // smoothed along the moving axis: the block's rows
+  double* fr = p1 + B * B;      // fixed and moving marginals, along their own axis yet to smooth
+  double* mr = fr + B;
+  double* fm = mr + B;          // the marginals
   double* mm = fm + B;
   const unsigned long long N = __ldcg(a.acc_n);
-  const double invN = N > 0 ? 1.0 / (double)N : 0.0;
-  for (int k = threadIdx.x; k < B * B; k += blockDim.x) p0[k] = (double)__ldcg(&a.hist[k]) * invN;
+  for (int k = threadIdx.x; k < B * B; k += blockDim.x) p0[k] = (double)__ldcg(&a.hist[k]);
+  if (threadIdx.x == blockDim.x / 2) inv_s = N > 0 ? 1.0 / (double)N : 0.0;
   __syncthreads();
-  double* pdf = p0;
-  if (C.radius > 0) {  // DiscreteGaussianImageFilter: the moving axis, then the fixed axis
-    jhmi_gauss_pass(p0, p1, B, 1, C);
-    __syncthreads();
-    jhmi_gauss_pass(p1, p0, B, 0, C);
-    __syncthreads();
-  }
-  // marginals: moving = sum over the fixed index, fixed = sum over the moving index;
-  // one warp per marginal bin: lane-strided loads, a fixed XOR tree (short FP64 chains)
-  {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int t = warp; t < 2 * B; t += nw) {
-      double s = 0.0;
-      if (t < B) {
-        for (int i = lane; i < B; i += 32) s += pdf[i + B * t];
-      } else {
-        for (int j = lane; j < B; j += 32) s += pdf[(t - B) + B * j];
-      }
-      s = warp_sum_d(s);
-      if (lane == 0) (t < B ? mm[t] : fm[t - B]) = s;
-    }
-  }
-  __syncthreads();
-  // the value over this block's share of the bins: per-thread sums in a fixed bin
-  // order, a fixed XOR tree per warp, the warps in order; the blocks' partials are
-  // added in block order by the last block.  Each block repeats the (small) PDF,
-  // smoothing and marginals so the FP64 logs spread over kJhmiFinalizeBlocks SMs.
+  const double invN = inv_s;
+  const bool smooth = C.radius > 0;
   const int q0 = (int)((long long)B * B * blockIdx.x / gridDim.x);
   const int q1 = (int)((long long)B * B * (blockIdx.x + 1) / gridDim.x);
+  const int j0 = q0 / B, rows = q1 > q0 ? (q1 - 1) / B - j0 + 1 : 0;
+  // the two marginals by the first warps, the rows' moving-axis smoothing by the last ones
+  for (int t = threadIdx.x; t < 2 * B; t += blockDim.x) {
+    const bool fixed = t < B;
+    const double* line = p0 + (fixed ? t : B * (t - B));
+    const int step = fixed ? B : 1;
+    double s = 0.0;
+    for (int k = 0; k < B; ++k) s += (smooth ? C.share[k] : 1.0) * line[k * step];
+    (fixed ? fr[t] : mr[t - B]) = s;
+  }
+  for (int t = blockDim.x - 1 - threadIdx.x; t < rows * B; t += blockDim.x) {
+    const int i = t % B, j = j0 + t / B;
+    p1[i + B * j] = smooth ? jhmi_smooth(p0 + i, B, j, B, C) : p0[i + B * j];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 2 * B; t += blockDim.x) {
+    const double* line = t < B ? fr : mr;
+    const int x = t < B ? t : t - B;
+    (t < B ? fm : mm)[x] = (smooth ? jhmi_smooth(line, 1, x, B, C) : line[x]) * invN;
+  }
+  __syncthreads();
+  // the value over this block's bins: per-thread sums in a fixed bin order, a fixed XOR tree
+  // per warp, the warps in order; the blocks' partials are added in block order by the last block
   double s = 0.0;
   for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
     const int i = q % B, j = q / B;
+    const double pxy = (smooth ? jhmi_smooth(p1 + B * j, 1, i, B, C) : p1[q]) * invN;
     const double denom = fm[i] * mm[j];
-    const double pxy = pdf[q];
     double local = 0.0;
     if (fabs(denom) > DBL_EPSILON && pxy / denom > DBL_EPSILON) local = pxy * log(pxy / denom);
     s += local;
@@ -206,9 +219,12 @@ __global__ void __launch_bounds__(kBlock) k_jhmi_finalize(EvalArgs a, const Jhmi
     a.part[blockIdx.x] = t;
   }
   if (!last_block(a.tickets + kTicketFinalize)) return;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
+    // lane-strided over the blocks, then a fixed XOR tree
     double t = 0.0;
-    for (int k = 0; k < (int)gridDim.x; ++k) t += __ldcg(&a.part[k]);
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += 32) t += __ldcg(&a.part[k]);
+    t = warp_sum_d(t);
+    if (threadIdx.x != 0) return;
     a.out[1] = (double)N;
     if (N == 0) {  // GetValue: VerifyNumberOfValidPoints, a warning and the maximum value
       a.out[0] = DBL_MAX;
@@ -310,11 +326,7 @@ __device__ __forceinline__ void jhmi_pass2_body(const EvalArgs& a, const JhmiCon
   griddep_launch_dependents();
   for (int k = threadIdx.x; k < B * B + B; k += blockDim.x) tab[k] = __ldcg(&a.pratio[k]);
   load_consts(a.consts, K);
-  {
-    const unsigned* src = reinterpret_cast<const unsigned*>(gC);
-    unsigned* dst = reinterpret_cast<unsigned*>(&C);
-    for (int k = threadIdx.x; k < (int)(sizeof(JhmiConsts) / 4); k += blockDim.x) dst[k] = __ldg(src + k);
-  }
+  load_jhmi(gC, C);
   __syncthreads();
   const float* pdf = tab;
   const float* mm = tab + B * B;
@@ -373,12 +385,6 @@ __global__ void __launch_bounds__(kBlock) k_jhmi_pass2(EvalArgs a, const JhmiCon
 // a_s = sf M^T g (zero for an invalid sample or one outside the B-spline's valid
 // region) in place, counts the derivative points, and leaves the sparse Jacobian
 // sums to the B-spline chunk and parameter kernels (MeanSquares form: sum / count).
-
-__device__ __forceinline__ void load_jhmi(const JhmiConsts* __restrict__ gC, JhmiConsts& C) {
-  const unsigned* src = reinterpret_cast<const unsigned*>(gC);
-  unsigned* dst = reinterpret_cast<unsigned*>(&C);
-  for (int k = threadIdx.x; k < (int)(sizeof(JhmiConsts) / 4); k += blockDim.x) dst[k] = __ldg(src + k);
-}
 
 // Dynamic shared memory: the B^2 histogram, then (16-byte aligned) the nodes.
 __host__ __device__ inline size_t jhmi_bspline_node_offset(int B) { return ((size_t)4 * B * B + 15) / 16 * 16; }

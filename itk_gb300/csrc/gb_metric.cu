@@ -758,6 +758,9 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
     C.inv_spacing_f = (float)C.inv_spacing;
     C.spacing_f = (float)C.spacing;
     C.radius = m->jhmi_variance > 0.0 ? discrete_gaussian_kernel(m->jhmi_variance, 0.01, 32, C.kernel) : 0;
+    for (int x = 0; x < (int)m->bins; ++x)  // bin x of a smoothed line takes kernel[k] of bin x + k - radius
+      for (int k = 0; k <= 2 * C.radius; ++k)
+        C.share[std::max(0, std::min((int)m->bins - 1, x + k - C.radius))] += C.kernel[k];
     m->mstate[0] = C.fmin;
     m->mstate[1] = C.fmax;
     m->mstate[2] = C.mmin;
@@ -1295,8 +1298,16 @@ static int enqueue_eval_corr_bspline(gb_metric* m, const EvalArgs& a, bool cd, b
   return enqueue_bspline_sums(m, a);
 }
 
-// Joint-histogram MI: the histogram pass, the one-block PDF / value kernel, the
-// derivative pass.
+static cudaError_t launch_jhmi_finalize(gb_metric* m, const EvalArgs& a, const JhmiConsts* C) {
+  // the same limit on every call: threads with other bin counts share it
+  const cudaError_t e = cudaFuncSetAttribute(k_jhmi_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)jhmi_finalize_shared(kJhmiMaxBins));
+  if (e != cudaSuccess) return e;
+  return launch_chain(m, k_jhmi_finalize, (unsigned)jhmi_finalize_blocks(a.bins), kBlock,
+                      jhmi_finalize_shared(a.bins), a, C);
+}
+
+// Joint-histogram MI: the histogram pass, the PDF / value kernel, the derivative pass.
 static int enqueue_eval_jhmi(gb_metric* m, const EvalArgs& a, bool cd, bool deriv, bool device_params) {
   const int B = (int)m->bins;
   const JhmiConsts* C = reinterpret_cast<const JhmiConsts*>(m->d_jhmi.p);
@@ -1312,9 +1323,7 @@ static int enqueue_eval_jhmi(gb_metric* m, const EvalArgs& a, bool cd, bool deri
                 : launch_wave(m, k_jhmi_pass1_field<kGradImage, kMapFieldDense>, sh1, a, C);
     GB_CUDA(e);
     m->mark();
-    const size_t shf = sizeof(double) * (2 * B * B + 2 * B);
-    GB_CUDA(cudaFuncSetAttribute(k_jhmi_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shf));
-    GB_CUDA(launch_chain(m, k_jhmi_finalize, (unsigned)kJhmiFinalizeBlocks, kBlock, shf, a, C));
+    GB_CUDA(launch_jhmi_finalize(m, a, C));
     m->mark();
     if (deriv) {
       const size_t sh2 = sizeof(float) * (B * B + B);
@@ -1343,9 +1352,7 @@ static int enqueue_eval_jhmi(gb_metric* m, const EvalArgs& a, bool cd, bool deri
                : launch_wave(m, k_jhmi_pass1<kGradImage>, sh1, a, C));
   }
   m->mark();
-  const size_t shf = sizeof(double) * (2 * B * B + 2 * B);
-  GB_CUDA(cudaFuncSetAttribute(k_jhmi_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shf));
-  GB_CUDA(launch_chain(m, k_jhmi_finalize, (unsigned)kJhmiFinalizeBlocks, kBlock, shf, a, C));
+  GB_CUDA(launch_jhmi_finalize(m, a, C));
   m->mark();
   if (deriv && !bs) {
     const size_t sh2 = sizeof(float) * (B * B + B);
@@ -1364,9 +1371,7 @@ static int enqueue_eval_jhmi(gb_metric* m, const EvalArgs& a, bool cd, bool deri
 
 // The evaluation chains whose first kernel can zero the accumulators and whose host
 // call can stage its inputs and results through prologue / epilogue kernels.
-static bool chain_clears_in_prepare(const gb_metric* m) {
-  return (m->kind == GB_METRIC_MATTES || m->kind == GB_METRIC_MEAN_SQUARES) && !is_field(m) && m->nsamples > 0;
-}
+static bool chain_clears_in_prepare(const gb_metric* m) { return !is_field(m) && m->nsamples > 0; }
 
 // Enqueues one evaluation; results land in d_out = [value, nvalid, derivative...].
 // device_params: the parameters are in device memory (d_params), so the affine
@@ -1377,8 +1382,7 @@ int gb::enqueue_eval(gb_metric* m, const double* d_params, double* d_out, bool d
   cudaStream_t st = m->stream;
   EvalArgs a;
   fill_eval_args(m, a, d_params, d_out, deriv);
-  // MeanSquares / Mattes under an affine or B-spline transform with device parameters:
-  // the prepare kernel zeroes the accumulators (one node fewer, and the chain stays
+  // an affine or B-spline transform with device parameters: the prepare kernel zeroes the accumulators (one node fewer, and the chain stays
   // kernel-to-kernel); otherwise a memset unless the caller has cleared them
   if (device_params && chain_clears_in_prepare(m)) a.clear_acc = 1;
   else if (!acc_cleared || m->nsamples == 0) GB_CUDA(cudaMemsetAsync(m->d_acc.p, 0, m->acc_bytes, st));
@@ -1490,7 +1494,7 @@ __global__ void k_host_epilogue(const double* out, int n, const int* status, dou
 
 // The host call's device work: the constants (affine) or float4 nodes (B-spline)
 // up from pinned memory, the evaluation, value / derivative / status down into
-// pinned memory.  MeanSquares / Mattes under affine and B-spline transforms do it with
+// pinned memory.  Affine and B-spline transforms do it with
 // a prologue and an epilogue kernel (pinned memory read and written by the device), so
 // that every node of the chain is a kernel launched with a programmatic dependency;
 // the other chains with copies and a memset.
