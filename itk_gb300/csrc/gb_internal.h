@@ -250,6 +250,7 @@ struct gb_metric {
   cudaGraphExec_t host_exec[2] = {nullptr, nullptr};
   bool host_graph_tried[2] = {false, false};
   void drop_host_graphs();
+  bool eval_host_out = false;  // while an affine host call's chain is enqueued: results to pinned memory
 
   size_t device_bytes() const;  // all device buffers of the handle (gb_metric.cu)
   void release_buffers();       // frees them in the handle's stream order (gb_metric.cu)

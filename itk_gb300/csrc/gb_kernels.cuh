@@ -1652,7 +1652,8 @@ __device__ __forceinline__ void mattes_pass2_affine_body(const EvalArgs& a, VGri
   if (failed) {
     // a copy never completed: report, wait (bounded) for the copies still in flight, leave
     if (threadIdx.x == 0) {
-      atomicExch(a.status, GB_ERR_TIMEOUT);
+      // the same word from every block that gives up (it may lie in host memory)
+      *reinterpret_cast<volatile int*>(a.status) = GB_ERR_TIMEOUT;
       // the tile (or, before the loop, the histogram) whose wait ran out is not waited on again
       for (int u = looped ? t + 1 : 0; u < issued; ++u)
         mbar_wait(&full[u % kStreamStages], (unsigned)(u / kStreamStages) & 1u);
