@@ -23,23 +23,24 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "gb_device.cuh"
 #include "gb_internal.h"
 
 namespace gb {
 
-// IIR coefficients of one pass: N0..N3, D1..D4, M1..M4, and the steady states of the
-// causal and anticausal parts over a constant line of ones.
+// IIR coefficients of one pass: N0..N3, D1..D4, M1..M4, BN1..BN4, BM1..BM4.
 struct RGCoef {
-  double n[4], d[4], m[4], edge_n, edge_m;
+  double n[4], d[4], m[4], bn[4], bm[4];
 };
-// The same as one five-tap recursion in either direction (step s is element s of the
-// causal part, the element s before the last of the anticausal part):
-//   o_s = sum_{k=0..4} a_k x_{s-k} - sum_{k=1..4} d_k o_{s-k}.
-// Before the line, x is its first element x_0 and o its steady state x_0 edge.
+// The same in FP32 as one recursion that runs in either direction:
+//   o_s = sum_{k=0..3} a_k u_{s-k} - sum_{k=1..4} d_k o_{s-k},
+// u the inputs in the direction's order (causal), or those one element behind (anticausal).
+// Before the line, u is its first element, and an output that is not there yet enters as
+// that element times b_k.
 struct RGTaps {
-  float a[5], d[4], edge;
+  float a[4], d[4], b[4];
 };
 struct RGCoefF {
   RGTaps dir[2];  // causal, anticausal
@@ -104,8 +105,10 @@ static int rg_setup(double sigma, double spacing, int order, bool normalize_acro
   const double sn = c.n[0] + c.n[1] + c.n[2] + c.n[3];
   const double sm = c.m[0] + c.m[1] + c.m[2] + c.m[3];
   const double sdd = 1.0 + c.d[0] + c.d[1] + c.d[2] + c.d[3];
-  c.edge_n = sn / sdd;
-  c.edge_m = sm / sdd;
+  for (int k = 0; k < 4; ++k) {
+    c.bn[k] = c.d[k] * sn / sdd;
+    c.bm[k] = c.d[k] * sm / sdd;
+  }
   return GB_OK;
 }
 
@@ -113,12 +116,11 @@ static RGCoefF to_float(const RGCoef& c) {
   RGCoefF f;
   for (int k = 0; k < 4; ++k) {
     f.dir[0].a[k] = (float)c.n[k];
-    f.dir[1].a[k + 1] = (float)c.m[k];
+    f.dir[1].a[k] = (float)c.m[k];
     f.dir[0].d[k] = f.dir[1].d[k] = (float)c.d[k];
+    f.dir[0].b[k] = (float)c.bn[k];
+    f.dir[1].b[k] = (float)c.bm[k];
   }
-  f.dir[0].a[4] = f.dir[1].a[0] = 0.f;
-  f.dir[0].edge = (float)c.edge_n;
-  f.dir[1].edge = (float)c.edge_m;
   return f;
 }
 
@@ -148,28 +150,52 @@ __device__ __forceinline__ void copy_async_rows(float* dst, int inc, const float
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// The recursion's state, advanced one element at a time: what the elements so far add to
-// each of the next four outputs.  In this form an element's terms are independent of one
-// another, two multiply-adds separate an output from the next, and the terms of an output
-// are added oldest (and smallest) first, so the roundings stay small.  (Summed from the
-// last inputs and outputs instead, an output's nine terms ran one after another: 36 to 41
-// cycles an element, with one or two warps a scheduler to hide them.)
+// The recursion's state, advanced one element at a time: the last inputs and outputs.  Sums
+// and roundings are written out, so that a line's values do not depend on which kernel runs
+// it or on what the compiler fuses there.
 struct RGLine {
-  float n1, n2, n3, n4;
-  __device__ __forceinline__ void start(const RGTaps& c, float x0) {
-    const float o = x0 * c.edge;
-    n4 = fmaf(c.a[4], x0, -c.d[3] * o);
-    n3 = fmaf(-c.d[2], o, fmaf(c.a[3], x0, n4));
-    n2 = fmaf(-c.d[1], o, fmaf(c.a[2], x0, n3));
-    n1 = fmaf(-c.d[0], o, fmaf(c.a[1], x0, n2));
+  float p;               // the element behind (anticausal input)
+  float u1, u2, u3;      // the last inputs
+  float o1, o2, o3, o4;  // the last outputs
+  // a0 u + a1 u1 + a2 u2 + a3 u3 (repeated: the first two elements are one, their terms
+  // added the other way round)
+  __device__ __forceinline__ float inputs(const RGTaps& c, float u, bool repeated) const {
+    const float s = repeated ? fmaf(u, c.a[0], __fmul_rn(u1, c.a[1])) : fmaf(u1, c.a[1], __fmul_rn(u, c.a[0]));
+    return fmaf(u3, c.a[3], fmaf(u2, c.a[2], s));
   }
-  __device__ __forceinline__ float step(const RGTaps& c, float x) {
-    const float o = fmaf(c.a[0], x, n1);
-    n1 = fmaf(-c.d[0], o, fmaf(c.a[1], x, n2));
-    n2 = fmaf(-c.d[1], o, fmaf(c.a[2], x, n3));
-    n3 = fmaf(-c.d[2], o, fmaf(c.a[3], x, n4));
-    n4 = fmaf(-c.d[3], o, c.a[4] * x);
+  __device__ __forceinline__ float next(float u, float in, float t) {
+    const float o = __fsub_rn(in, t);
+    u3 = u2;
+    u2 = u1;
+    u1 = u;
+    o4 = o3;
+    o3 = o2;
+    o2 = o1;
+    o1 = o;
     return o;
+  }
+  // back: whether the recursion is anticausal
+  template <typename Back>
+  __device__ __forceinline__ float step(const RGTaps& c, float x, Back back) {
+    const float u = back ? p : x;
+    p = x;
+    const float t = fmaf(o4, c.d[3], fmaf(o3, c.d[2], fmaf(o1, c.d[0], __fmul_rn(o2, c.d[1]))));
+    return next(u, inputs(c, u, false), t);
+  }
+  // the line's first four elements
+  template <typename Back>
+  __device__ __forceinline__ void start(const RGTaps& c, const float (&x)[4], float (&o)[4], Back back) {
+    const float v = x[0], x1 = back ? x[0] : x[1], x2 = back ? x[1] : x[2], x3 = back ? x[2] : x[3];
+    u1 = u2 = u3 = v;
+    o1 = o2 = o3 = o4 = 0.f;
+    o[0] = next(v, inputs(c, v, true),
+                fmaf(v, c.b[3], fmaf(v, c.b[2], fmaf(v, c.b[0], __fmul_rn(v, c.b[1])))));
+    o[1] = next(x1, inputs(c, x1, back), fmaf(v, c.b[3], fmaf(v, c.b[2], fmaf(v, c.b[1], __fmul_rn(o1, c.d[0])))));
+    o[2] = next(x2, inputs(c, x2, false),
+                fmaf(v, c.b[3], fmaf(v, c.b[2], fmaf(o2, c.d[1], __fmul_rn(o1, c.d[0])))));
+    o[3] = next(x3, inputs(c, x3, false),
+                fmaf(v, c.b[3], fmaf(o3, c.d[2], fmaf(o2, c.d[1], __fmul_rn(o1, c.d[0])))));
+    p = x[3];
   }
 };
 
@@ -178,8 +204,9 @@ struct RGLine {
 // requested what it adds to the next ones.  The next group of inputs is requested before the present one's outputs are stored (the compiler cannot
 // move a load above a store to shared memory).
 constexpr int kRGRun = 8;
-template <typename Put>
-__device__ __forceinline__ void rg_run(RGLine& l, const RGTaps& c, const float*& x, int inc, int count, Put& put) {
+template <typename Back, typename Put>
+__device__ __forceinline__ void rg_run(RGLine& l, const RGTaps& c, Back back, const float*& x, int inc, int count,
+                                       Put& put) {
   float v[kRGRun];
   if (count >= kRGRun) {
 #pragma unroll
@@ -192,21 +219,34 @@ __device__ __forceinline__ void rg_run(RGLine& l, const RGTaps& c, const float*&
       for (int u = 0; u < kRGRun; ++u) w[u] = x[u * inc];
       x += kRGRun * inc;
 #pragma unroll
-      for (int u = 0; u < kRGRun; ++u) v[u] = l.step(c, v[u]);
+      for (int u = 0; u < kRGRun; ++u) v[u] = l.step(c, v[u], back);
       put(v);
       put.fetch(kRGRun);
 #pragma unroll
       for (int u = 0; u < kRGRun; ++u) v[u] = w[u];
     }
 #pragma unroll
-    for (int u = 0; u < kRGRun; ++u) v[u] = l.step(c, v[u]);
+    for (int u = 0; u < kRGRun; ++u) v[u] = l.step(c, v[u], back);
     put(v);
   }
   for (; count > 0; --count, x += inc) {
     put.fetch(1);
-    float one[1] = {l.step(c, *x)};
+    float one[1] = {l.step(c, *x, back)};
     put(one);
   }
+}
+
+// The first `count` (>= 4) elements, from the line's start.
+template <typename Back, typename Put>
+__device__ __forceinline__ void rg_begin(RGLine& l, const RGTaps& c, Back back, const float*& x, int inc, int count,
+                                         Put& put) {
+  float v[4], o[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) v[u] = x[u * inc];
+  l.start(c, v, o, back);
+  put(o);
+  x += 4 * inc;
+  rg_run(l, c, back, x, inc, count - 4, put);
 }
 
 // put of a recursion's first half: parked in shared memory.
@@ -305,18 +345,18 @@ __device__ __forceinline__ void rg_tile(const RGPass& a, float* tile, int o, int
   const float* x = tile + first;
   float* sum = tile + (1 + o) * size + first;
   RGLine s;
-  s.start(c, *x);
+  const std::integral_constant<bool, (DIR < 0)> back{};
   RGPark park{sum, kInc};
-  rg_run(s, c, x, kInc, half, park);
+  rg_begin(s, c, back, x, kInc, half, park);
   __syncthreads();
   sum += half * kInc;
   if (X) {
     RGAdd add{sum, kInc, scale};
-    rg_run(s, c, x, kInc, ln - half, add);
+    rg_run(s, c, back, x, kInc, ln - half, add);
   } else {
     RGStore store{sum, kInc, scale, a.out[o].p + base + (DIR < 0 ? ln - 1 - half : half) * a.step,
                   DIR * a.step, live};
-    rg_run(s, c, x, kInc, ln - half, store);
+    rg_run(s, c, back, x, kInc, ln - half, store);
   }
 }
 
@@ -367,8 +407,9 @@ __global__ void __launch_bounds__(64 * NOUT) k_rg_pass(RGPass a) {
   }
 }
 
-// The same for lines too long for a tile: one thread per line, the causal part through
-// the output image.
+// The same for lines too long for a tile, or too short to meet past both starts (under
+// kRGShort elements): one thread per line, the causal part through the output image.
+constexpr int kRGShort = 8;
 __global__ void __launch_bounds__(128) k_rg_long(RGPass a) {
   const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= a.lines) return;
@@ -377,11 +418,17 @@ __global__ void __launch_bounds__(128) k_rg_long(RGPass a) {
   float* y = a.out[0].p + base;
   const RGCoefF& c = a.out[0].c;
   RGLine s;
-  s.start(c.dir[0], __ldg(x));
-  for (int64_t i = 0; i < a.ln; ++i) y[i * a.step] = s.step(c.dir[0], __ldg(x + i * a.step));
-  s.start(c.dir[1], __ldg(x + (a.ln - 1) * a.step));
-  for (int64_t i = a.ln - 1; i >= 0; --i)
-    y[i * a.step] = (y[i * a.step] + s.step(c.dir[1], __ldg(x + i * a.step))) * a.out[0].scale;
+  float v[4], o[4];
+  for (int u = 0; u < 4; ++u) v[u] = __ldg(x + u * a.step);
+  s.start(c.dir[0], v, o, false);
+  for (int u = 0; u < 4; ++u) y[u * a.step] = o[u];
+  for (int64_t i = 4; i < a.ln; ++i) y[i * a.step] = s.step(c.dir[0], __ldg(x + i * a.step), false);
+  const int64_t last = a.ln - 1;
+  for (int u = 0; u < 4; ++u) v[u] = __ldg(x + (last - u) * a.step);
+  s.start(c.dir[1], v, o, true);
+  for (int u = 0; u < 4; ++u) y[(last - u) * a.step] = (y[(last - u) * a.step] + o[u]) * a.out[0].scale;
+  for (int64_t i = last - 4; i >= 0; --i)
+    y[i * a.step] = (y[i * a.step] + s.step(c.dir[1], __ldg(x + i * a.step), true)) * a.out[0].scale;
 }
 
 // Largest dynamic shared memory of a block.
@@ -419,7 +466,7 @@ static cudaError_t rg_pass(cudaStream_t st, const float* in, const int64_t size[
                            int nout) {
   RGPass a = rg_lines(in, size, axis);
   const size_t shared = (1 + nout) * rg_tile_bytes(axis == 0, a.ln);
-  if (shared > kRGMaxShared) {
+  if (shared > kRGMaxShared || a.ln < kRGShort) {
     if (nout == 2) {
       const cudaError_t e = rg_pass(st, in, size, axis, out, 1);
       return e != cudaSuccess ? e : rg_pass(st, in, size, axis, out + 1, 1);
@@ -532,20 +579,20 @@ __global__ void __launch_bounds__(96) k_rg_grad_z(RGGradZ a) {
   __syncwarp();  // a warp's recursions read what the same warp has copied
   RGTaps c;  // this lane's direction, by selection: no divergent copies
 #pragma unroll
-  for (int k = 0; k < 5; ++k) c.a[k] = back ? a.out[comp].c.dir[1].a[k] : a.out[comp].c.dir[0].a[k];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) c.d[k] = a.out[comp].c.dir[0].d[k];
-  c.edge = back ? a.out[comp].c.dir[1].edge : a.out[comp].c.dir[0].edge;
+  for (int k = 0; k < 4; ++k) {
+    c.a[k] = back ? a.out[comp].c.dir[1].a[k] : a.out[comp].c.dir[0].a[k];
+    c.b[k] = back ? a.out[comp].c.dir[1].b[k] : a.out[comp].c.dir[0].b[k];
+    c.d[k] = a.out[comp].c.dir[0].d[k];
+  }
   const float scale = a.out[comp].scale;
   const float* x = xs;
   RGLine s;
-  s.start(c, *x);
   RGPark park{xs + size, kInc};
-  rg_run(s, c, x, kInc, half, park);
+  rg_begin(s, c, back != 0, x, kInc, half, park);
   __syncwarp();
   if (ln & 1) {  // the middle element, the last row, for both
     float* m = xs - lane + size + (ln - 1) * kRGzLines + line;
-    const float v = s.step(c, xs[(ln - 1) * kRGzLines - lane + line]);
+    const float v = s.step(c, xs[(ln - 1) * kRGzLines - lane + line], back != 0);
     if (!back) *m = v;
     __syncwarp();
     if (back) *m = (*m + v) * scale;
@@ -554,7 +601,7 @@ __global__ void __launch_bounds__(96) k_rg_grad_z(RGGradZ a) {
   const int last = (half - 1) * kInc - lane + (lane ^ kRGzLines);
   x = xs + last;
   RGAdd add{xs + size + last, -kInc, scale};
-  rg_run(s, c, x, -kInc, half, add);
+  rg_run(s, c, back != 0, x, -kInc, half, add);
   __syncthreads();
   const float *g0 = tile + size, *g1 = tile + 3 * size, *g2 = tile + 5 * size, *v0 = tile + 6 * size;
   constexpr int kOut = 8;  // rows read together
@@ -634,7 +681,7 @@ int gradient_rg_device(cudaStream_t st, const float* in, const int64_t size[3], 
   if (e == cudaSuccess) e = rg_pass(st, A, size, 1, oy, 1);
   if (e == cudaSuccess) e = rg_pass(st, B, size, 1, oy + 1, 2);
   const size_t shared = sizeof(float) * rgz_array((int)size[2]) * (out4 ? 7 : 6);
-  if (shared <= kRGMaxShared) {
+  if (shared <= kRGMaxShared && size[2] >= kRGShort) {
     RGGradZ z;
     memset(&z, 0, sizeof(z));
     z.in[0] = C;
