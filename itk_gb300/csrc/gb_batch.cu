@@ -3,13 +3,13 @@
 // Every registration keeps its own metric handle (images, samples, caches,
 // accumulators) and optimizer state in HBM.  One optimizer iteration of all of
 // them is one launch per phase:
-//   k_batch_clear    accumulators of every running registration
-//   k_batch_prepare  per-evaluation transform constants (22 FP64 entries each)
+//   (k_batch_clear and k_batch_prepare, before the first iteration: accumulators and
+//   transform constants of every running registration)
 //   k_batch_msq      MeanSquares value and derivative      } blocks of all
 //   k_batch_pass1    Mattes joint histogram                 } registrations in
 //                                                           } one grid, each
 //   k_batch_pass2    Mattes value and derivative            } block one virtual
-//   k_batch_step     AdvanceOneStep (one block per registration)   block of one
+//   k_batch_step     AdvanceOneStep, the next evaluation readied   block of one
 // captured once as a CUDA graph and relaunched per iteration.     registration
 // A registration's blocks are a fixed function of its own sample count and the
 // samples-per-block setting (chosen by gb_batch_autotune), so its results are
@@ -99,13 +99,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_pass2(const EvalArgs* __res
   mattes_pass2_affine_body<false>(sa, VGrid{w.y, w.z});
 }
 
-// AdvanceOneStep of one registration per block (step_block), one warp for the
-// 12 affine parameters.
-__global__ void __launch_bounds__(32) k_batch_step(const StepArgs* __restrict__ steps) {
+// AdvanceOneStep of one registration per block (step_small), and its next evaluation readied.
+__global__ void __launch_bounds__(kStepBlock) k_batch_step(const StepArgs* __restrict__ steps,
+                                                           const EvalArgs* __restrict__ regs) {
+  __shared__ double p_sh[32];
   griddep_wait();
   const StepArgs s = steps[blockIdx.x];
   griddep_launch_dependents();
-  step_block<32>(s);
+  if (step_small(s, p_sh)) prepare_next(regs[blockIdx.x], p_sh);
 }
 
 // ---------------------------------------------------------------------------
@@ -201,8 +202,9 @@ static __device__ __noinline__ void item_pass1(const EvalArgs& a, VGrid vg, bool
 }
 static __device__ __noinline__ void item_pass2(const EvalArgs& a, VGrid vg) { mattes_pass2_affine_body<false>(a, vg); }
 static __device__ __noinline__ void item_step(const StepArgs* steps, int r) {
+  __shared__ double p_sh[32];
   const StepArgs sarg = steps[r];
-  step_block<32>(sarg);  // every thread: its barrier is the block's
+  step_small(sarg, p_sh);  // every thread: its barrier is the block's
 }
 static __device__ __noinline__ void item_prepare(const EvalArgs* regs, int r, int e) {
   const EvalArgs& a = regs[r];
@@ -413,12 +415,24 @@ int64_t vblocks(int64_t n, int64_t spb) {
   return std::max<int64_t>(1, std::min<int64_t>(std::max((n + spb - 1) / spb, spread), kMaxBlocks));
 }
 
-// One iteration (or, with step = false, one evaluation of every running registration).
-int enqueue_iteration(gb_batch* b, bool step) {
+// Cleared accumulators and constants of every running registration.
+int enqueue_prepare_all(gb_batch* b) {
   const unsigned n = (unsigned)b->active.size();
   cudaStream_t st = b->stream;
   GB_B_CUDA(launch_dep(st, k_batch_clear, n, kBlock, 0, (const ClearItem*)b->d_clear.p));
   GB_B_CUDA(launch_dep(st, k_batch_prepare, n * kConstEntries, 32, 0, (const EvalArgs*)b->d_eval.p));
+  return GB_OK;
+}
+
+// One iteration, readied by enqueue_prepare_all or by the iteration before it (or, with
+// step = false, one evaluation of every running registration).
+int enqueue_iteration(gb_batch* b, bool step) {
+  const unsigned n = (unsigned)b->active.size();
+  cudaStream_t st = b->stream;
+  if (!step) {
+    const int rc = enqueue_prepare_all(b);
+    if (rc) return rc;
+  }
   const EvalArgs* regs = b->d_eval.p;
   const int4* w = b->d_work.p;
   if (b->gcnt[kGrpMsqImage])
@@ -435,7 +449,7 @@ int enqueue_iteration(gb_batch* b, bool step) {
                          regs, w + b->goff[kGrpP1CD]));
   if (b->gcnt[kGrpP2])
     GB_B_CUDA(launch_dep(st, k_batch_pass2, (unsigned)b->gcnt[kGrpP2], kBlock, b->smem2, regs, w + b->goff[kGrpP2]));
-  if (step) GB_B_CUDA(launch_dep(st, k_batch_step, n, 32, 0, (const StepArgs*)b->d_step.p));
+  if (step) GB_B_CUDA(launch_dep(st, k_batch_step, n, kStepBlock, 0, (const StepArgs*)b->d_step.p, regs));
   return GB_OK;
 }
 
@@ -747,6 +761,10 @@ extern "C" int gb_batch_run(gb_batch* b, int64_t max_iterations, int64_t* runnin
     }
     const int n = (int)b->active.size();
     if (n == 0) break;
+    if (!b->persistent) {  // on every call: the handles may have been evaluated in between
+      const int rc = enqueue_prepare_all(b);
+      if (rc) return rc;
+    }
     // Two batches of iterations in flight: batch j + 1 is enqueued before batch j's
     // halt words are read.  Stopped registrations stay in the tables (their blocks
     // return at once) until they hold half of the work items, then the tables are

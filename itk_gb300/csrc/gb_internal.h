@@ -162,6 +162,7 @@ inline void copy_parallel(void* dst, const void* src, size_t bytes) {
 namespace gb {
 int enqueue_eval(gb_metric* m, const double* d_params, double* d_out, bool deriv, bool device_params,
                  bool acc_cleared = false);
+int enqueue_prepare(gb_metric* m, const double* d_params);  // an affine evaluation's first kernel by itself
 struct EvalArgs;
 void batch_eval_args(gb_metric* m, EvalArgs& a);
 }

@@ -208,6 +208,16 @@ __host__ __device__ inline void affine_consts(const double* p, const double cent
   for (int e = 0; e < kConstEntries; ++e) affine_const_entry(e, p, center, m_p2i, m_origin, dom2phys, dom_origin, K);
 }
 
+// The same by the lanes of one warp, for parameters p that change while centre and domain
+// stay: lane e the map's entry e (matrix entries 0-8, offset rows 9-11).  The Jacobian terms
+// do not depend on p, and M^T and P2I M are not read under an affine transform.
+__device__ __forceinline__ void affine_map_warp(const double* p, const double center[3], const double m_p2i[9],
+                                                const double m_origin[3], const double* dom2phys,
+                                                const double* dom_origin, EvalConsts& K) {
+  const int e = threadIdx.x & 31;
+  if (e < 12) affine_const_entry(e, p, center, m_p2i, m_origin, dom2phys, dom_origin, K);
+}
+
 struct EvalArgs {
   const float4* __restrict__ samples;
   int64_t n;
@@ -296,6 +306,21 @@ __device__ __forceinline__ void clear_accumulators(const EvalArgs& a) {
     a.acc[k] = make_uint4(0u, 0u, 0u, 0u);
 }
 
+#endif  // GB_KERNELS_HELPERS_ONLY
+
+// What the next affine evaluation's prepare kernel would do, by the block that has just
+// taken the optimizer's step (32 threads form the map from p, the others zero the
+// accumulators): a launch less per iteration.
+__device__ __forceinline__ void prepare_next(const EvalArgs& a, const double* p) {
+  if (threadIdx.x < 32) {
+    affine_map_warp(p, a.center, a.m_p2i, a.m_origin, a.dense ? a.v_i2p : nullptr, a.v_origin,
+                    *const_cast<EvalConsts*>(a.consts));
+  } else {
+    for (int k = threadIdx.x - 32; k < a.acc_words; k += blockDim.x - 32) a.acc[k] = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
+#ifndef GB_KERNELS_HELPERS_ONLY
 __global__ void k_prepare_affine(EvalArgs a, EvalConsts* out) {
   griddep_wait();
   if (halted(a)) return;

@@ -123,13 +123,14 @@ static int full_wave(const gb_metric* m, K kernel, size_t smem, int64_t n) {
   return grid_for(m, n, per_sm);
 }
 
-// The same with the blocks evened out: every block runs the same number of iterations
-// (64^3 dense: 512 blocks of two 256-sample iterations, not 608 of one or two; 20 -> 17 us).
+// MeanSquares, affine: one full wave, of three blocks per SM below four iterations a block
+// (64^3 dense: 456 blocks 16.6 us, 512 or 608 17.6 and 20.5: the reduction's tail grows
+// with the blocks), else of all that fit (four; 256x256x200 dense 195 -> 181 us).
 template <typename K>
-static int even_wave(const gb_metric* m, K kernel, size_t smem, int64_t n) {
-  const int64_t tiles = std::max<int64_t>(1, (n + kBlock - 1) / kBlock), cap = full_wave(m, kernel, smem, n);
-  const int64_t each = (tiles + cap - 1) / cap;
-  return (int)((tiles + each - 1) / each);
+static int msq_blocks(const gb_metric* m, K kernel, int64_t n) {
+  const int64_t tiles = (n + kBlock - 1) / kBlock, three = 3 * (int64_t)m->ctx->sm_count;
+  const int wave = full_wave(m, kernel, 0, n);
+  return tiles <= 4 * three ? (int)std::min<int64_t>(wave, three) : wave;
 }
 
 static bool is_bspline(const gb_metric* m) {
@@ -1381,7 +1382,8 @@ static bool chain_clears_in_prepare(const gb_metric* m) { return !is_field(m) &&
 // Enqueues one evaluation; results land in d_out = [value, nvalid, derivative...].
 // device_params: the parameters are in device memory (d_params), so the affine
 // constants or the B-spline nodes are formed on the device; otherwise the host
-// has uploaded them.
+// has uploaded them.  acc_cleared: the accumulators are zero, and under an affine transform
+// the constants are in place as well.
 int gb::enqueue_eval(gb_metric* m, const double* d_params, double* d_out, bool deriv, bool device_params,
                      bool acc_cleared) {
   cudaStream_t st = m->stream;
@@ -1389,9 +1391,9 @@ int gb::enqueue_eval(gb_metric* m, const double* d_params, double* d_out, bool d
   fill_eval_args(m, a, d_params, d_out, deriv);
   // an affine or B-spline transform with device parameters: the prepare kernel zeroes the accumulators (one node fewer, and the chain stays
   // kernel-to-kernel); otherwise a memset unless the caller has cleared them
-  if (device_params && chain_clears_in_prepare(m)) a.clear_acc = 1;
+  if (device_params && !acc_cleared && chain_clears_in_prepare(m)) a.clear_acc = 1;
   else if (!acc_cleared || m->nsamples == 0) GB_CUDA(cudaMemsetAsync(m->d_acc.p, 0, m->acc_bytes, st));
-  if (device_params && !is_bspline(m) && !is_field(m))
+  if (device_params && !acc_cleared && !is_bspline(m) && !is_field(m))
     GB_CUDA(launch_chain(m, k_prepare_affine, kConstEntries, 32, 0, a, m->d_consts.p));
   if (m->nsamples == 0) {
     // no valid fixed sample at all: every point is invalid
@@ -1424,7 +1426,7 @@ int gb::enqueue_eval(gb_metric* m, const double* d_params, double* d_out, bool d
   if (m->kind == GB_METRIC_MEAN_SQUARES) {
     auto kernel = a.fp_res > 0.0 ? (cd ? k_msq_affine<kGradCentralDifference, true> : k_msq_affine<kGradImage, true>)
                                  : (cd ? k_msq_affine<kGradCentralDifference> : k_msq_affine<kGradImage>);
-    GB_CUDA(launch_chain(m, kernel, (unsigned)even_wave(m, kernel, 0, m->nsamples), kBlock, 0, a));
+    GB_CUDA(launch_chain(m, kernel, (unsigned)msq_blocks(m, kernel, m->nsamples), kBlock, 0, a));
     m->mark();
     return GB_OK;
   }
@@ -1442,6 +1444,14 @@ int gb::enqueue_eval(gb_metric* m, const double* d_params, double* d_out, bool d
     GB_CUDA(launch_pass2(m, a));
     m->mark();
   }
+  return GB_OK;
+}
+
+int gb::enqueue_prepare(gb_metric* m, const double* d_params) {
+  EvalArgs a;
+  fill_eval_args(m, a, d_params, m->d_out.p, true);
+  a.clear_acc = 1;
+  GB_CUDA(launch_chain(m, k_prepare_affine, kConstEntries, 32, 0, a, m->d_consts.p));
   return GB_OK;
 }
 

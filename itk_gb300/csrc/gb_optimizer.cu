@@ -26,6 +26,7 @@
 // of the result, so the two can differ in the last bit of ||g|| and g . g_prev.
 // Every other operation is the reference's, rounding for rounding (FP64, no
 // contraction).
+#define GB_KERNELS_HELPERS_ONLY
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -37,6 +38,7 @@
 
 #include "gb_device.cuh"
 #include "gb_internal.h"
+#include "gb_kernels.cuh"
 #include "gb_step.cuh"
 
 namespace gb {
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(kStepBlock) k_step_reduce(StepArgs s) {
   }
   if (lane != 0) return;
   S->ticket = 0u;
-  step_decide(s, S, status, x, y);
+  step_decide(s, *S, status, __ldcg(s.out), x, y);
 }
 
 __global__ void __launch_bounds__(kStepBlock) k_step_apply(StepArgs s) {
@@ -106,12 +108,13 @@ __global__ void __launch_bounds__(kStepBlock) k_step_apply(StepArgs s) {
   for (long long j = (long long)blockIdx.x * kStepBlock + threadIdx.x; j < s.P; j += stride) step_apply(s, S, act, j);
 }
 
-// The whole step of a registration with at most 32 parameters in one warp
-// (reduce, decide and apply in one launch).
-__global__ void __launch_bounds__(32) k_step_single(StepArgs s) {
+// The whole step of a registration with at most 32 parameters in one block (reduce, decide
+// and apply in one launch); with `prepare` it readies the next affine evaluation too.
+__global__ void __launch_bounds__(kStepBlock) k_step_single(StepArgs s, EvalArgs a, int prepare) {
+  __shared__ double p_sh[32];
   griddep_wait();
   griddep_launch_dependents();
-  step_block<32>(s);
+  if (step_small(s, p_sh) && prepare) prepare_next(a, p_sh);
 }
 
 // The loop ran out of iterations without another stop: MAXIMUM_NUMBER_OF_ITERATIONS.
@@ -154,22 +157,19 @@ static cudaError_t launch_dependent(cudaStream_t st, void (*kernel)(KArgs...), u
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// One optimizer iteration: the evaluation, then the step (one warp for at most 32
+// An affine loop's step kernel readies the next evaluation (prepare_next).
+static bool step_prepares(const gb_metric* m) { return m->tkind == GB_TRANSFORM_AFFINE && m->nsamples > 0; }
+
+// One optimizer iteration: the evaluation, then the step (one block for at most 32
 // parameters, else the multi-block reduce and apply).
 static int enqueue_iteration(gb_metric* m, const StepArgs& a, unsigned blocks) {
-  int rc = enqueue_eval(m, m->d_params.p, m->d_out.p, true, true);
+  const bool prepared = step_prepares(m);
+  int rc = enqueue_eval(m, m->d_params.p, m->d_out.p, true, true, prepared);
   if (rc) return rc;
   if (a.P <= 32) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1);
-    cfg.blockDim = dim3(32);
-    cfg.stream = m->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    GB_OPT_CUDA(cudaLaunchKernelEx(&cfg, k_step_single, a));
+    EvalArgs ea;
+    batch_eval_args(m, ea);
+    GB_OPT_CUDA(launch_dependent(m->stream, k_step_single, 1u, a, ea, prepared ? 1 : 0));
     return GB_OK;
   }
   GB_OPT_CUDA(launch_dependent(m->stream, k_step_reduce, blocks, a));
@@ -342,6 +342,10 @@ extern "C" int gb_metric_optimize_regular_step(gb_metric* m, const gb_regular_st
   m->profiling = false;
   m->eval_halt = &S->halt;
   const int64_t N = cfg->number_of_iterations;
+  if (step_prepares(m) && N > 0) {  // the first evaluation's constants and cleared accumulators
+    rc = enqueue_prepare(m, m->d_params.p);
+    if (rc) return rc;
+  }
 
   // one iteration as a CUDA graph (no graph when there is nothing to evaluate:
   // that path stages its result from host memory)

@@ -26,7 +26,7 @@ constexpr int kStepMaxBlocks = 256;  // blocks of the multi-block step (grid-str
 enum { kActNone = 0, kActStep = 1, kActRestoreBest = 2 };
 enum { kRunning = -1 };
 
-struct OptState {
+struct OptVars {
   double relaxation;   // m_CurrentLearningRateRelaxation
   double value;        // m_CurrentMetricValue
   double best_value;   // m_CurrentBestValue
@@ -39,6 +39,9 @@ struct OptState {
   int status;          // metric status of the last evaluation
   int action;          // what the apply phase does this iteration
   int save_best;       // the apply phase copies the new position to the best parameters
+};
+
+struct OptState : OptVars {
   unsigned ticket;
   double part[kStepMaxBlocks][4];  // per block: (hi, lo) of ||g||^2 and of g . g_prev
 };
@@ -77,7 +80,7 @@ __device__ __forceinline__ DD dd_shfl_down(DD v, int off) {
   return {__shfl_down_sync(0xffffffffu, v.hi, off), __shfl_down_sync(0xffffffffu, v.lo, off)};
 }
 
-// Sum over a block of NT threads (32 or kStepBlock) in a fixed order (lane tree,
+// Sum over a block of NT threads in a fixed order (lane tree,
 // then warp tree); the result is in thread 0.
 template <int NT = kStepBlock>
 __device__ __forceinline__ void block_dd2(DD& x, DD& y) {
@@ -90,7 +93,6 @@ __device__ __forceinline__ void block_dd2(DD& x, DD& y) {
       y = dd_add(y, oy);
     }
   }
-  if constexpr (NT == 32) return;
   __shared__ DD sx[NT / 32], sy[NT / 32];
   if (lane == 0) {
     sx[w] = x;
@@ -118,53 +120,52 @@ __device__ __forceinline__ bool metric_error(const StepArgs& s, int status) {
 
 // StopOptimization (itkGradientDescentOptimizerv4.hxx:59-68): with return-best,
 // the value becomes the best value and the apply phase restores the best parameters.
-__device__ __forceinline__ void stop_here(const StepArgs& s, OptState* S, int cond) {
-  S->stop = cond;
-  S->halt = 1;
+__device__ __forceinline__ void stop_here(const StepArgs& s, OptVars& S, int cond) {
+  S.stop = cond;
+  S.halt = 1;
   if (s.return_best) {
-    S->value = S->best_value;
-    S->action = kActRestoreBest;
+    S.value = S.best_value;
+    S.action = kActRestoreBest;
   } else {
-    S->action = kActNone;
+    S.action = kActNone;
   }
 }
 
-// The decisions of one iteration (one thread): the metric's status, ||g||^2 = x
-// and g . g_prev = y summed over all parameters.
-__device__ __forceinline__ void step_decide(const StepArgs& s, OptState* S, int status, DD x, DD y) {
-  S->status = status;
-  S->save_best = 0;
-  const double value = __ldcg(s.out);
-  S->value = value;
+// The decisions of one iteration: the metric's status and value, ||g||^2 = x and
+// g . g_prev = y summed over all parameters.
+__device__ __forceinline__ void step_decide(const StepArgs& s, OptVars& S, int status, double value, DD x, DD y) {
+  S.status = status;
+  S.save_best = 0;
+  S.value = value;
   if (metric_error(s, status)) {  // the metric threw: COSTFUNCTION_ERROR, no iteration counted
     stop_here(s, S, GB_STOP_COSTFUNCTION_ERROR);
     return;
   }
   const double mag = sqrt(__dadd_rn(x.hi, x.lo));
-  S->grad_mag = mag;
+  S.grad_mag = mag;
   if (mag < s.grad_tol) {
     stop_here(s, S, GB_STOP_GRADIENT_MAGNITUDE_TOLERANCE);
-    S->iteration += 1;
+    S.iteration += 1;
     return;
   }
   const double sp = __dadd_rn(y.hi, y.lo);
-  double relax = S->relaxation;
+  double relax = S.relaxation;
   if (sp < 0.0) relax = __dmul_rn(relax, s.relaxation_factor);
-  S->relaxation = relax;
+  S.relaxation = relax;
   const double step = __dmul_rn(relax, s.learning_rate);
-  S->step_length = step;
+  S.step_length = step;
   if (step < s.min_step) {
     stop_here(s, S, GB_STOP_STEP_TOO_SMALL);
-    S->iteration += 1;
+    S.iteration += 1;
     return;
   }
-  S->inv_mag = 1.0 / mag;
-  S->action = kActStep;
-  if (s.return_best && value < S->best_value) {
-    S->best_value = value;
-    S->save_best = 1;
+  S.inv_mag = 1.0 / mag;
+  S.action = kActStep;
+  if (s.return_best && value < S.best_value) {
+    S.best_value = value;
+    S.save_best = 1;
   }
-  S->iteration += 1;
+  S.iteration += 1;
 }
 
 // ModifyGradientByScalesOverSubRange for parameter j: g = derivative / scale,
@@ -193,50 +194,77 @@ __device__ __forceinline__ void step_apply(const StepArgs& s, const OptState* S,
   if (__ldcg(&S->save_best)) s.best[j] = p;
 }
 
-// One registration's whole step in one block of NT threads: the compensated sums,
-// the decisions, the update, then the NumberOfIterations stop that the reference
-// checks at the top of its next loop pass (itkGradientDescentOptimizerv4.hxx:82-89).
-// Called by every thread of the block; threads from NT on take part only in its
-// barrier (the batched engine's persistent kernel runs the step in larger blocks).
-template <int NT>
-__device__ __forceinline__ void step_block(const StepArgs& s) {
-  OptState* S = s.st;
-  // thread 0 reads the halt word for the block: thread 0 itself may set it below,
-  // and every thread must take the same branch (the block's barrier follows)
-  __shared__ int halted_s;
-  if (threadIdx.x == 0) halted_s = __ldcg(&S->halt);
-  __syncthreads();
-  if (halted_s) return;
-  const int status = __ldcg(s.status);
-  const bool err = metric_error(s, status);
-  const bool mine = (int)threadIdx.x < NT;
-  DD q = {0.0, 0.0}, r = {0.0, 0.0};
-  if (!err && mine)
-    for (long long j = threadIdx.x; j < s.P; j += NT) {
-      double qq, rr;
-      step_terms(s, j, qq, rr);
-      q = dd_add(q, DD{qq, 0.0});
-      r = dd_add(r, DD{rr, 0.0});
+// The whole step of a registration with at most 32 parameters, by the first warp of a
+// block: the compensated sums, the decisions, the update, then the NumberOfIterations stop
+// that the reference checks at the top of its next loop pass
+// (itkGradientDescentOptimizerv4.hxx:82-89).  A parameter per lane; everything it reads is
+// requested at once and stays in registers (a round trip to L2 is what a step waits for).
+// Every thread of the block calls it; false once the loop has stopped.  p_sh[0, P): the new
+// parameters.
+__device__ __forceinline__ bool step_small(const StepArgs& s, double* p_sh) {
+  __shared__ int running_s;
+  if (threadIdx.x < 32) {
+    const int j = threadIdx.x, P = (int)s.P;
+    OptState* S = s.st;
+    const bool mine = j < P;
+    const int halt = __ldcg(&S->halt), status = __ldcg(s.status);
+    const double value = __ldcg(s.out);
+    OptVars V;
+    V.relaxation = __ldcg(&S->relaxation);
+    V.best_value = __ldcg(&S->best_value);
+    V.grad_mag = __ldcg(&S->grad_mag);
+    V.step_length = __ldcg(&S->step_length);
+    V.inv_mag = __ldcg(&S->inv_mag);
+    V.iteration = __ldcg(&S->iteration);
+    V.stop = kRunning;
+    V.halt = 0;
+    const double is = mine ? __ldg(s.inv_scales + j) : 0.0, d = mine ? __ldcg(s.out + 2 + j) : 0.0;
+    const double prev = mine ? __ldcg(s.prev + j) : 0.0;
+    double p = mine ? __ldcg(s.params + j) : 0.0, best = mine && s.return_best ? __ldcg(s.best + j) : 0.0;
+    if (halt == 0) {
+      const bool err = metric_error(s, status);
+      // ModifyGradientByScalesOverSubRange: g = derivative / scale, g_prev / scale
+      const double g = __dmul_rn(d, is), gp = __dmul_rn(prev, is);
+      DD x = {err || !mine ? 0.0 : __dmul_rn(g, g), 0.0}, y = {err || !mine ? 0.0 : __dmul_rn(g, gp), 0.0};
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        if (off >= P) continue;  // those lanes add exact zeros
+        const DD ox = dd_shfl_down(x, off), oy = dd_shfl_down(y, off);
+        if (j < off) {
+          x = dd_add(x, ox);
+          y = dd_add(y, oy);
+        }
+      }
+      x = {__shfl_sync(0xffffffffu, x.hi, 0), __shfl_sync(0xffffffffu, x.lo, 0)};
+      y = {__shfl_sync(0xffffffffu, y.hi, 0), __shfl_sync(0xffffffffu, y.lo, 0)};
+      step_decide(s, V, status, value, x, y);
+      const int act = V.action;
+      const bool at_max = !V.halt && V.iteration >= s.max_iterations;
+      // ModifyGradientByLearningRateOverSubRange, then UpdateTransformParameters(g, 1 / ||g||),
+      // or the return-best restore
+      if (act == kActStep) {
+        const double glr = __dmul_rn(__dmul_rn(g, V.relaxation), s.learning_rate);
+        p = __dadd_rn(p, __dmul_rn(glr, V.inv_mag));
+        if (V.save_best) best = p;
+        if (mine) {
+          s.prev[j] = glr;
+          if (V.save_best) s.best[j] = p;
+        }
+      }
+      if (act == kActRestoreBest || (at_max && s.return_best)) p = best;
+      if (mine) s.params[j] = p;
+      if (at_max) {
+        V.stop = GB_STOP_MAXIMUM_NUMBER_OF_ITERATIONS;
+        V.halt = 1;
+        if (s.return_best) V.value = V.best_value;
+      }
+      if (j == 0) *static_cast<OptVars*>(S) = V;
     }
-  block_dd2<NT>(q, r);
-  __shared__ int act, fin_max;
-  if (threadIdx.x == 0) {
-    step_decide(s, S, status, q, r);
-    int fm = 0;
-    if (!S->halt && S->iteration >= s.max_iterations) {
-      S->stop = GB_STOP_MAXIMUM_NUMBER_OF_ITERATIONS;
-      S->halt = 1;
-      fm = 1;
-      if (s.return_best) S->value = S->best_value;
-    }
-    act = S->action;
-    fin_max = fm;
+    if (mine) p_sh[j] = p;
+    if (j == 0) running_s = halt == 0 && V.halt == 0 ? 1 : 0;
   }
   __syncthreads();
-  for (long long j = threadIdx.x; mine && j < s.P; j += NT) {
-    step_apply(s, S, act, j);
-    if (fin_max && s.return_best) s.params[j] = __ldcg(s.best + j);
-  }
+  return running_s != 0;
 }
 
 // Host side (gb_optimizer.cu).  opt_setup: StartOptimization of one registration
