@@ -274,3 +274,35 @@ def test_mattes_histogram_with_few_and_many_keys(levels, n):
     assert_value_close(v, r["value"], atol=MATTES_VALUE_ATOL)
     assert_deriv_close(d, r["derivative"])
     assert m.GetValue() == v
+
+
+@pytest.mark.parametrize("virtual", [True, False])
+@pytest.mark.parametrize("turned", [False, True])
+@pytest.mark.parametrize("size", [(9, 8, 7), (33, 1, 5), (300, 40, 3)])
+@pytest.mark.parametrize("origin", [0.0, -700.3])
+def test_fixed_samples_next_to_every_threshold(size, turned, virtual, origin):
+    """Points on and next to voxel centres, half-way planes and buffer edges: which of them count,
+    and the mean square of their interpolated values, as FP64 has them (a zero moving image)."""
+    rng = np.random.default_rng(7)
+    direction = np.eye(3)
+    if turned:
+        c, s = np.cos(0.4), np.sin(0.4)
+        direction = np.array([[c, -s, 0.0], [s, c, 0.0], [0.0, 0.0, 1.0]]) @ np.array(
+            [[1.0, 0.0, 0.0], [0.0, c, -s], [0.0, s, c]])
+    fixed = Image(rng.normal(0.0, 50.0, size[::-1]), spacing=(0.7, 1.0, 2.5), origin=(origin, origin, origin),
+                  direction=direction)
+    fixed.array[:, :, : size[0] // 3] = 0.0  # a flat part
+    span = 4.0 * max(np.linalg.norm(np.array(size) * fixed.spacing), 1.0)
+    moving = Image(np.zeros((2, 2, 2), np.float32), spacing=(span,) * 3, origin=(origin - span / 2,) * 3)
+    n = np.array(size)
+    idx = rng.integers(-1, n + 1, size=(6000, 3)) + rng.choice([-0.5, 0.0, 0.5, 0.25], size=(6000, 3))
+    idx = idx + rng.choice([0.0, 1e-7, -1e-6, 1e-5, 3e-3], size=(6000, 3))
+    idx[3000:] = rng.uniform(-1.0, n, size=(3000, 3))
+    m33 = direction * fixed.spacing
+    pts = (idx @ m33.T + fixed.origin).astype(np.float32)
+    T = AffineTransform()
+    m = make_metric("msq", fixed, moving, T, points=pts, points_virtual=virtual)
+    v = m.GetValue()
+    r = run_oracle("msq", fixed, moving, T, points=pts, compute_derivative=False)
+    assert m.GetNumberOfValidPoints() == r["nvalid"]
+    assert_value_close(v, r["value"], rtol=1e-6)  # values rounded to FP32 once, sums in more
