@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -118,6 +119,7 @@ void shrink_geometry(const int64_t size[3], const double spacing[3], const doubl
                      const int64_t factors[3], int64_t out_size[3], double out_spacing[3], double out_origin[3]);
 
 struct OptState;  // device optimizer state (gb_optimizer.cu)
+size_t opt_state_bytes();
 
 // body(k0, k1) over [0, n) split across the host's threads (at most 16, at least
 // `grain` items each); the caller's thread runs whatever no new thread could take.
@@ -167,9 +169,20 @@ struct EvalArgs;
 void batch_eval_args(gb_metric* m, EvalArgs& a);
 }
 
+// A metric handle's stream and block of pinned memory.  The block costs 110 us to get and as
+// much to give back, a tenth of a small registration each; a context keeps the last
+// kIdleKits of them that its handles gave back, idle and synchronized, until it is destroyed.
+struct HandleKit {
+  cudaStream_t stream = nullptr;
+  unsigned char* block = nullptr;
+};
+
 struct gb_ctx {
   int device = 0;
   int sm_count = 0;
+  static constexpr size_t kIdleKits = 16;
+  std::mutex kits_lock;
+  std::vector<HandleKit> kits;
 };
 
 struct gb_metric {
@@ -192,7 +205,8 @@ struct gb_metric {
   int grad_source = GB_GRADIENT_IMAGE;
   bool grad_set = false;
 
-  std::vector<float> h_points;
+  gb::DevBuf<float> d_points;  // sampled points (xyz)
+  int64_t npoints = 0;
   bool points_virtual = true;
   bool use_sampled = false;
 
@@ -255,7 +269,13 @@ struct gb_metric {
 
   size_t device_bytes() const;  // all device buffers of the handle (gb_metric.cu)
   void release_buffers();       // frees them in the handle's stream order (gb_metric.cu)
-  size_t h_cap = 0;             // doubles held by h_params and h_out (pinned, reused across levels)
+  // Pinned memory: one block holds the status, halts, constants, optimizer state and kHostDoubles
+  // of h_params and of h_out; longer parameter vectors have one of their own, kept while large
+  // enough.
+  static constexpr size_t kHostDoubles = 66;
+  unsigned char* h_block = nullptr;
+  double* h_long = nullptr;
+  size_t h_cap = 0;  // doubles held by h_params, and by h_out
 
   int inject_fault = GB_FAULT_NONE;  // gb_metric_set_fault_injection
   std::string last_error;            // text of the last error raised by a call on this handle

@@ -329,11 +329,17 @@ extern "C" int gb_ctx_create(int device, gb_ctx** out) {
   gb_ctx* c = new gb_ctx;
   c->device = device;
   c->sm_count = sms;
+  c->kits.reserve(gb_ctx::kIdleKits);
   *out = c;
   return GB_OK;
 }
 
 extern "C" int gb_ctx_destroy(gb_ctx* ctx) {
+  if (ctx && !ctx->kits.empty() && cudaSetDevice(ctx->device) == cudaSuccess)
+    for (const HandleKit& k : ctx->kits) {
+      cudaFreeHost(k.block);
+      cudaStreamDestroy(k.stream);
+    }
   delete ctx;
   return GB_OK;
 }
@@ -362,18 +368,38 @@ extern "C" int gb_metric_create(gb_ctx* ctx, int kind, gb_metric** out) {
   m->ctx = ctx;
   m->kind = kind;
   if (kind == GB_METRIC_JOINT_HISTOGRAM_MI) m->bins = 20;  // the joint-histogram metric's default
-  cudaError_t e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMallocHost(&m->h_status, sizeof(int) * 4);
-  if (e != cudaSuccess) {
-    delete m;
-    return cuda_fail(e, "gb_metric_create");
+  const size_t consts = 64, opt = consts + (sizeof(EvalConsts) + 63) / 64 * 64;
+  const size_t doubles = opt + (opt_state_bytes() + 63) / 64 * 64;
+  {
+    std::lock_guard<std::mutex> lock(ctx->kits_lock);
+    if (!ctx->kits.empty()) {
+      m->stream = ctx->kits.back().stream;
+      m->h_block = ctx->kits.back().block;
+      ctx->kits.pop_back();
+    }
   }
+  if (!m->stream) {
+    cudaError_t e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMallocHost(&m->h_block, doubles + 2 * gb_metric::kHostDoubles * sizeof(double));
+    if (e != cudaSuccess) {
+      if (m->stream) cudaStreamDestroy(m->stream);
+      delete m;
+      return cuda_fail(e, "gb_metric_create");
+    }
+  }
+  m->h_status = reinterpret_cast<int*>(m->h_block);
+  m->h_halt = m->h_status + 4;
+  m->h_consts = reinterpret_cast<EvalConsts*>(m->h_block + consts);
+  m->h_opt = m->h_block + opt;
+  m->h_params = reinterpret_cast<double*>(m->h_block + doubles);
+  m->h_out = m->h_params + gb_metric::kHostDoubles;
+  m->h_cap = gb_metric::kHostDoubles;
   *out = m;
   return GB_OK;
 }
 
 void gb_metric::release_buffers() {
-  d_fixed.reset(); d_moving.reset(); d_fixed_s.reset(); d_moving_s.reset(); d_grad_in.reset();
+  d_points.reset(); d_fixed.reset(); d_moving.reset(); d_fixed_s.reset(); d_moving_s.reset(); d_grad_in.reset();
   d_mov4.reset(); d_samples.reset(); d_cache.reset(); d_sup.reset(); d_chunks.reset();
   d_node_first.reset(); d_node_entries.reset(); d_chunk_part.reset(); d_nodes.reset(); d_voff.reset();
   d_jhmi.reset(); d_params.reset(); d_acc.reset(); d_scratch.reset(); d_out.reset(); d_status.reset(); d_pratio.reset(); d_pdf.reset();
@@ -386,16 +412,22 @@ extern "C" int gb_metric_destroy(gb_metric* m) {
   if (m->stream) cudaStreamSynchronize(m->stream);
   m->drop_host_graphs();
   m->release_buffers();  // stream-ordered frees, before the stream goes
-  if (m->stream) cudaStreamSynchronize(m->stream);
-  if (m->h_params) cudaFreeHost(m->h_params);
-  if (m->h_out) cudaFreeHost(m->h_out);
-  if (m->h_status) cudaFreeHost(m->h_status);
-  if (m->h_consts) cudaFreeHost(m->h_consts);
-  if (m->h_opt) cudaFreeHost(m->h_opt);
-  if (m->h_halt) cudaFreeHost(m->h_halt);
+  const bool idle = cudaStreamSynchronize(m->stream) == cudaSuccess;
+  if (m->h_long) cudaFreeHost(m->h_long);
   for (int i = 0; i < gb_metric::kMaxEvents; ++i)
     if (m->events[i]) cudaEventDestroy(m->events[i]);
-  if (m->stream) cudaStreamDestroy(m->stream);
+  bool kept = false;
+  if (idle) {
+    std::lock_guard<std::mutex> lock(m->ctx->kits_lock);
+    if (m->ctx->kits.size() < gb_ctx::kIdleKits) {
+      m->ctx->kits.push_back({m->stream, m->h_block});
+      kept = true;
+    }
+  }
+  if (!kept) {
+    cudaFreeHost(m->h_block);
+    cudaStreamDestroy(m->stream);
+  }
   delete m;
   return GB_OK;
 }
@@ -525,7 +557,17 @@ extern "C" int gb_metric_set_sampled_points(gb_metric* m, const float* xyz, int6
   if (!m) return fail(GB_ERR_BAD_ARG, "null metric");
   if (n < 0 || (n > 0 && !xyz)) return fail(GB_ERR_BAD_ARG, "bad point array");
   if (n > (int64_t)0x7fffffff) return fail(GB_ERR_BAD_ARG, "more than 2^31-1 sample points");
-  m->h_points.assign(xyz, xyz + 3 * n);
+  // straight to the device (327k points 35 us; a host copy of them took 245 us, and its upload
+  // the 35 at every Initialize)
+  GB_CUDA(cudaSetDevice(m->ctx->device));
+  m->initialized = false;
+  m->npoints = 0;
+  GB_CUDA(m->d_points.alloc_on(m->stream, 3 * (size_t)n));
+  if (n > 0) {
+    GB_CUDA(cudaMemcpyAsync(m->d_points.p, xyz, 3 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+    GB_CUDA(cudaStreamSynchronize(m->stream));
+  }
+  m->npoints = n;
   m->points_virtual = virtual_space != 0;
   m->initialized = false;
   return GB_OK;
@@ -732,16 +774,10 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
   }
 
   const bool sampled = m->use_sampled;
-  if (sampled && m->h_points.empty()) return fail(GB_ERR_BAD_ARG, "VirtualSampledPointSet must have 1 or more points.");
-  const int64_t ncand = sampled ? (int64_t)(m->h_points.size() / 3) : m->virt.voxels();
+  if (sampled && m->npoints == 0) return fail(GB_ERR_BAD_ARG, "VirtualSampledPointSet must have 1 or more points.");
+  const int64_t ncand = sampled ? m->npoints : m->virt.voxels();
   if (ncand > (int64_t)0x7fffffff) return fail(GB_ERR_UNSUPPORTED, "more than 2^31-1 domain points");
   m->ndomain = ncand;
-
-  DevBuf<float> d_pts;
-  if (sampled) {
-    GB_CUDA(d_pts.alloc_on(m->stream, m->h_points.size()));
-    GB_CUDA(cudaMemcpyAsync(d_pts.p, m->h_points.data(), m->h_points.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-  }
 
   // ---- intensity ranges: Mattes' fixed range is that of the sampled points (Mattes...v4.hxx:75-327),
   // joint-histogram MI takes the whole level images
@@ -754,7 +790,7 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
   k_init_stats<<<1, 32, 0, st>>>(d_stats.p);
   if (mattes || jhmi) {
     if (mattes && sampled)
-      k_minmax_points<<<grid_for(m, ncand, 4), kBlock, 0, st>>>(d_pts.p, ncand, dfixed, dfixed_df, m->fixed_img(),
+      k_minmax_points<<<grid_for(m, ncand, 4), kBlock, 0, st>>>(m->d_points.p, ncand, dfixed, dfixed_df, m->fixed_img(),
                                                                 d_stats.p->range);
     else
       k_minmax<<<grid_for(m, m->fixed.voxels(), 8), kBlock, 0, st>>>(m->fixed_img(), m->fixed.voxels(),
@@ -774,7 +810,7 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
   GB_CUDA(vals_sorted.alloc_on(m->stream, ncand));
   GB_CUDA(recs.alloc_on(m->stream, ncand));
   BuildArgs b{};
-  b.points = sampled ? d_pts.p : nullptr;
+  b.points = sampled ? m->d_points.p : nullptr;
   b.n = ncand;
   b.points_virtual = m->points_virtual ? 1 : 0;
   b.virt = dvirt;
@@ -814,7 +850,6 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
 
   // ---- one read-back for the ranges and the sample count, while the device goes on with
   // the moving gradient
-  if (!m->h_consts) GB_CUDA(cudaMallocHost(&m->h_consts, sizeof(EvalConsts)));
   static_assert(sizeof(InitStats) <= sizeof(EvalConsts), "the pinned constants take the read-back first");
   GB_CUDA(cudaMemcpyAsync(m->h_consts, d_stats.p, sizeof(InitStats), cudaMemcpyDeviceToHost, st));
   Event read_back;
@@ -1011,14 +1046,14 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
   m->d_cache.reset();
   if (m->kind == GB_METRIC_MATTES || jhmi || bspline)
     GB_CUDA(m->d_cache.alloc_on(m->stream, std::max<int64_t>(1, m->nsamples)));
-  if (m->h_cap < 2 + P) {  // pinned staging, reused while large enough (cudaFreeHost waits for the device)
-    if (m->h_params) cudaFreeHost(m->h_params);
-    if (m->h_out) cudaFreeHost(m->h_out);
-    m->h_params = nullptr;
-    m->h_out = nullptr;
+  if (m->h_cap < 2 + P) {
+    if (m->h_long) cudaFreeHost(m->h_long);  // waits for the device
+    m->h_long = nullptr;
+    m->h_params = m->h_out = nullptr;
     m->h_cap = 0;
-    GB_CUDA(cudaMallocHost(&m->h_params, sizeof(double) * (2 + P)));
-    GB_CUDA(cudaMallocHost(&m->h_out, sizeof(double) * (2 + P)));
+    GB_CUDA(cudaMallocHost(&m->h_long, 2 * sizeof(double) * (2 + P)));
+    m->h_params = m->h_long;
+    m->h_out = m->h_long + 2 + P;
     m->h_cap = 2 + P;
   }
   GB_CUDA(m->d_consts.alloc_on(m->stream, 1));
@@ -1766,7 +1801,7 @@ extern "C" int gb_metric_get_mattes_state(gb_metric* m, double out8[8]) {
 }
 
 size_t gb_metric::device_bytes() const {
-  return d_fixed.bytes() + d_moving.bytes() + d_fixed_s.bytes() + d_moving_s.bytes() + d_grad_in.bytes() +
+  return d_points.bytes() + d_fixed.bytes() + d_moving.bytes() + d_fixed_s.bytes() + d_moving_s.bytes() + d_grad_in.bytes() +
          d_mov4.bytes() + d_samples.bytes() + d_cache.bytes() + d_sup.bytes() + d_chunks.bytes() +
          d_node_first.bytes() + d_node_entries.bytes() + d_chunk_part.bytes() + d_nodes.bytes() + d_voff.bytes() +
          d_jhmi.bytes() +

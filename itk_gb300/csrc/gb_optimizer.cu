@@ -238,8 +238,6 @@ int opt_setup(gb_metric* m, const gb_regular_step_settings* cfg, const double* s
   cudaStream_t st = m->stream;
   GB_OPT_CUDA(m->d_opt.alloc_on(st, sizeof(OptState)));
   GB_OPT_CUDA(m->d_opt_vec.alloc_on(st, (size_t)(4 * P)));
-  if (!m->h_opt) GB_OPT_CUDA(cudaMallocHost(&m->h_opt, sizeof(OptState)));
-  if (!m->h_halt) GB_OPT_CUDA(cudaMallocHost(&m->h_halt, 2 * sizeof(int)));
   OptState* S = reinterpret_cast<OptState*>(m->d_opt.p);
   double* d_prev = m->d_opt_vec.p;
   double* d_grad = d_prev + P;
@@ -327,6 +325,8 @@ extern "C" int gb_metric_set_optimizer_graphs(gb_metric* m, int on) {
   m->opt_graphs = on != 0;
   return GB_OK;
 }
+
+size_t gb::opt_state_bytes() { return sizeof(OptState); }
 
 extern "C" int gb_metric_optimize_regular_step(gb_metric* m, const gb_regular_step_settings* cfg,
                                                const double* scales, int64_t nscales, gb_optimizer_report* report) {

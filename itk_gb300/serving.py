@@ -77,13 +77,13 @@ def estimate_device_bytes(req: RegistrationRequest) -> int:
     """Device memory a request holds at its finest level, before it is admitted:
     fixed and moving images and their smoothed copies (4 B each per voxel), the
     packed moving value + gradient (16 B per voxel), samples and caches (32 B per
-    sample) and the per-handle scratch."""
+    sample), the sampled points (12 B each) and the per-handle scratch."""
     vf = int(np.prod(req.fixed.GetSize()))
     vm = int(np.prod(req.moving.GetSize()))
     smooth = any(s > 0 for s in req.smoothing_sigmas)
     img = (vf + vm) * 4 * (2 if smooth else 1) + vm * 16
     n = vf if req.sampling == NONE else sample_count(req.sampling, req.fixed.GetSize(), req.sampling_percentage)
-    return img + 32 * n + (1 << 20)
+    return img + (32 if req.sampling == NONE else 44) * n + (1 << 20)
 
 
 class _Job:

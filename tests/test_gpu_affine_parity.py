@@ -306,3 +306,25 @@ def test_fixed_samples_next_to_every_threshold(size, turned, virtual, origin):
     r = run_oracle("msq", fixed, moving, T, points=pts, compute_derivative=False)
     assert m.GetNumberOfValidPoints() == r["nvalid"]
     assert_value_close(v, r["value"], rtol=1e-6)  # values rounded to FP32 once, sums in more
+
+
+def test_handles_made_and_dropped_by_several_threads():
+    """More handles at once than a context keeps streams and pinned blocks for, from three threads, twice."""
+    from concurrent.futures import ThreadPoolExecutor
+    fixed, moving, T = small_pair()[:3]
+    grad = data.gradient_image(moving)
+    transforms = [perturbed(T, k) for k in range(7)]
+    want = [make_metric("msq", fixed, moving, t, grad).GetValueAndDerivative() for t in transforms]
+
+    def work(_):
+        ok = True
+        for _ in range(2):
+            held = [make_metric("msq", fixed, moving, t, grad) for t in transforms]
+            for m, (v, d) in zip(held, want):
+                got, deriv = m.GetValueAndDerivative()
+                ok = ok and got == v and np.array_equal(deriv, d)
+            del m, held
+        return ok
+
+    with ThreadPoolExecutor(3) as pool:
+        assert all(pool.map(work, range(3)))
