@@ -76,47 +76,109 @@ __device__ __forceinline__ const float4* stage_nodes(const EvalArgs& a, float4* 
   }
 }
 
-// Moving continuous index of one sample under the B-spline (+ initial affine):
-// cidx = A x + b + P2I M u, A x + b in double-float, the displacement u in FP32.
-// has_jac: inside the B-spline valid region (else the transform is the identity
-// there and its Jacobian is zero, itkBSplineTransform.hxx:519-523,610-616).
-__device__ __forceinline__ DFPos bspline_position(const EvalConsts& K, const float4* nodes, const EvalArgs& a,
-                                                  const float4& s, const float4& su, bool& has_jac) {
-  DFPos p = map_pos(K.map, s.x, s.y, s.z);
-  int sx, sy, sz;
-  bool valid;
-  unpack_support(su.w, sx, sy, sz, valid);
-  has_jac = valid;
-  if (!valid) return p;
-  float wx[4], wy[4], wz[4];
-  bspline_basis(su.x, wx);
-  bspline_basis(su.y, wy);
-  bspline_basis(su.z, wz);
-  float u0 = 0.f, u1 = 0.f, u2 = 0.f;
+// Displacements of R samples in one cell (start node sx, sy, sz; in-cell positions in su),
+// axis by axis, x and y components in pairs.
+//
+// A warp's 16-byte loads of one node take four cycles of the SM's 128-byte shared-memory path
+// whatever the lanes read: 256 cycles for the 64 nodes against some 150 for all of a sample's
+// instructions.  Two samples to a thread share them (173x181x149, 20 %, mesh 8: MeanSquares 46.1
+// -> 42.0 us; 256x256x200, 40 %, mesh 3: 177 -> 150 us); what remains is the moving image's gathers.
+template <int R>
+__device__ __forceinline__ void bspline_displacements(const float4* nodes, const EvalArgs& a, int sx, int sy, int sz,
+                                                      const float4 su[R], float u[R][3]) {
+  float wx[R][4], wy[R][4], wz[R][4];
 #pragma unroll
-  for (int kz = 0; kz < 4; ++kz)
+  for (int r = 0; r < R; ++r) {
+    bspline_basis(su[r].x, wx[r]);
+    bspline_basis(su[r].y, wy[r]);
+    bspline_basis(su[r].z, wz[r]);
+  }
+  f32x2 uxy[R];
+#pragma unroll
+  for (int kz = 0; kz < 4; ++kz) {
+    f32x2 pxy[R];
+    float pz[R];
 #pragma unroll
     for (int ky = 0; ky < 4; ++ky) {
-      const float4* row = nodes + (sx + a.gx * ((sy + ky) + a.gy * (sz + kz)));
-      const float wyz = wy[ky] * wz[kz];
+      const ulonglong2* row =
+          reinterpret_cast<const ulonglong2*>(nodes + (sx + a.gx * ((sy + ky) + a.gy * (sz + kz))));
+      f32x2 rxy[R];
+      float rz[R];
 #pragma unroll
       for (int kx = 0; kx < 4; ++kx) {
-        const float W = wx[kx] * wyz;
-        const float4 c = row[kx];
-        u0 = fmaf(W, c.x, u0);
-        u1 = fmaf(W, c.y, u1);
-        u2 = fmaf(W, c.z, u2);
+        const ulonglong2 c = row[kx];  // (x, y), (z, 0)
+        float cz, none;
+        unpair(c.y, cz, none);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const f32x2 w = pair(wx[r][kx]);
+          rxy[r] = kx == 0 ? mul2(w, c.x) : fma2(w, c.x, rxy[r]);
+          rz[r] = kx == 0 ? wx[r][kx] * cz : fmaf(wx[r][kx], cz, rz[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const f32x2 w = pair(wy[r][ky]);
+        pxy[r] = ky == 0 ? mul2(w, rxy[r]) : fma2(w, rxy[r], pxy[r]);
+        pz[r] = ky == 0 ? wy[r][ky] * rz[r] : fmaf(wy[r][ky], rz[r], pz[r]);
       }
     }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float corr = fmaf(K.Pm[3 * k], u0, fmaf(K.Pm[3 * k + 1], u1, K.Pm[3 * k + 2] * u2));
-    float hs, he;
-    two_sum(p.hi[k], corr, hs, he);
-    he = __fadd_rn(he, p.lo[k]);
-    p.hi[k] = __fadd_rn(hs, he);
-    p.lo[k] = __fsub_rn(he, __fsub_rn(p.hi[k], hs));
+    for (int r = 0; r < R; ++r) {
+      const f32x2 w = pair(wz[r][kz]);
+      uxy[r] = kz == 0 ? mul2(w, pxy[r]) : fma2(w, pxy[r], uxy[r]);
+      u[r][2] = kz == 0 ? wz[r][kz] * pz[r] : fmaf(wz[r][kz], pz[r], u[r][2]);
+    }
   }
+#pragma unroll
+  for (int r = 0; r < R; ++r) unpair(uxy[r], u[r][0], u[r][1]);
+}
+
+// Moving continuous indices of R samples under the B-spline (+ initial affine):
+// cidx = A x + b + P2I M u, A x + b in double-float, the displacement u in FP32.
+// has_jac: inside the B-spline valid region (else the transform is the identity
+// there and its Jacobian is zero, itkBSplineTransform.hxx:519-523,610-616).
+template <int R>
+__device__ __forceinline__ void bspline_positions(const EvalConsts& K, const float4* nodes, const EvalArgs& a,
+                                                  const float4 s[R], const float4 su[R], DFPos p[R],
+                                                  bool has_jac[R]) {
+  float u[R][3];
+  int sx, sy, sz;
+  unpack_support(su[0].w, sx, sy, sz, has_jac[0]);
+  bool together = R > 1;
+#pragma unroll
+  for (int r = 1; r < R; ++r) together = together && __float_as_uint(su[r].w) == __float_as_uint(su[0].w);
+  if (together) {
+#pragma unroll
+    for (int r = 1; r < R; ++r) has_jac[r] = has_jac[0];
+    if (has_jac[0]) bspline_displacements<R>(nodes, a, sx, sy, sz, su, u);
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      unpack_support(su[r].w, sx, sy, sz, has_jac[r]);
+      if (has_jac[r]) bspline_displacements<1>(nodes, a, sx, sy, sz, su + r, u + r);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    p[r] = map_pos(K.map, s[r].x, s[r].y, s[r].z);
+    if (!has_jac[r]) continue;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float corr = fmaf(K.Pm[3 * k], u[r][0], fmaf(K.Pm[3 * k + 1], u[r][1], K.Pm[3 * k + 2] * u[r][2]));
+      float hs, he;
+      two_sum(p[r].hi[k], corr, hs, he);
+      he = __fadd_rn(he, p[r].lo[k]);
+      p[r].hi[k] = __fadd_rn(hs, he);
+      p[r].lo[k] = __fsub_rn(he, __fsub_rn(p[r].hi[k], hs));
+    }
+  }
+}
+
+__device__ __forceinline__ DFPos bspline_position(const EvalConsts& K, const float4* nodes, const EvalArgs& a,
+                                                  const float4& s, const float4& su, bool& has_jac) {
+  DFPos p;
+  bspline_positions<1>(K, nodes, a, &s, &su, &p, &has_jac);
   return p;
 }
 
@@ -128,8 +190,10 @@ __device__ __forceinline__ float3 grad_map(const EvalConsts& K, float3 g) {
 
 #ifndef GB_KERNELS_HELPERS_ONLY
 // MeanSquares, B-spline: value sum and count; per sample a = 2 (f - m) M^T g in the cache.
-template <int GRAD, bool SMEM>
-__global__ void __launch_bounds__(kBlock) k_msq_bspline(EvalArgs a) {
+// R samples to a thread, 32 apart, so that a warp's 32 R consecutive samples mostly lie in one
+// cell.
+template <int GRAD, bool SMEM, int R>
+__global__ void __launch_bounds__(kBlock, SMEM && R == 1 ? 4 : 3) k_msq_bspline(EvalArgs a) {
   extern __shared__ float4 nodes_sh[];
   __shared__ EvalConsts K;
   __shared__ float red[kBlock / 32][1];
@@ -143,26 +207,38 @@ __global__ void __launch_bounds__(kBlock) k_msq_bspline(EvalArgs a) {
   KahanF acc[1];
   acc[0].zero();
   unsigned nv = 0;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride) {
-    const float4 s = __ldcs(a.samples + i);
-    const float4 su = __ldcs(a.sup + i);
-    bool has_jac;
-    const DFPos p = bspline_position(K, nodes, a, s, su, has_jac);
-    float m;
-    float3 g;
-    float4 cache = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (eval_moving<GRAD>(a, p, a.with_derivative != 0 && has_jac, m, g)) {
-      const float diff = s.w - m;  // MeanSquares...Threader.hxx:46
-      acc[0].add(diff * diff);
-      ++nv;
-      if (has_jac) {
-        const float3 gm = grad_map(K, g);
-        const float t = 2.f * diff;
-        cache = make_float4(t * gm.x, t * gm.y, t * gm.z, 1.f);
-      }
+  const int64_t stride = (int64_t)gridDim.x * kBlock * R;
+  const int64_t first = (int64_t)blockIdx.x * kBlock * R + (threadIdx.x >> 5) * 32 * R + (threadIdx.x & 31);
+  for (int64_t i0 = first; i0 < a.n; i0 += stride) {
+    float4 s[R], su[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const bool live = r == 0 || i0 + 32 * r < a.n;
+      s[r] = live ? __ldcs(a.samples + i0 + 32 * r) : make_float4(0.f, 0.f, 0.f, 0.f);
+      su[r] = live ? __ldcs(a.sup + i0 + 32 * r) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    if (a.with_derivative) __stcs(a.cache + i, cache);
+    DFPos p[R];
+    bool has_jac[R];
+    bspline_positions<R>(K, nodes, a, s, su, p, has_jac);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int64_t i = i0 + 32 * r;
+      if (r > 0 && i >= a.n) break;
+      float m;
+      float3 g;
+      float4 cache = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (eval_moving<GRAD>(a, p[r], a.with_derivative != 0 && has_jac[r], m, g)) {
+        const float diff = s[r].w - m;  // MeanSquares...Threader.hxx:46
+        acc[0].add(diff * diff);
+        ++nv;
+        if (has_jac[r]) {
+          const float3 gm = grad_map(K, g);
+          const float t = 2.f * diff;
+          cache = make_float4(t * gm.x, t * gm.y, t * gm.z, 1.f);
+        }
+      }
+      if (a.with_derivative) __stcs(a.cache + i, cache);
+    }
   }
   block_count(nv, a.acc_n);
   block_sums<1>(acc, red, blk);
@@ -187,8 +263,8 @@ __host__ __device__ inline size_t mattes_bspline_node_offset(int B) {
 }
 
 // Mattes pass 1, B-spline: as k_mattes_pass1_affine, caching (term, M^T g).
-template <int GRAD, bool SMEM>
-__global__ void __launch_bounds__(kBlock, SMEM ? 4 : 3) k_mattes_pass1_bspline(EvalArgs a) {
+template <int GRAD, bool SMEM, int R>
+__global__ void __launch_bounds__(kBlock, SMEM && R == 1 ? 4 : 3) k_mattes_pass1_bspline(EvalArgs a) {
   extern __shared__ __align__(16) unsigned smem_hist[];
   const int B = a.bins;
   __shared__ unsigned long long warp_total[kBlock / 32];
@@ -203,45 +279,57 @@ __global__ void __launch_bounds__(kBlock, SMEM ? 4 : 3) k_mattes_pass1_bspline(E
   const float4* nodes = stage_nodes<SMEM>(a, nodes_sh);
   __syncthreads();
   // 32-bit sample indices (a handle holds at most 2^31 - 1)
-  const unsigned n = (unsigned)a.n, stride = (unsigned)(gridDim.x * kBlock);
+  const unsigned n = (unsigned)a.n, stride = (unsigned)(gridDim.x * kBlock * R);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  unsigned base = (unsigned)(blockIdx.x * kBlock);  // the block's samples: base + thread
-  // the next iteration's record and support travel while this one is evaluated
-  float4 s_next = base + threadIdx.x < n ? __ldcs(a.samples + base + threadIdx.x) : zero;
-  float4 su_next = base + threadIdx.x < n ? __ldcs(a.sup + base + threadIdx.x) : zero;
+  const unsigned mine = (threadIdx.x >> 5) * 32 * R + (threadIdx.x & 31);  // then 32 apart
+  unsigned base = (unsigned)(blockIdx.x * kBlock * R);
   for (;;) {
-    int left = kHistSamples / kBlock;
+    int left = kHistSamples / (kBlock * R);
     for (; left > 0 && base < n; base += stride, --left) {
-      const unsigned i = base + threadIdx.x;
-      const bool live = i < n;
-      const float4 s = s_next, su = su_next;
-      s_next = i + stride < n ? __ldcs(a.samples + i + stride) : zero;
-      su_next = i + stride < n ? __ldcs(a.sup + i + stride) : zero;
-      float m = 0.f;
-      float3 g = make_float3(0.f, 0.f, 0.f);
-      bool ok = false, has_jac = false;
-      if (live) {
-        const DFPos p = bspline_position(K, nodes, a, s, su, has_jac);
-        ok = eval_moving<GRAD>(a, p, a.with_derivative != 0 && has_jac, m, g);
-        ok = ok && !(m < a.mmin) && !(m > a.mmax);  // Mattes...Threader.hxx:238-245
-      }
-      const float term = fmaf(m - a.mmin, a.m_inv_bs, 2.f);
-      if (a.with_derivative && live) {
-        const float3 gm = has_jac ? grad_map(K, g) : make_float3(0.f, 0.f, 0.f);
-        __stcs(a.cache + i, ok ? make_float4(term, gm.x, gm.y, gm.z)
-                               : make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f));
-      }
-      int pdfm = 0;
-      unsigned q[4] = {0u, 0u, 0u, 0u};
-      const int fidx = __float_as_int(s.w);
-      if (ok) {
-        float t, w6[4];
-        parzen_window(term, B, pdfm, t);
-        parzen6(t, w6);
+      const unsigned i0 = base + mine;
+      float4 s[R], su[R];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) q[k] = (__float2uint_rn(w6[k] * kQScale) + 3u) / 6u;
+      for (int r = 0; r < R; ++r) {
+        const unsigned i = i0 + 32 * r;
+        s[r] = i < n ? __ldcs(a.samples + i) : zero;
+        su[r] = i < n ? __ldcs(a.sup + i) : zero;
+        if (i + stride < n) {  // the next iteration's records towards L2 (held in registers they cost 16)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(a.samples + i + stride));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(a.sup + i + stride));
+        }
       }
-      hist_add_aggregated(ok, fidx * B + pdfm, fidx, q, h.bins, h.fm);
+      DFPos p[R];
+      bool has_jac[R];
+      bspline_positions<R>(K, nodes, a, s, su, p, has_jac);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const unsigned i = i0 + 32 * r;
+        const bool live = i < n;
+        float m = 0.f;
+        float3 g = make_float3(0.f, 0.f, 0.f);
+        bool ok = false;
+        if (live) {
+          ok = eval_moving<GRAD>(a, p[r], a.with_derivative != 0 && has_jac[r], m, g);
+          ok = ok && !(m < a.mmin) && !(m > a.mmax);  // Mattes...Threader.hxx:238-245
+        }
+        const float term = fmaf(m - a.mmin, a.m_inv_bs, 2.f);
+        if (a.with_derivative && live) {
+          const float3 gm = has_jac[r] ? grad_map(K, g) : make_float3(0.f, 0.f, 0.f);
+          __stcs(a.cache + i, ok ? make_float4(term, gm.x, gm.y, gm.z)
+                                 : make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f));
+        }
+        int pdfm = 0;
+        unsigned q[4] = {0u, 0u, 0u, 0u};
+        const int fidx = __float_as_int(s[r].w);
+        if (ok) {
+          float t, w6[4];
+          parzen_window(term, B, pdfm, t);
+          parzen6(t, w6);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) q[k] = (__float2uint_rn(w6[k] * kQScale) + 3u) / 6u;
+        }
+        hist_add_aggregated(ok, fidx * B + pdfm, fidx, q, h.bins, h.fm);
+      }
     }
     __syncthreads();
     mattes_hist_flush(a, h, hw_grid());

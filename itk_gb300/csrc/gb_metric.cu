@@ -1255,6 +1255,16 @@ static cudaError_t launch_pass2(gb_metric* m, const EvalArgs& a) {
 // B-spline / composite evaluation: node conversion (large grids), the per-sample
 // pass (MeanSquares or Mattes pass 1), then the value (Mattes without the
 // derivative: finalize) or the per-chunk and per-parameter reductions.
+// Two samples to a thread (bspline_positions): where a cell holds enough samples that pairs 32
+// apart mostly share it, and the samples fill the resident threads three times over.  Pass 1 with
+// one and two to a thread: MeanSquares 164k samples 19.5 and 19.5 us, 328k 23.6 and 23.6, 933k
+// 46.1 and 42.0; Mattes 164k 17.4 and 19.5, 328k 23.6 and 25.6, 590k 35.8 and 33.9, 3.9M 156 and 146.
+static bool bspline_pairs(const gb_metric* m) {
+  int64_t cells = 1;
+  for (int i = 0; i < 3; ++i) cells *= std::max(1, m->grid[i] - 3);
+  return m->nsamples >= (int64_t)m->ctx->sm_count * 1024 * 3 && m->nsamples >= 256 * cells;
+}
+
 static int enqueue_eval_bspline(gb_metric* m, const EvalArgs& a, bool cd, bool deriv, bool device_params) {
   const int nper = (int)m->nper;
   const bool sm = a.nodes_smem != 0;
@@ -1264,12 +1274,14 @@ static int enqueue_eval_bspline(gb_metric* m, const EvalArgs& a, bool cd, bool d
   }
   const size_t nb = sm ? bspline_node_bytes(m) : 0;
   const bool mattes = m->kind == GB_METRIC_MATTES;
+  const bool two = bspline_pairs(m);
   if (!mattes) {
     cudaError_t e;
-    if (cd) e = sm ? launch_wave(m, k_msq_bspline<kGradCentralDifference, true>, nb, a)
-                   : launch_wave(m, k_msq_bspline<kGradCentralDifference, false>, nb, a);
-    else e = sm ? launch_wave(m, k_msq_bspline<kGradImage, true>, nb, a)
-                : launch_wave(m, k_msq_bspline<kGradImage, false>, nb, a);
+    if (cd) e = sm ? launch_wave(m, k_msq_bspline<kGradCentralDifference, true, 1>, nb, a)
+                   : launch_wave(m, k_msq_bspline<kGradCentralDifference, false, 1>, nb, a);
+    else if (!sm) e = launch_wave(m, k_msq_bspline<kGradImage, false, 1>, nb, a);
+    else e = two ? launch_wave(m, k_msq_bspline<kGradImage, true, 2>, nb, a)
+                 : launch_wave(m, k_msq_bspline<kGradImage, true, 1>, nb, a);
     GB_CUDA(e);
     m->mark();
   } else {
@@ -1277,10 +1289,11 @@ static int enqueue_eval_bspline(gb_metric* m, const EvalArgs& a, bool cd, bool d
     const size_t sh1 = mattes_bspline_node_offset(B) + nb;
     if (sh1 > 200 * 1024) return fail(GB_ERR_UNSUPPORTED, "histogram too large for shared memory (bins > 160)");
     cudaError_t e;
-    if (cd) e = sm ? launch_wave(m, k_mattes_pass1_bspline<kGradCentralDifference, true>, sh1, a)
-                   : launch_wave(m, k_mattes_pass1_bspline<kGradCentralDifference, false>, sh1, a);
-    else e = sm ? launch_wave(m, k_mattes_pass1_bspline<kGradImage, true>, sh1, a)
-                : launch_wave(m, k_mattes_pass1_bspline<kGradImage, false>, sh1, a);
+    if (cd) e = sm ? launch_wave(m, k_mattes_pass1_bspline<kGradCentralDifference, true, 1>, sh1, a)
+                   : launch_wave(m, k_mattes_pass1_bspline<kGradCentralDifference, false, 1>, sh1, a);
+    else if (!sm) e = launch_wave(m, k_mattes_pass1_bspline<kGradImage, false, 1>, sh1, a);
+    else e = two ? launch_wave(m, k_mattes_pass1_bspline<kGradImage, true, 2>, sh1, a)
+                 : launch_wave(m, k_mattes_pass1_bspline<kGradImage, true, 1>, sh1, a);
     GB_CUDA(e);
     m->mark();
     if (!deriv) {  // with the derivative the value is formed by the chunk and params kernels
