@@ -22,7 +22,8 @@
 
 namespace gb {
 
-constexpr int kChunkLen = 256;     // samples per chunk (at most); also the chunk kernel's block size
+constexpr int kChunkBatch = 256;   // samples staged at a time by the chunk kernel; its block size
+constexpr int kChunkLen = 2048;    // samples per chunk (at most): 32 FP32 additions to each of its slices
 constexpr int kParamsBlock = 256;  // k_bspline_params: 8 nodes per block (warp form) or 1 (block form)
 
 __device__ __forceinline__ void unpack_support(float w, int& sx, int& sy, int& sz, bool& valid) {
@@ -341,25 +342,29 @@ __global__ void __launch_bounds__(kBlock, SMEM && R == 1 ? 4 : 3) k_mattes_pass1
   mattes_pass1_epilogue(a, h);
 }
 
-// One block per chunk of same-cell samples (at most kChunkLen = blockDim).
-// Load phase: thread j stages sample j's 12 axis weights and its 3-vector
-// a_s = 2 (f - m) M^T g (MeanSquares) or w(term) M^T g (Mattes,
-// w = sum_k log(p/pm)[f][m_k] beta3'(m_k - term)).  Sum phase: thread t owns
-// the 4 x-adjacent support nodes of row (ky, kz) = (t & 3, (t >> 2) & 3) over
-// the sample slice t >> 4 (16 slices, slice s holding samples s, s + 16, ...): per
-// sample one 16-byte load of the x weights, 12 FMAs.  The 16 slice sums of each
-// output are then added in slice order.
-constexpr int kChunkSlices = 16;
-// Grid-stride over the chunks (one full wave of blocks): block b forms chunks b, b + G, ...
-// The next chunk's per-sample inputs are loaded into registers while the current
-// chunk is summed, and (Mattes) the log(p / pm) table is staged in shared memory
-// (dynamic shared memory, bins^2 floats) once per block.
+// The sums of a_s W_k over chunks of same-cell samples, for the cell's 64 support nodes k and
+// three components (a 64 x samples by samples x 3 product).  Block b forms chunks
+// chunk_first[b] .. chunk_first[b + 1], laid out at Initialize so that the blocks of one wave
+// hold equal numbers of samples and a long cell is cut where a block ends.
+//
+// Load phase, kChunkBatch samples at a time: thread j stages sample j's 12 axis weights and its
+// 3-vector a_s = 2 (f - m) M^T g (MeanSquares) or w(term) M^T g (Mattes,
+// w = sum_k log(p/pm)[f][m_k] beta3'(m_k - term)); the next samples' inputs travel meanwhile.
+// Sum phase: lane (kz, slice) holds the 16 nodes of plane kz, 48 sums in registers, over the
+// samples of its slice (64 slices: 8 to a warp), through all of the chunk's batches.  At a
+// chunk's end the 8 slices of a warp are added by halving exchanges and the 8 warps in order.
+//
+// The sum phase is bound by its shared-memory reads and its FMAs alike: a sample costs 13
+// wavefronts and 8 x 63 FMAs to eight lanes.  With a row of 4 nodes to a thread it cost 40
+// wavefronts, and a sum over the slices and one set of partial sums for each 256 samples.  933k
+// samples in 512 cells: 28.3 -> 22.1 us, the parameters (k_bspline_params) 14.3 -> 10.2 us; 5.2M in
+// 27: 120 -> 93 and 59 -> 12.3 us.
 template <bool MATTES>
-__global__ void __launch_bounds__(kChunkLen) k_bspline_chunks(EvalArgs a) {
-  extern __shared__ float pr_sh[];
-  __shared__ __align__(16) float W1[kChunkLen][12];
-  __shared__ float4 AV[kChunkLen];
-  __shared__ float qs[kChunkSlices][192];
+__global__ void __launch_bounds__(kChunkBatch, 3) k_bspline_chunks(EvalArgs a) {
+  extern __shared__ float pr_sh[];  // Mattes: the log(p / pm) table
+  __shared__ __align__(16) float W1[kChunkBatch][12];
+  __shared__ float4 AV[kChunkBatch];
+  __shared__ __align__(16) float qs[kChunkBatch / 32][192];
   griddep_wait();
   if (halted(a)) return;
   const int B = a.bins;
@@ -368,96 +373,119 @@ __global__ void __launch_bounds__(kChunkLen) k_bspline_chunks(EvalArgs a) {
     mattes_value_groups(a);  // the value's group partials (blocks b, b + G, ...) and their sum
     for (int k = t; k < B * B; k += blockDim.x) pr_sh[k] = __ldcg(a.pratio + k);
   }
-  // this thread's inputs of one chunk: the run, the sample's support, cache and fixed bin
+  // this thread's inputs of one batch: the sample's support, cache and fixed bin
   struct In {
-    int4 ch;
     float4 su, c;
     int fbin;
   };
-  auto fetch = [&](int cidx) {
+  auto fetch = [&](int pos, int end) {
     In in;
-    in.ch = make_int4(0, 0, 0, 0);
     in.su = in.c = make_float4(0.f, 0.f, 0.f, 0.f);
     in.fbin = 0;
-    if (cidx < a.nchunks) {
-      in.ch = __ldg(a.chunks + cidx);
-      if (t < in.ch.y - in.ch.x) {
-        const int64_t i = (int64_t)in.ch.x + t;
-        in.su = __ldg(a.sup + i);
-        in.c = __ldcg(a.cache + i);
-        if (MATTES) in.fbin = __float_as_int(__ldg(&a.samples[i].w));
-      }
+    if (t < end - pos) {
+      const int64_t i = (int64_t)pos + t;
+      in.su = __ldg(a.sup + i);
+      in.c = __ldcg(a.cache + i);
+      if (MATTES) in.fbin = __float_as_int(__ldg(&a.samples[i].w));
     }
     return in;
   };
-  In cur = fetch(blockIdx.x);
+  const bool mine = (int)blockIdx.x < a.chunk_blocks;
+  int c = mine ? __ldg(a.chunk_first + blockIdx.x) : 0;
+  const int c1 = mine ? __ldg(a.chunk_first + blockIdx.x + 1) : 0;
+  int2 run = c < c1 ? __ldg(a.chunks + c) : make_int2(0, 0);
+  In cur = fetch(run.x, run.y);
   __syncthreads();  // the staged table
-  for (int cidx = blockIdx.x; cidx < a.nchunks; cidx += gridDim.x) {
-    const In nxt = fetch(cidx + gridDim.x);  // in flight while this chunk is summed
-    const int len = cur.ch.y - cur.ch.x;
+  const int lane = t & 31, warp = t >> 5, kz = lane >> 3, slice = warp * 8 + (lane & 7);
+  f32x2 acc[4][3][2];  // [ky][component][kx pair]
+#pragma unroll
+  for (int k = 0; k < 24; ++k) (&acc[0][0][0])[k] = 0ull;
+  while (c < c1) {
+    const int len = min(kChunkBatch, run.y - run.x);
+    int cn = c;
+    int2 next = make_int2(run.x + kChunkBatch, run.y);
+    if (next.x >= next.y) {
+      ++cn;
+      next = cn < c1 ? __ldg(a.chunks + cn) : make_int2(0, 0);
+    }
     if (t < len) {
       float4 av = make_float4(0.f, 0.f, 0.f, 0.f);
       if (MATTES) {
-        const float4 c = cur.c;
-        if (c.x == c.x) {
+        const float4 c4 = cur.c;
+        if (c4.x == c4.x) {
           int pdfm;
           float tt, d[4];
-          parzen_window(c.x, B, pdfm, tt);
+          parzen_window(c4.x, B, pdfm, tt);
           parzen_deriv(tt, d);
           const float* row = pr_sh + cur.fbin * B + pdfm;
           const float w = row[0] * d[0] + row[1] * d[1] + row[2] * d[2] + row[3] * d[3];
-          av = make_float4(w * c.y, w * c.z, w * c.w, 0.f);
+          av = make_float4(w * c4.y, w * c4.z, w * c4.w, 0.f);
         }
       } else {
         av = make_float4(cur.c.x, cur.c.y, cur.c.z, 0.f);
       }
-      bspline_basis(cur.su.x, &W1[t][0]);
-      bspline_basis(cur.su.y, &W1[t][4]);
-      bspline_basis(cur.su.z, &W1[t][8]);
+      float w4[12];
+      bspline_basis(cur.su.x, w4);
+      bspline_basis(cur.su.y, w4 + 4);
+      bspline_basis(cur.su.z, w4 + 8);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        *reinterpret_cast<float4*>(&W1[t][4 * k]) = make_float4(w4[4 * k], w4[4 * k + 1], w4[4 * k + 2], w4[4 * k + 3]);
       AV[t] = av;
     }
+    cur = fetch(next.x, next.y);  // in flight while this batch is summed
     __syncthreads();
-    // slice sl sums samples sl, sl + 16, ...: the two half-warps read adjacent rows of
-    // W1 and AV, in different shared-memory banks
-    const int ky = t & 3, kz = (t >> 2) & 3, sl = t >> 4;
-    float acc[4][3];
-#pragma unroll
-    for (int kx = 0; kx < 4; ++kx) acc[kx][0] = acc[kx][1] = acc[kx][2] = 0.f;
-    for (int j = sl; j < len; j += kChunkSlices) {
-      const float4 wx = *reinterpret_cast<const float4*>(&W1[j][0]);
-      const float wyz = W1[j][4 + ky] * W1[j][8 + kz];
+    for (int j = slice; j < len; j += 64) {
+      const ulonglong2 wx = *reinterpret_cast<const ulonglong2*>(&W1[j][0]);
+      const float4 wy = *reinterpret_cast<const float4*>(&W1[j][4]);
+      const float wz = W1[j][8 + kz];
       const float4 v = AV[j];
-      const float w[4] = {wx.x * wyz, wx.y * wyz, wx.z * wyz, wx.w * wyz};
+      const float vz[3] = {v.x * wz, v.y * wz, v.z * wz}, wys[4] = {wy.x, wy.y, wy.z, wy.w};
 #pragma unroll
-      for (int kx = 0; kx < 4; ++kx) {
-        acc[kx][0] = fmaf(w[kx], v.x, acc[kx][0]);
-        acc[kx][1] = fmaf(w[kx], v.y, acc[kx][1]);
-        acc[kx][2] = fmaf(w[kx], v.z, acc[kx][2]);
+      for (int ky = 0; ky < 4; ++ky)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const f32x2 p = pair(vz[d] * wys[ky]);
+          acc[ky][d][0] = fma2(wx.x, p, acc[ky][d][0]);
+          acc[ky][d][1] = fma2(wx.y, p, acc[ky][d][1]);
+        }
+    }
+    if (cn != c) {
+      // halving exchanges over the slice bits: lane bits 2 and 1 choose the ky kept, bit 0 the kx pair
+      auto halve = [&](f32x2 low, f32x2 high, int bit) {
+        const bool up = (lane & bit) != 0;
+        return add2(up ? high : low, __shfl_xor_sync(0xffffffffu, up ? low : high, bit));
+      };
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        f32x2 h[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+          h[x] = halve(halve(acc[0][d][x], acc[2][d][x], 4), halve(acc[1][d][x], acc[3][d][x], 4), 2);
+        const f32x2 sum = halve(h[0], h[1], 1);
+        const int node = 2 * (lane & 1) + 4 * (2 * ((lane >> 2) & 1) + ((lane >> 1) & 1)) + 16 * kz;
+        *reinterpret_cast<f32x2*>(&qs[warp][64 * d + node]) = sum;
+      }
+#pragma unroll
+      for (int k = 0; k < 24; ++k) (&acc[0][0][0])[k] = 0ull;
+      __syncthreads();
+      if (t < 192) {
+        float sum = qs[0][t];
+#pragma unroll
+        for (int q = 1; q < kChunkBatch / 32; ++q) sum = __fadd_rn(sum, qs[q][t]);
+        reinterpret_cast<float*>(a.chunk_part)[((size_t)c * 64 + (t & 63)) * 4 + (t >> 6)] = sum;
       }
     }
-    const int k0 = 4 * ky + 16 * kz;
-#pragma unroll
-    for (int kx = 0; kx < 4; ++kx) {
-      qs[sl][k0 + kx] = acc[kx][0];
-      qs[sl][64 + k0 + kx] = acc[kx][1];
-      qs[sl][128 + k0 + kx] = acc[kx][2];
-    }
-    __syncthreads();
-    if (t < 192) {
-      float sum = qs[0][t];
-#pragma unroll
-      for (int q = 1; q < kChunkSlices; ++q) sum = __fadd_rn(sum, qs[q][t]);
-      a.chunk_part[(size_t)cidx * 192 + t] = sum;
-    }
-    __syncthreads();  // the next chunk overwrites W1, AV and qs
-    cur = nxt;
+    __syncthreads();  // the next batch overwrites W1, AV and qs
+    c = cn;
+    run = next;
   }
   griddep_launch_dependents();
 }
 
 // For each node n and its three parameters (n + d * nper): the sum of the
 // chunk sums of every cell whose 4x4x4 support holds n, listed at Initialize in
-// node_entries (chunk * 192 + support position).  Compensated FP32 over the
+// node_entries (chunk * 64 + support position).  Compensated FP32 over the
 // list, fixed XOR trees, FP64 only for the metric's scale (1/N for MeanSquares,
 // -1/(binsize N) for Mattes, MeanSquares...Threader.hxx:71-79,
 // Mattes...Threader.hxx:446-457).  BLOCK = false: one warp per node (lane-strided
@@ -468,26 +496,25 @@ template <bool MATTES, bool BLOCK>
 __global__ void __launch_bounds__(kParamsBlock) k_bspline_params(EvalArgs a) {
   const int n = BLOCK ? (int)blockIdx.x : (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
+  // the list is Initialize's: its first entries are read before the wait for the chunk sums
+  const int first = BLOCK ? (int)threadIdx.x : lane;
+  const int step = BLOCK ? (int)blockDim.x : 32;
+  int e = 0, e1 = 0, entry = 0;
+  if (n < a.nper) {
+    e = __ldg(a.node_first + n) + first;
+    e1 = __ldg(a.node_first + n + 1);
+    if (e < e1) entry = __ldg(a.node_entries + e);
+  }
   griddep_wait();
   if (halted(a)) return;
   griddep_launch_dependents();
   // MeanSquares: the status of the value pass, scale 1 / N; Mattes: the scale formed by
   // the table kernel (0 unless the status is OK), and block 0 writes the value summed by
   // the chunk kernel's last group warp, the count and the status
-  double scale;
-  if (MATTES) {
-    scale = __ldcg(&a.marg[2]);
-  } else {
-    __shared__ double scale_s;  // FP64 division: once per block
-    if (threadIdx.x == 0) {
-      const unsigned long long N = __ldcg(a.acc_n);
-      scale_s = (__ldcg(a.status) == GB_OK && N > 0) ? 1.0 / (double)N : 0.0;
-    }
-    __syncthreads();
-    scale = scale_s;
-  }
+  const unsigned long long N = __ldcg(a.acc_n);
+  const double table_scale = MATTES ? __ldcg(&a.marg[2]) : 0.0;
+  const int status = MATTES ? GB_OK : __ldcg(a.status);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const unsigned long long N = __ldcg(a.acc_n);
     a.out[1] = (double)N;
     if (MATTES) {
       const int st = mattes_status(a);
@@ -496,20 +523,18 @@ __global__ void __launch_bounds__(kParamsBlock) k_bspline_params(EvalArgs a) {
     }
   }
   if (n >= a.nper) return;
-  const int e0 = __ldg(a.node_first + n), e1 = __ldg(a.node_first + n + 1);
   KahanF s0, s1, s2;
   s0.zero();
   s1.zero();
   s2.zero();
-  const int first = BLOCK ? (int)threadIdx.x : lane;
-  const int step = BLOCK ? (int)blockDim.x : 32;
+  auto add = [&](const float4& q) {
+    s0.add(q.x);
+    s1.add(q.y);
+    s2.add(q.z);
+  };
+  if (e < e1) add(__ldcg(a.chunk_part + entry));
 #pragma unroll 4
-  for (int e = e0 + first; e < e1; e += step) {
-    const float* src = a.chunk_part + __ldg(a.node_entries + e);
-    s0.add(__ldcg(src));
-    s1.add(__ldcg(src + 64));
-    s2.add(__ldcg(src + 128));
-  }
+  for (e += step; e < e1; e += step) add(__ldcg(a.chunk_part + __ldg(a.node_entries + e)));
   float t0 = warp_sum(s0.value()), t1 = warp_sum(s1.value()), t2 = warp_sum(s2.value());
   if (BLOCK) {
     __shared__ float wsum[kParamsBlock / 32][3];
@@ -535,6 +560,7 @@ __global__ void __launch_bounds__(kParamsBlock) k_bspline_params(EvalArgs a) {
     t2 = b2.value();
   }
   if (lane == 0) {
+    const double scale = MATTES ? table_scale : status == GB_OK && N > 0 ? 1.0 / (double)N : 0.0;
     a.out[2 + n] = (double)t0 * scale;
     a.out[2 + a.nper + n] = (double)t1 * scale;
     a.out[2 + 2 * a.nper + n] = (double)t2 * scale;

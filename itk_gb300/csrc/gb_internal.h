@@ -222,16 +222,17 @@ struct gb_metric {
   gb::DevBuf<float4> d_samples;  // (x, y, z, fixed value | fixed Parzen bin)
   gb::DevBuf<float4> d_cache;    // per-sample pass-1 result for the derivative pass
   gb::DevBuf<float4> d_sup;      // per-sample B-spline support (tx, ty, tz, packed start | valid)
-  gb::DevBuf<int4> d_chunks;     // (first sample, end sample, cell, 0) of same-cell sample runs
+  gb::DevBuf<int2> d_chunks;     // (first sample, end sample) of same-cell sample runs
+  gb::DevBuf<int> d_chunk_first; // per block of the chunk kernel: its first chunk (chunk_blocks + 1)
   gb::DevBuf<int> d_node_first;    // per node: first entry in d_node_entries (nper + 1)
-  gb::DevBuf<int> d_node_entries;  // chunk * 192 + support position of each (node, chunk) pair
-  gb::DevBuf<float> d_chunk_part;  // nchunks x 192 Jacobian partial sums
+  gb::DevBuf<int> d_node_entries;  // chunk * 64 + support position of each (node, chunk) pair
+  gb::DevBuf<float4> d_chunk_part;  // nchunks x 64 Jacobian partial sums
   gb::DevBuf<float4> d_nodes;    // B-spline coefficients as float4 nodes
   gb::DevBuf<uint32_t> d_voff;   // displacement field on a point set: each sample's nearest virtual voxel
   double jhmi_variance = 1.5;    // joint-histogram MI: variance of the joint-PDF smoothing
   double fp_res = 0.0;           // UseFloatingPointCorrection resolution, 0 = off
   gb::DevBuf<unsigned char> d_jhmi;  // joint-histogram MI constants (JhmiConsts)
-  int64_t nchunks = 0;
+  int chunk_blocks = 0;
   int64_t node_entries_count = 0;  // (node, chunk) pairs: chooses the parameter gather's shape
   int grid[3] = {0, 0, 0};       // B-spline control grid
   double mstate[8] = {0, 0, 0, 0, 0, 0, 0, 0};

@@ -262,11 +262,12 @@ struct EvalArgs {
   float4* nodes;                     // coefficient nodes (cx, cy, cz, 0), written by k_prepare_bspline
   int gx, gy, gz, nper;
   int nodes_smem;                    // evaluation kernels stage the nodes in shared memory
-  const int4* __restrict__ chunks;   // (first sample, end sample, cell id, 0) of same-cell sample runs
-  int nchunks;
+  const int2* __restrict__ chunks;   // (first sample, end sample) of same-cell sample runs
+  const int* __restrict__ chunk_first;   // per block of the chunk kernel: its first chunk (chunk_blocks + 1)
+  int chunk_blocks;
   const int* __restrict__ node_first;    // per node: first entry in node_entries (nper + 1 values)
-  const int* __restrict__ node_entries;  // chunk * 192 + support position of each (node, chunk) pair
-  float* chunk_part;                 // nchunks x 192 per-chunk Jacobian partial sums
+  const int* __restrict__ node_entries;  // chunk * 64 + support position of each (node, chunk) pair
+  float4* chunk_part;                // nchunks x 64 per-chunk Jacobian partial sums (x, y, z, -)
   // optimizer loop: nonzero once the optimizer has stopped; every evaluation
   // kernel then returns at once (iterations enqueued ahead become no-ops)
   const int* halt;

@@ -400,7 +400,7 @@ extern "C" int gb_metric_create(gb_ctx* ctx, int kind, gb_metric** out) {
 
 void gb_metric::release_buffers() {
   d_points.reset(); d_fixed.reset(); d_moving.reset(); d_fixed_s.reset(); d_moving_s.reset(); d_grad_in.reset();
-  d_mov4.reset(); d_samples.reset(); d_cache.reset(); d_sup.reset(); d_chunks.reset();
+  d_mov4.reset(); d_samples.reset(); d_cache.reset(); d_sup.reset(); d_chunks.reset(); d_chunk_first.reset();
   d_node_first.reset(); d_node_entries.reset(); d_chunk_part.reset(); d_nodes.reset(); d_voff.reset();
   d_jhmi.reset(); d_params.reset(); d_acc.reset(); d_scratch.reset(); d_out.reset(); d_status.reset(); d_pratio.reset(); d_pdf.reset();
   d_consts.reset(); d_opt.reset(); d_opt_vec.reset();
@@ -662,6 +662,23 @@ extern "C" int gb_metric_get_number_of_parameters(gb_metric* m, int64_t* nparams
   if (!m || !nparams) return fail(GB_ERR_BAD_ARG, "null argument");
   *nparams = (int64_t)m->tparams.size();
   return GB_OK;
+}
+
+// The chunk kernel's dynamic shared memory (Mattes: the staged table), and a full wave of it.
+constexpr int kChunkTableMax = 160 * 1024;  // one limit for all threads; pass 1 refuses bins above 160
+static size_t chunk_smem(const gb_metric* m) {
+  return m->kind == GB_METRIC_MATTES ? sizeof(float) * (size_t)(m->bins * m->bins) : 0;
+}
+static int64_t chunk_wave(const gb_metric* m) {
+  auto k = m->kind == GB_METRIC_MATTES ? k_bspline_chunks<true> : k_bspline_chunks<false>;
+  const size_t smem = chunk_smem(m);
+  int per_sm = 0;
+  if ((smem > 0 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkTableMax) != cudaSuccess) ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kChunkBatch, smem) != cudaSuccess || per_sm < 1) {
+    (void)cudaGetLastError();  // a table beyond shared memory is refused by the evaluation
+    per_sm = 1;
+  }
+  return (int64_t)m->ctx->sm_count * per_sm;
 }
 
 // ===========================================================================
@@ -963,30 +980,51 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
         bspline ? m->d_sup.p : nullptr, want_voff ? voff.p : nullptr, want_voff ? m->d_voff.p : nullptr, fixed_bins);
   GB_CUDA(cudaGetLastError());
 
-  // ---- B-spline: runs of same-cell samples (at most kChunkLen each) for the
-  // derivative's per-cell reduction, and each cell's first run
-  m->nchunks = 0;
+  // ---- B-spline: chunks of same-cell samples for the derivative's per-cell reduction, each
+  // cell's first chunk, and each chunk-kernel block's
+  m->chunk_blocks = 0;
   if (bspline) {
     std::vector<uint64_t> hk((size_t)m->nsamples);
     if (m->nsamples > 0)
       GB_CUDA(cudaMemcpyAsync(hk.data(), keys_sorted.p, sizeof(uint64_t) * m->nsamples, cudaMemcpyDeviceToHost, st));
     GB_CUDA(cudaStreamSynchronize(st));
-    std::vector<int4> chunks;
+    std::vector<int2> chunks;
     std::vector<int> cell_first((size_t)m->nper + 2, 0);
-    for (int64_t i = 0; i < m->nsamples;) {
+    // one wave of blocks takes `share` consecutive samples each: a block's chunks are those that
+    // start in its share, and a cell of more than one batch is also cut where a share ends (but
+    // for a cut that would leave less than 64 samples), into chunks of at most kChunkLen
+    int64_t first = 0;  // the samples outside the B-spline's valid region (cell 0) come first
+    while (first < m->nsamples && (hk[first] >> cell_shift) == 0) ++first;
+    const int64_t wave = chunk_wave(m);
+    const int64_t share = std::max<int64_t>(1, (m->nsamples - first + wave - 1) / wave);
+    const int64_t step = std::max<int64_t>(share, 128);
+    std::vector<int> chunk_first;
+    for (int64_t i = first; i < m->nsamples;) {
       const uint64_t cell = hk[i] >> cell_shift;
       int64_t j = i + 1;
-      while (j < m->nsamples && (hk[j] >> cell_shift) == cell && j - i < kChunkLen) ++j;
-      if (cell > 0) {
-        chunks.push_back(make_int4((int)i, (int)j, (int)cell, 0));
-        ++cell_first[cell + 1];
+      while (j < m->nsamples && (hk[j] >> cell_shift) == cell) ++j;
+      const bool whole = j - i <= kChunkBatch;
+      while (i < j) {
+        int64_t end = j, block = (i - first) / share;
+        if (!whole) {  // less than 64 samples before a share's end: part of the next one
+          block = std::min(wave - 1, (i - first + 63) / share);
+          const int64_t cut = first + ((i - first + 63) / step + 1) * step;
+          if (j - cut >= 64) end = cut;
+        }
+        const int64_t pieces = (end - i + kChunkLen - 1) / kChunkLen, piece = (end - i + pieces - 1) / pieces;
+        while ((int64_t)chunk_first.size() <= block) chunk_first.push_back((int)chunks.size());
+        for (; i < end; i = std::min(i + piece, end)) {
+          chunks.push_back(make_int2((int)i, (int)std::min(i + piece, end)));
+          ++cell_first[cell + 1];
+        }
       }
-      i = j;
     }
+    m->chunk_blocks = (int)chunk_first.size();
+    chunk_first.push_back((int)chunks.size());
     for (size_t c = 1; c < cell_first.size(); ++c) cell_first[c] += cell_first[c - 1];
-    if (chunks.size() > (size_t)(0x7fffffff / 192) || chunks.size() * 64 > (size_t)0x7fffffff)
+    if (chunks.size() * 64 > (size_t)0x7fffffff)
       return fail(GB_ERR_UNSUPPORTED, "too many B-spline sample chunks for 32-bit chunk-sum indices");
-    // per node: the chunk-sum entries (chunk * 192 + support position k) of every
+    // per node: the chunk-sum entries (chunk * 64 + support position k) of every
     // cell whose 4x4x4 support holds the node, cells in z, y, x order, chunks in order
     const int gx = m->grid[0], gy = m->grid[1], gz = m->grid[2];
     std::vector<int> node_first((size_t)m->nper + 1, 0);
@@ -1000,12 +1038,12 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
           for (int cx = std::max(0, ix - 3); cx <= std::min(ix, gx - 4); ++cx) {
             const int64_t cell = 1 + cx + (int64_t)gx * (cy + (int64_t)gy * cz);
             const int k = (ix - cx) + 4 * (iy - cy) + 16 * (iz - cz);
-            for (int q = cell_first[cell]; q < cell_first[cell + 1]; ++q) entries.push_back(q * 192 + k);
+            for (int q = cell_first[cell]; q < cell_first[cell + 1]; ++q) entries.push_back(q * 64 + k);
           }
     }
     node_first[m->nper] = (int)entries.size();
-    m->nchunks = (int64_t)chunks.size();
     m->d_chunks.reset();
+    m->d_chunk_first.reset();
     m->d_node_first.reset();
     m->d_node_entries.reset();
     m->d_chunk_part.reset();
@@ -1013,9 +1051,12 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
     GB_CUDA(m->d_node_first.alloc_on(m->stream, node_first.size()));
     GB_CUDA(m->d_node_entries.alloc_on(m->stream, std::max<size_t>(1, entries.size())));
     m->node_entries_count = (int64_t)entries.size();
-    GB_CUDA(m->d_chunk_part.alloc_on(m->stream, std::max<size_t>(1, chunks.size()) * 192));
+    GB_CUDA(m->d_chunk_part.alloc_on(m->stream, std::max<size_t>(1, chunks.size()) * 64));
+    GB_CUDA(m->d_chunk_first.alloc_on(m->stream, chunk_first.size()));
+    GB_CUDA(cudaMemcpyAsync(m->d_chunk_first.p, chunk_first.data(), sizeof(int) * chunk_first.size(),
+                            cudaMemcpyHostToDevice, st));
     if (!chunks.empty())
-      GB_CUDA(cudaMemcpyAsync(m->d_chunks.p, chunks.data(), sizeof(int4) * chunks.size(), cudaMemcpyHostToDevice, st));
+      GB_CUDA(cudaMemcpyAsync(m->d_chunks.p, chunks.data(), sizeof(int2) * chunks.size(), cudaMemcpyHostToDevice, st));
     GB_CUDA(cudaMemcpyAsync(m->d_node_first.p, node_first.data(), sizeof(int) * node_first.size(),
                             cudaMemcpyHostToDevice, st));
     if (!entries.empty())
@@ -1175,7 +1216,8 @@ static void fill_eval_args(gb_metric* m, EvalArgs& a, const double* d_params, do
     a.nper = (int)m->nper;
     a.nodes_smem = nodes_in_smem(m) ? 1 : 0;
     a.chunks = m->d_chunks.p;
-    a.nchunks = (int)m->nchunks;
+    a.chunk_first = m->d_chunk_first.p;
+    a.chunk_blocks = m->chunk_blocks;
     a.node_first = m->d_node_first.p;
     a.node_entries = m->d_node_entries.p;
     a.chunk_part = m->d_chunk_part.p;
@@ -1255,6 +1297,20 @@ static cudaError_t launch_pass2(gb_metric* m, const EvalArgs& a) {
 // B-spline / composite evaluation: node conversion (large grids), the per-sample
 // pass (MeanSquares or Mattes pass 1), then the value (Mattes without the
 // derivative: finalize) or the per-chunk and per-parameter reductions.
+// The chunk sums (Mattes: at least one block per value group).
+static cudaError_t launch_chunks(gb_metric* m, const EvalArgs& a) {
+  const bool mattes = m->kind == GB_METRIC_MATTES;
+  const int blocks = mattes ? std::max(m->chunk_blocks, mattes_groups((int)m->bins)) : m->chunk_blocks;
+  if (blocks == 0) return cudaSuccess;
+  const size_t smem = chunk_smem(m);
+  cudaError_t e = cudaSuccess;
+  if (mattes) e = cudaFuncSetAttribute(k_bspline_chunks<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkTableMax);
+  if (e == cudaSuccess)
+    e = launch_chain(m, mattes ? k_bspline_chunks<true> : k_bspline_chunks<false>, (unsigned)blocks, kChunkBatch, smem, a);
+  if (e == cudaSuccess) m->mark();
+  return e;
+}
+
 // Two samples to a thread (bspline_positions): where a cell holds enough samples that pairs 32
 // apart mostly share it, and the samples fill the resident threads three times over.  Pass 1 with
 // one and two to a thread: MeanSquares 164k samples 19.5 and 19.5 us, 328k 23.6 and 23.6, 933k
@@ -1307,21 +1363,7 @@ static int enqueue_eval_bspline(gb_metric* m, const EvalArgs& a, bool cd, bool d
     GB_CUDA(launch_chain(m, k_mattes_table, (unsigned)((BB + kBlock - 1) / kBlock), kBlock, 0, a));
     m->mark();
   }
-  // the chunk sums, grid-stride over one full wave (Mattes: at least one block per value
-  // group; the table staged in dynamic shared memory)
-  const int64_t want = mattes ? std::max<int64_t>(m->nchunks, mattes_groups((int)m->bins)) : m->nchunks;
-  if (want > 0) {
-    auto kc = mattes ? k_bspline_chunks<true> : k_bspline_chunks<false>;
-    const size_t csm = mattes ? sizeof(float) * (size_t)(m->bins * m->bins) : 0;
-    GB_CUDA(cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kc, kChunkLen, csm) != cudaSuccess || per_sm < 1)
-      per_sm = 4;
-    const int64_t wave = (int64_t)m->ctx->sm_count * per_sm;
-    const int64_t cblocks = std::min<int64_t>(want, std::max<int64_t>(wave, mattes ? mattes_groups((int)m->bins) : 1));
-    GB_CUDA(launch_chain(m, kc, (unsigned)cblocks, kChunkLen, csm, a));
-    m->mark();
-  }
+  GB_CUDA(launch_chunks(m, a));
   // one warp per node, or one block per node when the nodes hold many chunk entries
   const bool per_block = m->node_entries_count >= (int64_t)kParamsBlock * nper;
   if (per_block) {
@@ -1382,10 +1424,7 @@ static int enqueue_eval_field(gb_metric* m, const EvalArgs& a, bool cd, bool der
 // The B-spline chunk sums and the per-parameter gather of per-sample factors in the
 // cache (the MeanSquares form: sums / count).
 static int enqueue_bspline_sums(gb_metric* m, const EvalArgs& a) {
-  if (m->nchunks > 0) {
-    GB_CUDA(launch_chain(m, k_bspline_chunks<false>, (unsigned)m->nchunks, kChunkLen, 0, a));
-    m->mark();
-  }
+  GB_CUDA(launch_chunks(m, a));
   const int nper = (int)m->nper;
   if (m->node_entries_count >= (int64_t)kParamsBlock * nper) {
     GB_CUDA(launch_chain(m, k_bspline_params<false, true>, (unsigned)nper, kParamsBlock, 0, a));
@@ -1815,7 +1854,7 @@ extern "C" int gb_metric_get_mattes_state(gb_metric* m, double out8[8]) {
 
 size_t gb_metric::device_bytes() const {
   return d_points.bytes() + d_fixed.bytes() + d_moving.bytes() + d_fixed_s.bytes() + d_moving_s.bytes() + d_grad_in.bytes() +
-         d_mov4.bytes() + d_samples.bytes() + d_cache.bytes() + d_sup.bytes() + d_chunks.bytes() +
+         d_mov4.bytes() + d_samples.bytes() + d_cache.bytes() + d_sup.bytes() + d_chunks.bytes() + d_chunk_first.bytes() +
          d_node_first.bytes() + d_node_entries.bytes() + d_chunk_part.bytes() + d_nodes.bytes() + d_voff.bytes() +
          d_jhmi.bytes() +
          d_params.bytes() +

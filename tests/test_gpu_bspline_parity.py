@@ -177,3 +177,13 @@ def test_repeatable_and_updates(bpair_mm):
     r = run_oracle("mattes", fixed, moving, T, gradient=grad)
     assert_value_close(v3, r["value"], atol=MATTES_VALUE_ATOL)
     assert_deriv_close(d3, r["derivative"])
+
+
+@pytest.mark.parametrize("kind", ["msq", "mattes"])
+@pytest.mark.parametrize("size,mesh", [((83, 79, 73), (3, 2, 3)), ((61, 97, 83), (7, 8, 6)), ((31, 30, 29), (2, 2, 2))])
+def test_many_samples_to_a_cell_and_few(kind, size, mesh):
+    """Dense domains of 27k to 491k samples: two samples to a thread and one, cells cut between
+    blocks and into chunks, cells shorter than a batch, remainders of both."""
+    fixed, moving, A, B = data.pair_bspline(size, mesh, instance=2, multimodal_map=kind == "mattes")
+    T = composite(A, bspline_with(fixed, mesh, 5))
+    check(kind, fixed, moving, T, data.gradient_image(moving), nvalid_slack=2)
