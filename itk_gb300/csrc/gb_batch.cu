@@ -353,6 +353,7 @@ struct gb_batch {
     gb_optimizer_report report;
     int rc = GB_OK;
     bool done = false;
+    int64_t launched = 0;  // iterations enqueued
   };
   gb_ctx* ctx = nullptr;
   cudaStream_t stream = nullptr;
@@ -724,7 +725,6 @@ static int collect_halted(gb_batch* b, bool& any) {
   const int n = (int)b->active.size();
   any = false;
   if (n == 0) return GB_OK;
-  GB_B_CUDA(cudaStreamSynchronize(st));
   GB_B_CUDA(launch_dep(st, k_batch_halts, 1u, kBlock, 0, (const StepArgs*)b->d_step.p, n, b->d_halts.p,
                        (const LaunchSync*)b->d_ls.p));
   GB_B_CUDA(cudaMemcpyAsync(b->h_halts, b->d_halts.p, sizeof(int) * (n + 2), cudaMemcpyDeviceToHost, st));
@@ -772,7 +772,19 @@ extern "C" int gb_batch_run(gb_batch* b, int64_t max_iterations, int64_t* runnin
     int slot = 0;
     bool pending = false, shrink = false;
     while (max_iterations <= 0 || done < max_iterations) {
-      const int64_t k = max_iterations <= 0 ? batch : std::min(batch, max_iterations - done);
+      // no further than the last registration's own limit: past it every block returns at
+      // once, but an iteration still takes its launches' 8 us (ten iterations of eight small
+      // registrations enqueued 30: 1180 -> 968 us)
+      int64_t left = 0;
+      for (int r : b->active) {
+        const gb_batch::Reg& R = b->regs[(size_t)r];
+        if (!R.done) left = std::max<int64_t>(left, R.step.max_iterations - R.launched);
+      }
+      if (left == 0) {  // all have stopped
+        shrink = true;
+        break;
+      }
+      const int64_t k = std::min(left, max_iterations <= 0 ? batch : std::min(batch, max_iterations - done));
       if (b->persistent) {
         // one launch for all k iterations (plain launch: the next must not start early)
         PersistentArgs pa = persistent_args_of(b, (unsigned)k);
@@ -791,6 +803,7 @@ extern "C" int gb_batch_run(gb_batch* b, int64_t max_iterations, int64_t* runnin
       }
       done += k;
       b->iterations += k;
+      for (int r : b->active) b->regs[(size_t)r].launched += k;
       batch = std::min<int64_t>(batch * 2, 16);
       int* hh = b->h_halts + slot * (n + 2);
       GB_B_CUDA(launch_dep(st, k_batch_halts, 1u, kBlock, 0, (const StepArgs*)b->d_step.p, n, b->d_halts.p,
