@@ -357,6 +357,8 @@ struct gb_batch {
   };
   gb_ctx* ctx = nullptr;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;  // the Mattes phases, where both metrics run
+  cudaEvent_t fork_ev[2] = {};
   int64_t spb[3] = {8192, 8192, 8192};  // samples per virtual block: MeanSquares, Mattes pass 1, Mattes pass 2
   bool use_graph = true;
   bool persistent = false;  // k_batch_persistent: several iterations per launch
@@ -436,21 +438,47 @@ int enqueue_iteration(gb_batch* b, bool step) {
   }
   const EvalArgs* regs = b->d_eval.p;
   const int4* w = b->d_work.p;
+  // The MeanSquares registrations' blocks and the Mattes ones' two phases side by side on two
+  // streams (two branches of the captured graph): neither fills the device alone where the
+  // registrations are small, and they share nothing before the step (four of each of 226k to
+  // 290k voxels, ten iterations: 968 -> 855 us).
+  const bool msq = b->gcnt[kGrpMsqImage] || b->gcnt[kGrpMsqCD];
+  const bool mattes = b->gcnt[kGrpP1Image] || b->gcnt[kGrpP1CD];
+  const bool fork = msq && mattes;
+  cudaStream_t mt = fork ? b->side : st;
+  if (fork) {
+    GB_B_CUDA(cudaEventRecord(b->fork_ev[0], st));
+    GB_B_CUDA(cudaStreamWaitEvent(mt, b->fork_ev[0], 0));
+  }
   if (b->gcnt[kGrpMsqImage])
     GB_B_CUDA(launch_dep(st, k_batch_msq<kGradImage>, (unsigned)b->gcnt[kGrpMsqImage], kBlock, 0, regs,
                          w + b->goff[kGrpMsqImage]));
   if (b->gcnt[kGrpMsqCD])
     GB_B_CUDA(launch_dep(st, k_batch_msq<kGradCentralDifference>, (unsigned)b->gcnt[kGrpMsqCD], kBlock, 0, regs,
                          w + b->goff[kGrpMsqCD]));
-  if (b->gcnt[kGrpP1Image])
-    GB_B_CUDA(launch_dep(st, k_batch_pass1<kGradImage>, (unsigned)b->gcnt[kGrpP1Image], kBlock, b->smem1, regs,
-                         w + b->goff[kGrpP1Image]));
-  if (b->gcnt[kGrpP1CD])
-    GB_B_CUDA(launch_dep(st, k_batch_pass1<kGradCentralDifference>, (unsigned)b->gcnt[kGrpP1CD], kBlock, b->smem1,
-                         regs, w + b->goff[kGrpP1CD]));
-  if (b->gcnt[kGrpP2])
-    GB_B_CUDA(launch_dep(st, k_batch_pass2, (unsigned)b->gcnt[kGrpP2], kBlock, b->smem2, regs, w + b->goff[kGrpP2]));
-  if (step) GB_B_CUDA(launch_dep(st, k_batch_step, n, kStepBlock, 0, (const StepArgs*)b->d_step.p, regs));
+  // a branch's first kernel and the one after the join are ordinary launches
+  bool first = fork;
+  auto launch_mattes = [&](auto kernel, int group, size_t smem) {
+    const unsigned blocks = (unsigned)b->gcnt[group];
+    const int4* items = w + b->goff[group];
+    if (!first) return launch_dep(mt, kernel, blocks, kBlock, smem, regs, items);
+    first = false;
+    kernel<<<blocks, kBlock, smem, mt>>>(regs, items);
+    return cudaGetLastError();
+  };
+  if (b->gcnt[kGrpP1Image]) GB_B_CUDA(launch_mattes(k_batch_pass1<kGradImage>, kGrpP1Image, b->smem1));
+  if (b->gcnt[kGrpP1CD]) GB_B_CUDA(launch_mattes(k_batch_pass1<kGradCentralDifference>, kGrpP1CD, b->smem1));
+  if (b->gcnt[kGrpP2]) GB_B_CUDA(launch_mattes(k_batch_pass2, kGrpP2, b->smem2));
+  if (fork) {
+    GB_B_CUDA(cudaEventRecord(b->fork_ev[1], mt));
+    GB_B_CUDA(cudaStreamWaitEvent(st, b->fork_ev[1], 0));
+  }
+  if (step && fork) {
+    k_batch_step<<<n, kStepBlock, 0, st>>>((const StepArgs*)b->d_step.p, regs);
+    GB_B_CUDA(cudaGetLastError());
+  } else if (step) {
+    GB_B_CUDA(launch_dep(st, k_batch_step, n, kStepBlock, 0, (const StepArgs*)b->d_step.p, regs));
+  }
   return GB_OK;
 }
 
@@ -627,6 +655,9 @@ extern "C" int gb_batch_create(gb_ctx* ctx, gb_batch** out) {
   gb_batch* b = new gb_batch();
   b->ctx = ctx;
   cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
+  for (cudaEvent_t& ev : b->fork_ev)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev[0], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev[1], cudaEventDisableTiming);
   if (e != cudaSuccess) {
@@ -655,6 +686,9 @@ extern "C" int gb_batch_destroy(gb_batch* b) {
   for (cudaEvent_t e : b->ev)
     if (e) cudaEventDestroy(e);
   if (b->h_halts) cudaFreeHost(b->h_halts);
+  for (cudaEvent_t e : b->fork_ev)
+    if (e) cudaEventDestroy(e);
+  cudaStreamDestroy(b->side);
   cudaStreamDestroy(b->stream);
   delete b;
   return GB_OK;
