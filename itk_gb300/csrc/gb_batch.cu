@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kBlock) k_batch_msq(const EvalArgs* __restrict
   __shared__ EvalArgs sa;
   const int4 w = work[blockIdx.x];
   load_reg(regs, w.x, sa);
-  msq_affine_body<GRAD>(sa, VGrid{w.y, w.z});
+  msq_affine_body<GRAD, false, true>(sa, VGrid{w.y, w.z});
 }
 
 template <int GRAD>
@@ -193,8 +193,8 @@ __device__ __forceinline__ void block_signal(unsigned* c) {
 // The bodies out of line: each gets its own register allocation, and a call costs
 // once per work item.
 static __device__ __noinline__ void item_msq(const EvalArgs& a, VGrid vg, bool cd) {
-  if (cd) msq_affine_body<kGradCentralDifference>(a, vg);
-  else msq_affine_body<kGradImage>(a, vg);
+  if (cd) msq_affine_body<kGradCentralDifference, false, true>(a, vg);
+  else msq_affine_body<kGradImage, false, true>(a, vg);
 }
 static __device__ __noinline__ void item_pass1(const EvalArgs& a, VGrid vg, bool cd) {
   if (cd) mattes_pass1_affine_body<kGradCentralDifference>(a, vg);

@@ -507,6 +507,42 @@ __device__ __forceinline__ void block_sums_df(KahanF (&acc)[NV], float (*red)[NV
   __syncthreads();
 }
 
+// block_sums without a rounding to FP32 on the way: the threads' compensated sums as
+// double-floats, added by halving exchanges (a lane keeps half of its values at each step, so
+// the sixteen cost as many shuffles as two trees), the warps in FP64.  For batched registrations,
+// whose many small blocks each rounded their sums: the optimizer's steps magnify that where a
+// gradient is small beside its terms (ten iterations, error against 64 bits 1.4e-6 -> 1.2e-6 in
+// the worst of 9 registrations of 69x47x41; 1300 -> 1310 us for eight of 72x72x56).
+template <int NV>
+__device__ __forceinline__ void block_sums_exact(const KahanF (&acc)[NV], double (*red)[16], double* out) {
+  static_assert(NV <= 16, "sixteen values in four halvings");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  DFloat v[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = k < NV ? DFloat{acc[k].s, -acc[k].c} : DFloat{0.f, 0.f};
+#pragma unroll
+  for (int bit = 16; bit >= 1; bit >>= 1) {
+    const bool up = (lane & bit) != 0;
+    const int half = bit / 2 > 0 ? bit / 2 : 1;  // 8, 4, 2, 1 values kept, then the last pair of lanes
+#pragma unroll
+    for (int k = 0; k < half; ++k) {
+      const DFloat keep = bit > 1 && up ? v[k + half] : v[k], send = bit > 1 && !up ? v[k + half] : v[k];
+      const DFloat got{__shfl_xor_sync(0xffffffffu, send.hi, bit), __shfl_xor_sync(0xffffffffu, send.lo, bit)};
+      const DFloat s = df_two_sum(keep.hi, got.hi);
+      v[k] = df_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(keep.lo, got.lo)));
+    }
+  }
+  const int k = lane >> 1;  // this pair of lanes' value
+  if ((lane & 1) == 0) red[warp][k] = df_to_double(v[0]);
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double s = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w][threadIdx.x];
+    out[threadIdx.x] = s;
+  }
+  __syncthreads();
+}
+
 // strided_sums in double-float: dst[k] = sum_{j < cnt} src[j * NV + k], one warp per k,
 // lane l adding entries l, l + 32, ... (loads in flight together), then a fixed XOR tree.
 template <int NV>
@@ -678,10 +714,11 @@ __device__ __forceinline__ bool last_block(unsigned* ticket, VGrid vg = hw_grid(
 // ---------------------------------------------------------------------------
 // MeanSquares, affine: value = sum (f - m)^2 / N, d[p] = sum 2 (f - m) (J^T g)[p] / N
 
-template <int GRAD, bool FPC = false>
+template <int GRAD, bool FPC = false, bool EXACT = false>
 __device__ __forceinline__ void msq_affine_body(const EvalArgs& a, VGrid vg) {
   __shared__ EvalConsts K;
-  __shared__ float red[kBlock / 32][13];
+  __shared__ float red[EXACT ? 1 : kBlock / 32][13];
+  __shared__ double redx[EXACT ? kBlock / 32 : 1][16];
   __shared__ double redd[FPC ? kBlock / 32 : 1][12];
   __shared__ double blk[13], fin[13];
   double dacc[FPC ? 12 : 1];
@@ -733,7 +770,8 @@ __device__ __forceinline__ void msq_affine_body(const EvalArgs& a, VGrid vg) {
   KahanF acc[13];
   acc[0] = sq;
   jac.split(acc + 1);
-  block_sums<13>(acc, red, blk);
+  if constexpr (EXACT) block_sums_exact<13>(acc, redx, blk);
+  else block_sums<13>(acc, red, blk);
   if (FPC) {
     // the truncated derivatives: FP64 warp trees, warps in order
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
