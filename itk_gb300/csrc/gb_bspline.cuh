@@ -12,8 +12,8 @@
 // shared memory when they fit).  The Jacobian has 192 nonzeros per sample,
 //   (J^T g)[n_k + d * nper] = W_k (M^T g)_d,
 // M the composite's initial affine (identity for a plain B-spline).  Samples
-// are sorted by B-spline cell; a chunk kernel sums W_k a_s over each run of
-// same-cell samples (one thread per support node), and a gather kernel adds,
+// are sorted by B-spline cell; a chunk kernel sums W_k a_s over chunks of
+// same-cell samples (a lane keeps a plane of the support's nodes), and a gather kernel adds,
 // for every parameter, the chunk sums of the cells whose support holds its
 // node -- in a fixed order, with no atomics.
 #pragma once
