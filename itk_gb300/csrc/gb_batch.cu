@@ -804,7 +804,7 @@ extern "C" int gb_batch_run(gb_batch* b, int64_t max_iterations, int64_t* runnin
     // return at once) until they hold half of the work items, then the tables are
     // rebuilt without them.
     int slot = 0;
-    bool pending = false, shrink = false;
+    bool pending = false, shrink = false, spent = false;
     while (max_iterations <= 0 || done < max_iterations) {
       // no further than the last registration's own limit: past it every block returns at
       // once, but an iteration still takes its launches' 8 us (ten iterations of eight small
@@ -815,7 +815,7 @@ extern "C" int gb_batch_run(gb_batch* b, int64_t max_iterations, int64_t* runnin
         if (!R.done) left = std::max<int64_t>(left, R.step.max_iterations - R.launched);
       }
       if (left == 0) {  // all have stopped
-        shrink = true;
+        shrink = spent = true;
         break;
       }
       const int64_t k = std::min(left, max_iterations <= 0 ? batch : std::min(batch, max_iterations - done));
@@ -870,7 +870,7 @@ extern "C" int gb_batch_run(gb_batch* b, int64_t max_iterations, int64_t* runnin
     const int rc = collect_halted(b, any);
     if (rc) return rc;
     collected = collected || any;
-    if (!shrink) break;  // iteration budget of this call used up
+    if (!shrink || (spent && !any)) break;  // iteration budget of this call used up
     b->dirty = true;
   }
   // the caller may re-initialize or destroy the metrics of finished registrations:
