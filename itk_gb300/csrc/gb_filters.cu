@@ -332,31 +332,44 @@ struct RGPass {
 __host__ __device__ inline int rg_pitch(int ln) { return ln | 1; }  // odd: a column of lines hits every bank
 static size_t rg_tile_bytes(bool x, int ln) { return sizeof(float) * kRGLines * (size_t)(x ? rg_pitch(ln) : ln); }
 
-// The recursion DIR (1 causal, -1 anticausal) of output o of the tile's lines.
+// The recursion DIR (1 causal, -1 anticausal) of output o of the tile's lines, in two halves:
+// the block's barrier between them stands in the kernel, where every warp meets it (the
+// directions are two branches, and a barrier in either would be one of its own).
+struct RGHalf {
+  RGLine s;
+  const float* x;
+  float* sum;
+};
 template <bool X, int DIR>
-__device__ __forceinline__ void rg_tile(const RGPass& a, float* tile, int o, int64_t l0, int64_t base, bool live) {
+__device__ __forceinline__ void rg_first_half(const RGPass& a, float* tile, int o, RGHalf& h) {
   constexpr int kInc = X ? DIR : DIR * kRGLines;
   const int ln = a.ln, lane = threadIdx.x & 31;
   const int pitch = rg_pitch(ln), size = X ? kRGLines * pitch : kRGLines * ln;
   const RGTaps c = a.out[o].c.dir[DIR < 0];
-  const float scale = a.out[o].scale;
   const int half = DIR < 0 ? ln / 2 : (ln + 1) / 2;
   const int first = X ? lane * pitch + (DIR < 0 ? ln - 1 : 0) : lane + (DIR < 0 ? (ln - 1) * kRGLines : 0);
-  const float* x = tile + first;
-  float* sum = tile + (1 + o) * size + first;
-  RGLine s;
+  h.x = tile + first;
+  h.sum = tile + (1 + o) * size + first;
   const std::integral_constant<bool, (DIR < 0)> back{};
-  RGPark park{sum, kInc};
-  rg_begin(s, c, back, x, kInc, half, park);
-  __syncthreads();
-  sum += half * kInc;
+  RGPark park{h.sum, kInc};
+  rg_begin(h.s, c, back, h.x, kInc, half, park);
+  h.sum += half * kInc;
+}
+template <bool X, int DIR>
+__device__ __forceinline__ void rg_second_half(const RGPass& a, int o, RGHalf& h, int64_t base, bool live) {
+  constexpr int kInc = X ? DIR : DIR * kRGLines;
+  const int ln = a.ln;
+  const RGTaps c = a.out[o].c.dir[DIR < 0];
+  const float scale = a.out[o].scale;
+  const int half = DIR < 0 ? ln / 2 : (ln + 1) / 2;
+  const std::integral_constant<bool, (DIR < 0)> back{};
   if (X) {
-    RGAdd add{sum, kInc, scale};
-    rg_run(s, c, back, x, kInc, ln - half, add);
+    RGAdd add{h.sum, kInc, scale};
+    rg_run(h.s, c, back, h.x, kInc, ln - half, add);
   } else {
-    RGStore store{sum, kInc, scale, a.out[o].p + base + (DIR < 0 ? ln - 1 - half : half) * a.step,
+    RGStore store{h.sum, kInc, scale, a.out[o].p + base + (DIR < 0 ? ln - 1 - half : half) * a.step,
                   DIR * a.step, live};
-    rg_run(s, c, back, x, kInc, ln - half, store);
+    rg_run(h.s, c, back, h.x, kInc, ln - half, store);
   }
 }
 
@@ -390,9 +403,13 @@ __global__ void __launch_bounds__(64 * NOUT) k_rg_pass(RGPass a) {
   }
   copy_async_wait();
   __syncthreads();
-  // causal and anticausal warps take the same code with their own strides
-  if (warp & 1) rg_tile<X, -1>(a, tile, warp >> 1, l0, base, live);
-  else rg_tile<X, 1>(a, tile, warp >> 1, l0, base, live);
+  // even warps causal, odd ones anticausal; past the middle each adds what the other parked
+  RGHalf h;
+  if (warp & 1) rg_first_half<X, -1>(a, tile, warp >> 1, h);
+  else rg_first_half<X, 1>(a, tile, warp >> 1, h);
+  __syncthreads();
+  if (warp & 1) rg_second_half<X, -1>(a, warp >> 1, h, base, live);
+  else rg_second_half<X, 1>(a, warp >> 1, h, base, live);
   if (X) {
     // rows leave in order
     __syncthreads();
