@@ -418,11 +418,14 @@ int64_t vblocks(int64_t n, int64_t spb) {
   return std::max<int64_t>(1, std::min<int64_t>(std::max((n + spb - 1) / spb, spread), kMaxBlocks));
 }
 
-// Cleared accumulators and constants of every running registration.
+// Cleared accumulators and constants of every running registration.  The clear is an ordinary
+// launch: the evaluation before it may have ended in a join of two streams, and it writes what
+// both of them used (once per run, or per evaluation of the autotuning).
 int enqueue_prepare_all(gb_batch* b) {
   const unsigned n = (unsigned)b->active.size();
   cudaStream_t st = b->stream;
-  GB_B_CUDA(launch_dep(st, k_batch_clear, n, kBlock, 0, (const ClearItem*)b->d_clear.p));
+  k_batch_clear<<<n, kBlock, 0, st>>>((const ClearItem*)b->d_clear.p);
+  GB_B_CUDA(cudaGetLastError());
   GB_B_CUDA(launch_dep(st, k_batch_prepare, n * kConstEntries, 32, 0, (const EvalArgs*)b->d_eval.p));
   return GB_OK;
 }
