@@ -335,9 +335,7 @@ __global__ void __launch_bounds__(kBlock, SMEM && R == 1 ? 4 : 3) k_mattes_pass1
     __syncthreads();
     mattes_hist_flush(a, h, hw_grid());
     if (base >= n) break;
-    __syncthreads();
-    for (int k = threadIdx.x; k < 2 * B * B; k += blockDim.x) h.bins[k] = 0u;
-    __syncthreads();
+    mattes_hist_restart(a, h);
   }
   mattes_pass1_epilogue(a, h);
 }

@@ -1150,6 +1150,10 @@ __device__ __forceinline__ float u64_to_float(unsigned long long v) {
 
 // Shared memory of Mattes pass 1: the joint histogram, the column sums (two words each:
 // the low kColBits bits of every bin's count, and those above) and the fixed-bin counts.
+// A column's words hold one flush: its low word takes less than 2^20 from each of at most 160
+// rows (2^27.4), its high one the weights of kHistSamples samples (below 2^40) less those 20
+// bits.  They go to global memory before the next flush; run on, the low word wraps after
+// 4096 / bins flushes at the earliest.
 constexpr int kColBits = 20;
 struct MattesHist {
   unsigned *bins, *cols, *fm;
@@ -1188,6 +1192,22 @@ __device__ __forceinline__ void mattes_hist_flush(const EvalArgs& a, const Matte
   if ((threadIdx.x & 31) == 0) h.warp_total[threadIdx.x >> 5] += t;
 }
 
+__device__ __forceinline__ void mattes_add_column(const EvalArgs& a, const MattesHist& h, int k) {
+  const unsigned long long c = (unsigned long long)h.cols[2 * k] + ((unsigned long long)h.cols[2 * k + 1] << kColBits);
+  if (c) atomicAdd(&a.colsum[k], c);
+}
+
+// Between two flushes: the column sums to global memory, bins and columns to zero.
+__device__ __forceinline__ void mattes_hist_restart(const EvalArgs& a, const MattesHist& h) {
+  __syncthreads();
+  for (int k = threadIdx.x; k < a.bins; k += blockDim.x) {
+    mattes_add_column(a, h, k);
+    h.cols[2 * k] = h.cols[2 * k + 1] = 0u;
+  }
+  for (int k = threadIdx.x; k < 2 * a.bins * a.bins; k += blockDim.x) h.bins[k] = 0u;
+  __syncthreads();
+}
+
 // End of Mattes pass 1 (any transform), after the last flush: the marginals, the valid
 // count (every valid sample counts in one fixed bin) and the histogram's total (the value's
 // normalization, JointPDFSum).  Each is one integer atomic per block and entry, so the
@@ -1200,9 +1220,7 @@ __device__ __forceinline__ void mattes_pass1_epilogue(const EvalArgs& a, const M
     const unsigned f = h.fm[k];
     if (f) atomicAdd(&a.fmarg[k], (unsigned long long)f);
     n += f;
-    const unsigned long long c =
-        (unsigned long long)h.cols[2 * k] + ((unsigned long long)h.cols[2 * k + 1] << kColBits);
-    if (c) atomicAdd(&a.colsum[k], c);
+    mattes_add_column(a, h, k);
   }
   n = warp_sum_u(n);
   if ((threadIdx.x & 31) == 0 && n) atomicAdd(a.acc_n, (unsigned long long)n);
@@ -1430,9 +1448,7 @@ __device__ __forceinline__ void mattes_pass1_affine_body(const EvalArgs& a, VGri
     __syncthreads();
     mattes_hist_flush(a, h, vg);
     if (base >= n) break;
-    __syncthreads();
-    for (int k = threadIdx.x; k < 2 * a.bins * a.bins; k += blockDim.x) h.bins[k] = 0u;
-    __syncthreads();
+    mattes_hist_restart(a, h);
   }
   mattes_pass1_epilogue(a, h);
 }
