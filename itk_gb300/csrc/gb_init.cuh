@@ -99,6 +99,7 @@ __device__ __forceinline__ bool d_nearest_index(const DGeom& g, const double p[3
 struct DFMap {
   float hi[9], lo[9], bhi[3], blo[3];
   float size[3];  // sum of |coefficient * origin|, at least |b|
+  float unit;     // error of an index / (size + sum of |coefficient * point|)
   int n[3];
 };
 
@@ -106,18 +107,22 @@ struct DFMap {
 // cycles of its SM, an FP32 one a quarter of a cycle, so Initialize takes the point's index
 // and value this way and leaves to FP64 only the points whose result could differ: `sure`
 // says that floor, rounding and the buffer test are those of the FP64 index, whose distance
-// from this one is at most err (2^-43 of the summed magnitudes; two-sums and FMA products
-// lose a few 2^-46).  NaN and infinity are never sure.
+// from this one is at most err.  NaN and infinity are never sure.
+//
+// With u = 2^-24, B the sum of |coefficient * origin| and A the |coefficient * point| in order:
+// the coefficients' pairs lose u^2 (B + A1 + A2 + A3), the products' errors 2 u^2 (A1 + A2 + A3),
+// the additions u + qe and then to e (|e| reaches u (4B + 5A1 + 4A2 + 3A3)) u^2 (12B + 17A1 + 11A2
+// + 6A3), the last pair u |e| (where e exceeds s), and t and its pair 3 u^2: below 2^-43 of the
+// sum.  With one product to a row those are 4B + 9A1, 2B + 3A1 and 3: below 2^-44.
 struct DFIndex {
   int floor[3], nearest[3];
   float t[3], tl[3];  // c - floor in [0, 1], as a pair
-  float err;
+  float err[3];
   bool sure;
 };
 
 __device__ __forceinline__ DFIndex df_index(const DFMap& M, const float p[3]) {
   DFIndex c;
-  c.err = 0.f;
   c.sure = true;
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
@@ -132,7 +137,7 @@ __device__ __forceinline__ DFIndex df_index(const DFMap& M, const float p[3]) {
       e = __fadd_rn(e, __fadd_rn(u, qe));
       size += fabsf(q);
     }
-    const float err = size * 0x1p-43f;
+    const float err = size * M.unit;
     const float hi = __fadd_rn(s, e), lo = __fsub_rn(e, __fsub_rn(hi, s));
     const float f = floorf(hi);
     float t, tl, d, dl;
@@ -149,7 +154,7 @@ __device__ __forceinline__ DFIndex df_index(const DFMap& M, const float p[3]) {
     c.nearest[r] = c.floor[r] + (half >= 0.f ? 1 : 0);
     c.t[r] = t;
     c.tl[r] = tl;
-    c.err = fmaxf(c.err, err);
+    c.err[r] = err;
     c.sure = c.sure && fabsf(hi) < 4194304.f && t > 2.f * err &&
              __fsub_rn(__fsub_rn(1.f, t), tl) > 2.f * err && fabsf(half) > 2.f * err;
   }
@@ -176,11 +181,10 @@ __device__ __forceinline__ DFVal df_lerp(const DFVal& a, const DFVal& b, float t
   return {h, __fsub_rn(e, __fsub_rn(h, s))};
 }
 
-// interp_d rounded to float; false if the pairs' error leaves the rounding open.  The index's
-// error moves the value by at most err times the corners' range along each axis; a sixteenth
-// of that bound, still above what occurs, is asked for here (a float past it would be the
-// other neighbour of a value half-way between two): with the whole bound a fifth of the warps
-// went on to FP64.
+// interp_d rounded to float; false if the pairs' error leaves the rounding open.  The
+// interpolation is linear along each axis, so an index's error moves the value by at most err
+// times the largest difference along that axis; the interpolations themselves lose 26 u^2 of
+// the largest corner along x and 53 u^2 each along y and z (u = 2^-24; 2^-40 is 256).
 __device__ __forceinline__ bool df_interp(const float* __restrict__ img, const DFMap& M, const DFIndex& c, float& out) {
   int b0[3], b1[3];
   float t[3], tl[3];
@@ -205,7 +209,14 @@ __device__ __forceinline__ bool df_interp(const float* __restrict__ img, const D
   const DFVal xx0 = df_lerp(x00, x10, t[1], tl[1]), xx1 = df_lerp(x01, x11, t[1], tl[1]);
   const DFVal r = df_lerp(xx0, xx1, t[2], tl[2]);
   const float range = hi - lo, big = fmaxf(fabsf(lo), fabsf(hi));
-  const float e = fmaf(0.25f * c.err, range, 0x1p-41f * big);
+  float e = 0x1p-40f * big;
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    const int x = 1 << r, y = r == 0 ? 2 : 1, z = r == 2 ? 2 : 4;  // this axis, the others
+    const float slope = fmaxf(fmaxf(fabsf(v[x] - v[0]), fabsf(v[x + y] - v[y])),
+                              fmaxf(fabsf(v[x + z] - v[z]), fabsf(v[x + y + z] - v[y + z])));
+    e = fmaf(c.err[r], slope, e);
+  }
   out = __fadd_rn(r.h, __fadd_rn(r.l, e));
   const bool flat = range == 0.f;  // eight equal values (a background): that value
   if (flat) out = __fadd_rn(v[0], 0.f);

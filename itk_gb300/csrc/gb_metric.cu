@@ -113,10 +113,14 @@ static DGeom to_dgeom(const Geom& g) {
 
 static DFMap to_dfmap(const Geom& g) {
   DFMap d;
+  d.unit = 0x1p-44f;
   for (int r = 0; r < 3; ++r) {
     double b = 0.0, size = 0.0;
     for (int k = 0; k < 3; ++k) {
-      split_df(g.p2i[3 * r + k], d.hi[3 * r + k], d.lo[3 * r + k]);
+      const double a = g.p2i[3 * r + k];
+      split_df(a, d.hi[3 * r + k], d.lo[3 * r + k]);
+      if (r != k && a != 0.0) d.unit = 0x1p-43f;
+      if (a != 0.0 && std::fabs(a) < 0x1p-100) d.hi[3 * r + k] = NAN;  // its pair would be subnormal: never sure
       b -= g.p2i[3 * r + k] * g.origin[k];
       size += std::fabs(g.p2i[3 * r + k] * g.origin[k]);
     }
