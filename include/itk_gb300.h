@@ -72,7 +72,9 @@ const char *gb_metric_last_error(gb_metric *m);
 const char *gb_version(void);
 
 /* ---- device context ---------------------------------------------------- */
-/* Binds a CUDA device; the context owns no stream of its own. */
+/* Binds a CUDA device.  The context keeps the streams and pinned blocks of up to 16 destroyed
+ * metric handles for the next ones.  A context destroyed before its metric and batch handles
+ * stays valid for them and goes with the last; no new handle is made from it. */
 int gb_ctx_create(int device, gb_ctx **out);
 int gb_ctx_destroy(gb_ctx *ctx);
 /* Number of SMs and total/free device memory in bytes. */

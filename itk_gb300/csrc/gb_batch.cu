@@ -667,6 +667,7 @@ extern "C" int gb_batch_create(gb_ctx* ctx, gb_batch** out) {
     delete b;
     return cuda_fail(e, "gb_batch_create");
   }
+  ctx_retain(ctx);
   *out = b;
   return GB_OK;
 }
@@ -693,6 +694,7 @@ extern "C" int gb_batch_destroy(gb_batch* b) {
     if (e) cudaEventDestroy(e);
   cudaStreamDestroy(b->side);
   cudaStreamDestroy(b->stream);
+  ctx_release(b->ctx);
   delete b;
   return GB_OK;
 }

@@ -172,6 +172,8 @@ void batch_eval_args(gb_metric* m, EvalArgs& a);
 // A metric handle's stream and block of pinned memory.  The block costs 110 us to get and as
 // much to give back, a tenth of a small registration each; a context keeps the last
 // kIdleKits of them that its handles gave back, idle and synchronized, until it is destroyed.
+// Handles give theirs back into their context, so a context that is destroyed before its
+// handles goes with the last of them (ctx_retain, ctx_release).
 struct HandleKit {
   cudaStream_t stream = nullptr;
   unsigned char* block = nullptr;
@@ -181,9 +183,16 @@ struct gb_ctx {
   int device = 0;
   int sm_count = 0;
   static constexpr size_t kIdleKits = 16;
-  std::mutex kits_lock;
+  std::mutex lock;
   std::vector<HandleKit> kits;
+  int handles = 0;         // metric and batch handles alive
+  bool destroyed = false;  // by gb_ctx_destroy
 };
+
+namespace gb {
+void ctx_retain(gb_ctx* ctx);
+void ctx_release(gb_ctx* ctx);
+}
 
 struct gb_metric {
   gb_ctx* ctx = nullptr;

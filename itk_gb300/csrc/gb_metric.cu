@@ -338,13 +338,38 @@ extern "C" int gb_ctx_create(int device, gb_ctx** out) {
   return GB_OK;
 }
 
-extern "C" int gb_ctx_destroy(gb_ctx* ctx) {
-  if (ctx && !ctx->kits.empty() && cudaSetDevice(ctx->device) == cudaSuccess)
+static void ctx_free(gb_ctx* ctx) {
+  if (!ctx->kits.empty() && cudaSetDevice(ctx->device) == cudaSuccess)
     for (const HandleKit& k : ctx->kits) {
       cudaFreeHost(k.block);
       cudaStreamDestroy(k.stream);
     }
   delete ctx;
+}
+
+void gb::ctx_retain(gb_ctx* ctx) {
+  std::lock_guard<std::mutex> lock(ctx->lock);
+  ++ctx->handles;
+}
+
+void gb::ctx_release(gb_ctx* ctx) {
+  bool last;
+  {
+    std::lock_guard<std::mutex> lock(ctx->lock);
+    last = --ctx->handles == 0 && ctx->destroyed;
+  }
+  if (last) ctx_free(ctx);
+}
+
+extern "C" int gb_ctx_destroy(gb_ctx* ctx) {
+  if (!ctx) return GB_OK;
+  bool last;
+  {
+    std::lock_guard<std::mutex> lock(ctx->lock);
+    ctx->destroyed = true;
+    last = ctx->handles == 0;
+  }
+  if (last) ctx_free(ctx);
   return GB_OK;
 }
 
@@ -375,7 +400,7 @@ extern "C" int gb_metric_create(gb_ctx* ctx, int kind, gb_metric** out) {
   const size_t consts = 64, opt = consts + (sizeof(EvalConsts) + 63) / 64 * 64;
   const size_t doubles = opt + (opt_state_bytes() + 63) / 64 * 64;
   {
-    std::lock_guard<std::mutex> lock(ctx->kits_lock);
+    std::lock_guard<std::mutex> lock(ctx->lock);
     if (!ctx->kits.empty()) {
       m->stream = ctx->kits.back().stream;
       m->h_block = ctx->kits.back().block;
@@ -398,6 +423,7 @@ extern "C" int gb_metric_create(gb_ctx* ctx, int kind, gb_metric** out) {
   m->h_params = reinterpret_cast<double*>(m->h_block + doubles);
   m->h_out = m->h_params + gb_metric::kHostDoubles;
   m->h_cap = gb_metric::kHostDoubles;
+  ctx_retain(ctx);
   *out = m;
   return GB_OK;
 }
@@ -422,7 +448,7 @@ extern "C" int gb_metric_destroy(gb_metric* m) {
     if (m->events[i]) cudaEventDestroy(m->events[i]);
   bool kept = false;
   if (idle) {
-    std::lock_guard<std::mutex> lock(m->ctx->kits_lock);
+    std::lock_guard<std::mutex> lock(m->ctx->lock);
     if (m->ctx->kits.size() < gb_ctx::kIdleKits) {
       m->ctx->kits.push_back({m->stream, m->h_block});
       kept = true;
@@ -432,6 +458,7 @@ extern "C" int gb_metric_destroy(gb_metric* m) {
     cudaFreeHost(m->h_block);
     cudaStreamDestroy(m->stream);
   }
+  ctx_release(m->ctx);
   delete m;
   return GB_OK;
 }
