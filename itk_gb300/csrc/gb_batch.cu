@@ -758,7 +758,12 @@ extern "C" int gb_batch_add(gb_batch* b, gb_metric* m, const gb_regular_step_set
   return GB_OK;
 }
 
+static int dependency_timeout() {
+  return fail(GB_ERR_TIMEOUT, "batched iteration: a dependency wait ran out in the persistent kernel");
+}
+
 // Collects every registration of the current tables that has stopped (the stream drains first).
+// The last iterations' halt words are read only here, so their error word is too.
 static int collect_halted(gb_batch* b, bool& any) {
   cudaStream_t st = b->stream;
   const int n = (int)b->active.size();
@@ -768,6 +773,7 @@ static int collect_halted(gb_batch* b, bool& any) {
                        (const LaunchSync*)b->d_ls.p));
   GB_B_CUDA(cudaMemcpyAsync(b->h_halts, b->d_halts.p, sizeof(int) * (n + 2), cudaMemcpyDeviceToHost, st));
   GB_B_CUDA(cudaStreamSynchronize(st));
+  if (b->h_halts[n + 1] != 0) return dependency_timeout();
   std::vector<int> idx;
   for (int k = 0; k < n; ++k)
     if (b->h_halts[k] && !b->regs[(size_t)b->active[k]].done) idx.push_back(b->active[k]);
@@ -852,8 +858,7 @@ extern "C" int gb_batch_run(gb_batch* b, int64_t max_iterations, int64_t* runnin
       if (pending) {
         GB_B_CUDA(cudaEventSynchronize(b->ev[slot ^ 1]));
         const int* ph = b->h_halts + (slot ^ 1) * (n + 2);
-        if (ph[n + 1] != 0)
-          return fail(GB_ERR_TIMEOUT, "batched iteration: a dependency wait ran out in the persistent kernel");
+        if (ph[n + 1] != 0) return dependency_timeout();
         if (ph[n] == 0) {  // all stopped
           shrink = true;
           break;
