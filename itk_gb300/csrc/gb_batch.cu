@@ -537,6 +537,7 @@ int rebuild_tables(gb_batch* b) {
     m->eval_halt = &R.step.st->halt;
     batch_eval_args(m, ev[k]);
     m->eval_halt = nullptr;
+    m->status_on_host = false;
     sa[k] = R.step;
     ci[k] = ClearItem{reinterpret_cast<unsigned long long*>(m->d_acc.p), (long long)(m->acc_bytes / 8),
                       &R.step.st->halt};
@@ -806,6 +807,7 @@ extern "C" int gb_batch_run(gb_batch* b, int64_t max_iterations, int64_t* runnin
     }
     const int n = (int)b->active.size();
     if (n == 0) break;
+    for (int r : b->active) b->regs[(size_t)r].m->status_on_host = false;  // evaluated since, maybe
     if (!b->persistent) {  // on every call: the handles may have been evaluated in between
       const int rc = enqueue_prepare_all(b);
       if (rc) return rc;

@@ -276,6 +276,7 @@ struct gb_metric {
   bool host_graph_tried[2] = {false, false};
   void drop_host_graphs();
   bool eval_host_out = false;  // while an affine host call's chain is enqueued: results to pinned memory
+  bool status_on_host = false;  // the last evaluation was such a call: d_status holds an earlier one's
 
   size_t device_bytes() const;  // all device buffers of the handle (gb_metric.cu)
   void release_buffers();       // frees them in the handle's stream order (gb_metric.cu)

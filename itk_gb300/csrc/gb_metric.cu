@@ -1582,6 +1582,7 @@ int gb::enqueue_eval(gb_metric* m, const double* d_params, double* d_out, bool d
   cudaStream_t st = m->stream;
   EvalArgs a;
   fill_eval_args(m, a, d_params, d_out, deriv);
+  m->status_on_host = m->eval_host_out;
   // an affine or B-spline transform with device parameters: the prepare kernel zeroes the accumulators (one node fewer, and the chain stays
   // kernel-to-kernel); otherwise a memset unless the caller has cleared them
   if (device_params && !acc_cleared && chain_clears_in_prepare(m)) a.clear_acc = 1;
@@ -1783,6 +1784,7 @@ static int run_host_chain(gb_metric* m, bool deriv) {
   }
   if (m->host_exec[k]) {
     GB_CUDA(cudaGraphLaunch(m->host_exec[k], m->stream));
+    m->status_on_host = chain_clears_in_prepare(m) && !is_bspline(m);  // as host_chain chooses
     return GB_OK;
   }
   return host_chain(m, deriv);
@@ -1920,7 +1922,8 @@ extern "C" int gb_metric_synchronize(gb_metric* m) {
   gb::ErrorScope scope_(m, __func__);
   if (!m) return fail(GB_ERR_BAD_ARG, "null metric");
   GB_CUDA(cudaSetDevice(m->ctx->device));
-  GB_CUDA(cudaMemcpyAsync(m->h_status, m->d_status.p, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+  if (!m->status_on_host)
+    GB_CUDA(cudaMemcpyAsync(m->h_status, m->d_status.p, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
   GB_CUDA(cudaStreamSynchronize(m->stream));
   return *m->h_status;
 }
