@@ -12,9 +12,9 @@
 //   k_batch_step     AdvanceOneStep, the next evaluation readied   block of one
 // captured once as a CUDA graph and relaunched per iteration.     registration
 // A registration's blocks are a fixed function of its own sample count and the
-// samples-per-block setting (chosen by gb_batch_autotune), so its results are
-// the same alone and in any mix: the reduction orders do not depend on the
-// other registrations.  Registrations that stop are collected between batches
+// samples-per-block setting (chosen by gb_batch_autotune), or, in pass 1, sum integers only,
+// so its results are the same alone and in any mix: the reduction orders do not depend on
+// the other registrations.  Registrations that stop are collected between batches
 // of iterations and the tables are rebuilt without them.
 //
 // Reference semantics: the single-registration loop (gb_optimizer.cu) and the
@@ -403,19 +403,33 @@ struct gb_batch {
 namespace {
 
 // Virtual blocks of a registration with n samples: at most spb samples each, and the
-// samples of a small one spread over up to kSpread blocks of at least kSpreadSamples.
-// Both are functions of n and spb alone (the result does not depend on the batch).  About
-// 80 because Mattes pass 2 forms its FP64 value groups (79 of them for 50 bins) one per
-// block before it streams: with n / spb blocks, a registration of 30,000 samples formed 20
-// in each of 4 blocks (139 us of a 430 us iteration) on 4 of 152 SMs.  Below 512 samples a
-// block's histogram flush costs what the spread gains (80 x 256: 2 %, 40 x 1024: -15 %).
-// Eight registrations of 27,000 to 290,000 samples, ten iterations: 4546 -> 1859 us; the 64
-// of the benchmark (autotuned): 938 -> 974 registrations/s, its 32 Mattes ones 1037 -> 1146.
-constexpr int64_t kSpread = 80, kSpreadSamples = 512;
+// samples of a small one spread over up to kSpread blocks of at least kSpreadMsq or
+// kSpreadSamples.  Both are functions of n and spb alone (the result does not depend on the
+// batch).  About 80 because Mattes pass 2 forms its FP64 value groups (79 of them for 50 bins,
+// 128 for 64) one per block before it streams: with n / spb blocks, a registration of 30,000
+// samples formed 20 in each of 4 blocks (139 us of a 430 us iteration) on 4 of 152 SMs.  Below
+// 512 samples a block's own work costs what the spread gains (80 x 256: 2 %, 40 x 1024: -15 %).
+// MeanSquares has no groups, and a block's sums cost as much as 1000 samples: with blocks of 512,
+// 200 registrations of 64,000 samples took 13 % longer than with n / spb, the persistent form
+// 44 %; with 2560 (ten to a thread) -15 and -1 %.  One alone takes 780 us (512: 670, n / spb:
+// 1350), one of 262,144 samples 930 (930, 1580).
+// Eight registrations of 27,000 to 290,000 samples, ten iterations: 4510 -> 1305 us.
+constexpr int64_t kSpread = 80, kSpreadSamples = 512, kSpreadMsq = 2560;
 
-int64_t vblocks(int64_t n, int64_t spb) {
-  const int64_t spread = std::min<int64_t>(kSpread, (n + kSpreadSamples - 1) / kSpreadSamples);
+int64_t vblocks(int64_t n, int64_t spb, int64_t least) {
+  const int64_t spread = std::min<int64_t>(kSpread, (n + least - 1) / least);
   return std::max<int64_t>(1, std::min<int64_t>(std::max((n + spb - 1) / spb, spread), kMaxBlocks));
+}
+
+// Mattes pass 1's follow the batch as well: its sums are integers, the same for any blocks.  The
+// whole batch takes about `fill` of them, but no registration fewer than n / spb: a block clears
+// and flushes a histogram.  In the persistent form the blocks that are resident (64 registrations
+// of 52,429 samples, 30 iterations: 12.8 -> 9.8 ms, 200 of 12,800: 17.4 -> 14.6), per phase two
+// waves (9.6 -> 9.3 and 13.1 -> 12.9 ms; one wave 9.7 and 13.2).
+constexpr int64_t kFillPersistent = 3, kFillPhase = 10;  // per SM
+int64_t pass1_vblocks(int64_t n, int64_t spb, int64_t total, int64_t fill) {
+  const int64_t most = vblocks(n, spb, kSpreadSamples), least = std::min(most, (n + spb - 1) / spb);
+  return std::max<int64_t>(1, std::max(least, std::min(most, (n * fill + total - 1) / total)));
 }
 
 // Cleared accumulators and constants of every running registration.  The clear is an ordinary
@@ -531,6 +545,13 @@ int rebuild_tables(gb_batch* b) {
   int maxbins = 0;
   b->reg_work.assign(n, 0);
   b->total_work = 0;
+  int64_t mattes_samples = 0;
+  for (int r : b->active) {
+    const gb_metric* m = b->regs[(size_t)r].m;
+    if (m->kind != GB_METRIC_MEAN_SQUARES) mattes_samples += m->nsamples;
+  }
+  const int64_t fill = (b->persistent ? kFillPersistent : kFillPhase) * b->ctx->sm_count;
+  std::vector<int64_t> first(n);  // virtual blocks of the MeanSquares pass or Mattes pass 1
   for (size_t k = 0; k < n; ++k) {
     gb_batch::Reg& R = b->regs[(size_t)b->active[k]];
     gb_metric* m = R.m;
@@ -543,16 +564,16 @@ int rebuild_tables(gb_batch* b) {
                       &R.step.st->halt};
     const bool cd = m->grad_source == GB_GRADIENT_CENTRAL_DIFFERENCE;
     if (m->kind == GB_METRIC_MEAN_SQUARES) {
-      const int64_t nv = vblocks(m->nsamples, b->spb[kSpbMsq]);
+      const int64_t nv = first[k] = vblocks(m->nsamples, b->spb[kSpbMsq], kSpreadMsq);
       for (int64_t v = 0; v < nv; ++v)
         work[cd ? kGrpMsqCD : kGrpMsqImage].push_back(make_int4((int)k, (int)v, (int)nv, 0));
       b->reg_work[k] = nv;
     } else {
       maxbins = std::max(maxbins, (int)m->bins);
-      const int64_t n1 = vblocks(m->nsamples, b->spb[kSpbPass1]);
+      const int64_t n1 = first[k] = pass1_vblocks(m->nsamples, b->spb[kSpbPass1], mattes_samples, fill);
       for (int64_t v = 0; v < n1; ++v)
         work[cd ? kGrpP1CD : kGrpP1Image].push_back(make_int4((int)k, (int)v, (int)n1, 0));
-      const int64_t n2 = vblocks(m->nsamples, b->spb[kSpbPass2]);
+      const int64_t n2 = vblocks(m->nsamples, b->spb[kSpbPass2], kSpreadSamples);
       for (int64_t v = 0; v < n2; ++v) work[kGrpP2].push_back(make_int4((int)k, (int)v, (int)n2, 0));
       b->reg_work[k] = n1 + n2;
     }
@@ -580,11 +601,11 @@ int rebuild_tables(gb_batch* b) {
     gb_metric* m = b->regs[(size_t)b->active[(size_t)k]].m;
     const bool cd = m->grad_source == GB_GRADIENT_CENTRAL_DIFFERENCE;
     const bool msq = m->kind == GB_METRIC_MEAN_SQUARES;
-    const int64_t nv = vblocks(m->nsamples, b->spb[msq ? kSpbMsq : kSpbPass1]);
+    const int64_t nv = first[(size_t)k];
     const int kind = msq ? (cd ? kItMsqCD : kItMsqImage) : (cd ? kItP1CD : kItP1Image);
     for (int64_t v = 0; v < nv; ++v) items.push_back(make_int4(kind, k, (int)v, (int)nv));
     meta[(size_t)k].x = (int)nv;
-    if (!msq) meta[(size_t)k].y = (int)vblocks(m->nsamples, b->spb[kSpbPass2]);
+    if (!msq) meta[(size_t)k].y = (int)vblocks(m->nsamples, b->spb[kSpbPass2], kSpreadSamples);
   }
   for (int k : order)
     for (int v = 0; v < meta[(size_t)k].y; ++v) items.push_back(make_int4(kItP2, k, v, meta[(size_t)k].y));
