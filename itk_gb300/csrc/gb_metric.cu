@@ -1697,8 +1697,8 @@ __global__ void k_host_prologue(EvalArgs a, const uint4* src, uint4* dst, int wo
 __global__ void k_host_epilogue(const double* out, int n, const int* status, double* h_out, int* h_status) {
   griddep_wait();
   griddep_launch_dependents();
-  for (int k = threadIdx.x; k < n; k += blockDim.x) h_out[k] = __ldcg(out + k);
-  if (threadIdx.x == 0) *h_status = __ldcg(status);
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) h_out[k] = __ldcg(out + k);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *h_status = __ldcg(status);
 }
 
 // The host call's device work: the constants (affine) or float4 nodes (B-spline)
@@ -1734,7 +1734,11 @@ static int host_chain(gb_metric* m, bool deriv) {
     }
     int rc = enqueue_eval(m, nullptr, m->d_out.p, deriv, false, true);
     if (rc) return rc;
-    GB_CUDA(launch_chain(m, k_host_epilogue, 1u, 256, 0, (const double*)m->d_out.p, (int)(2 + (deriv ? P : 0)),
+    const int results = (int)(2 + (deriv ? P : 0));
+    // four results to a thread: one block for all of them took 83 us longer for 89,373 (mesh 28),
+    // 35 for 27,783 (mesh 20), 3 for 3995 (mesh 8), and more than the driver's copies from mesh 20 on
+    const unsigned eblocks = (unsigned)std::min(32, (results + 1023) / 1024);
+    GB_CUDA(launch_chain(m, k_host_epilogue, eblocks, 256, 0, (const double*)m->d_out.p, results,
                          (const int*)m->d_status.p, (double*)out_dev, (int*)status_dev));
     return GB_OK;
   }
