@@ -344,16 +344,18 @@ __global__ void __launch_bounds__(kBlock, SMEM && R == 1 ? 4 : 3) k_mattes_pass1
 }
 
 // The sums of a_s W_k over chunks of same-cell samples, for the cell's 64 support nodes k and
-// three components (a 64 x samples by samples x 3 product).  Block b forms chunks
-// chunk_first[b] .. chunk_first[b + 1], laid out at Initialize so that the blocks of one wave
-// hold equal numbers of samples and a long cell is cut where a block ends.
+// three components (a 64 x samples by samples x 3 product).  A team of TEAM threads forms a
+// chunk: a block (chunks chunk_first[b] .. chunk_first[b + 1], laid out at Initialize so that the
+// blocks of one wave hold equal numbers of samples and a long cell is cut where a block ends) or,
+// where the cells are small and many, a warp (warp w of block b: b + w G, then every 8 G-th).
 //
-// Load phase, kChunkBatch samples at a time: thread j stages sample j's 12 axis weights and its
+// Load phase, TEAM samples at a time: thread j stages sample j's 12 axis weights and its
 // 3-vector a_s = 2 (f - m) M^T g (MeanSquares) or w(term) M^T g (Mattes,
 // w = sum_k log(p/pm)[f][m_k] beta3'(m_k - term)); the next samples' inputs travel meanwhile.
 // Sum phase: lane (kz, slice) holds the 16 nodes of plane kz, 48 sums in registers, over the
-// samples of its slice (kChunkSlices: 8 to a warp).  After kFoldBatches batches, and at a chunk's
-// end, the 8 slices of a warp are added by halving exchanges; the 8 warps follow, compensated.
+// samples of its slice (kChunkSlices of a block's: 8 to a warp).  After kFoldBatches batches, and at a
+// chunk's end, the 8 slices of a warp are added by halving exchanges; a block's 8 warps follow,
+// compensated.
 //
 // A sum's last additions are its largest, so a chunk of 2048 samples summed plainly to its end loses
 // more than eight of 256 do: roundings of 23 (u S)^2 in the mean square against 17 (S the chunk's
@@ -367,7 +369,14 @@ __global__ void __launch_bounds__(kBlock, SMEM && R == 1 ? 4 : 3) k_mattes_pass1
 // wavefronts, and a sum over the slices and one set of partial sums for each 256 samples.  933k
 // samples in 512 cells: 28.3 -> 22.1 us, the parameters (k_bspline_params) 14.3 -> 10.2 us; 5.2M in
 // 27: 120 -> 93 and 59 -> 12.3 us.
-template <bool MATTES>
+//
+// A block spends 2 us on a chunk whatever its size.  546k samples, by blocks and by warps: 21,952
+// cells 86 and 22.5 us, 8000 36.5 and 18.2; MeanSquares calls 282 and 224 us, 142 and 124, 4096 cells 105
+// and 101, 2744 90 and 88; 1728 cells alike, 512 22 us more (a warp needs 8 times as long for a
+// cell).  Hence the rule: chunks of less than kWarpChunk samples in the mean, and at least
+// kWarpChunks of them to a block.
+constexpr int kWarpChunk = 256, kWarpChunks = 6;
+template <bool MATTES, int TEAM>
 __global__ void __launch_bounds__(kChunkBatch, 3) k_bspline_chunks(EvalArgs a) {
   extern __shared__ float pr_sh[];  // Mattes: the log(p / pm) table
   __shared__ __align__(16) float W1[kChunkBatch][12];
@@ -376,10 +385,11 @@ __global__ void __launch_bounds__(kChunkBatch, 3) k_bspline_chunks(EvalArgs a) {
   griddep_wait();
   if (halted(a)) return;
   const int B = a.bins;
-  const int t = threadIdx.x;
+  constexpr bool kWarps = TEAM == 32;
+  const int t = threadIdx.x % TEAM, w0 = threadIdx.x - t;  // in the team, its first staging row
   if (MATTES) {
     mattes_value_groups(a);  // the value's group partials (blocks b, b + G, ...) and their sum
-    for (int k = t; k < B * B; k += blockDim.x) pr_sh[k] = __ldcg(a.pratio + k);
+    for (int k = threadIdx.x; k < B * B; k += blockDim.x) pr_sh[k] = __ldcg(a.pratio + k);
   }
   // this thread's inputs of one batch: the sample's support, cache and fixed bin
   struct In {
@@ -399,22 +409,27 @@ __global__ void __launch_bounds__(kChunkBatch, 3) k_bspline_chunks(EvalArgs a) {
     return in;
   };
   const bool mine = (int)blockIdx.x < a.chunk_blocks;
-  int c = mine ? __ldg(a.chunk_first + blockIdx.x) : 0;
-  const int c1 = mine ? __ldg(a.chunk_first + blockIdx.x + 1) : 0;
+  const int next_chunk = kWarps ? (int)gridDim.x * (kChunkBatch / TEAM) : 1;
+  int c = kWarps ? (int)(blockIdx.x + gridDim.x * (threadIdx.x / TEAM)) : mine ? __ldg(a.chunk_first + blockIdx.x) : 0;
+  const int c1 = kWarps ? __ldg(a.chunk_first + a.chunk_blocks) : mine ? __ldg(a.chunk_first + blockIdx.x + 1) : 0;
+  auto sync = [] {
+    if (kWarps) __syncwarp();
+    else __syncthreads();
+  };
   int2 run = c < c1 ? __ldg(a.chunks + c) : make_int2(0, 0);
   In cur = fetch(run.x, run.y);
   __syncthreads();  // the staged table
-  const int lane = t & 31, warp = t >> 5, kz = lane >> 3, slice = warp * 8 + (lane & 7);
+  const int lane = t & 31, warp = threadIdx.x >> 5, kz = lane >> 3, slice = (t >> 5) * 8 + (lane & 7);
   f32x2 acc[4][3][2];  // [ky][component][kx pair]
 #pragma unroll
   for (int k = 0; k < 24; ++k) (&acc[0][0][0])[k] = 0ull;
   int batch = 0;  // of the chunk
   while (c < c1) {
-    const int len = min(kChunkBatch, run.y - run.x);
+    const int len = min(TEAM, run.y - run.x);
     int cn = c;
-    int2 next = make_int2(run.x + kChunkBatch, run.y);
+    int2 next = make_int2(run.x + TEAM, run.y);
     if (next.x >= next.y) {
-      ++cn;
+      cn += next_chunk;
       next = cn < c1 ? __ldg(a.chunks + cn) : make_int2(0, 0);
     }
     if (t < len) {
@@ -439,16 +454,16 @@ __global__ void __launch_bounds__(kChunkBatch, 3) k_bspline_chunks(EvalArgs a) {
       bspline_basis(cur.su.z, w4 + 8);
 #pragma unroll
       for (int k = 0; k < 3; ++k)
-        *reinterpret_cast<float4*>(&W1[t][4 * k]) = make_float4(w4[4 * k], w4[4 * k + 1], w4[4 * k + 2], w4[4 * k + 3]);
-      AV[t] = av;
+        *reinterpret_cast<float4*>(&W1[w0 + t][4 * k]) = make_float4(w4[4 * k], w4[4 * k + 1], w4[4 * k + 2], w4[4 * k + 3]);
+      AV[w0 + t] = av;
     }
     cur = fetch(next.x, next.y);  // in flight while this batch is summed
-    __syncthreads();
-    for (int j = slice; j < len; j += kChunkSlices) {
-      const ulonglong2 wx = *reinterpret_cast<const ulonglong2*>(&W1[j][0]);
-      const float4 wy = *reinterpret_cast<const float4*>(&W1[j][4]);
-      const float wz = W1[j][8 + kz];
-      const float4 v = AV[j];
+    sync();
+    for (int j = slice; j < len; j += kChunkSlices / (kChunkBatch / TEAM)) {
+      const ulonglong2 wx = *reinterpret_cast<const ulonglong2*>(&W1[w0 + j][0]);
+      const float4 wy = *reinterpret_cast<const float4*>(&W1[w0 + j][4]);
+      const float wz = W1[w0 + j][8 + kz];
+      const float4 v = AV[w0 + j];
       const float vz[3] = {v.x * wz, v.y * wz, v.z * wz}, wys[4] = {wy.x, wy.y, wy.z, wy.w};
 #pragma unroll
       for (int ky = 0; ky < 4; ++ky)
@@ -483,8 +498,13 @@ __global__ void __launch_bounds__(kChunkBatch, 3) k_bspline_chunks(EvalArgs a) {
     ++batch;
     if (cn != c) {
       batch = 0;
-      __syncthreads();
-      if (t < 192) {
+      sync();
+      if (kWarps) {  // two nodes to a lane
+        const float* q = qs[warp];
+#pragma unroll
+        for (int node = lane; node < 64; node += 32)
+          a.chunk_part[(size_t)c * 64 + node] = make_float4(q[node], q[64 + node], q[128 + node], 0.f);
+      } else if (t < 192) {
         KahanF sum;
         sum.zero();
 #pragma unroll
@@ -492,7 +512,7 @@ __global__ void __launch_bounds__(kChunkBatch, 3) k_bspline_chunks(EvalArgs a) {
         reinterpret_cast<float*>(a.chunk_part)[((size_t)c * 64 + (t & 63)) * 4 + (t >> 6)] = sum.value();
       }
     }
-    __syncthreads();  // the next batch overwrites W1, AV and qs
+    sync();  // the next batch overwrites W1, AV and qs
     c = cn;
     run = next;
   }

@@ -242,6 +242,7 @@ struct gb_metric {
   double fp_res = 0.0;           // UseFloatingPointCorrection resolution, 0 = off
   gb::DevBuf<unsigned char> d_jhmi;  // joint-histogram MI constants (JhmiConsts)
   int chunk_blocks = 0;
+  int chunk_warp_blocks = 0;     // blocks of the chunk kernel where a warp takes a chunk, else 0
   int64_t node_entries_count = 0;  // (node, chunk) pairs: chooses the parameter gather's shape
   int grid[3] = {0, 0, 0};       // B-spline control grid
   double mstate[8] = {0, 0, 0, 0, 0, 0, 0, 0};

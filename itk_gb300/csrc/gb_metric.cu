@@ -701,7 +701,7 @@ static size_t chunk_smem(const gb_metric* m) {
   return m->kind == GB_METRIC_MATTES ? sizeof(float) * (size_t)(m->bins * m->bins) : 0;
 }
 static int64_t chunk_wave(const gb_metric* m) {
-  auto k = m->kind == GB_METRIC_MATTES ? k_bspline_chunks<true> : k_bspline_chunks<false>;
+  auto k = m->kind == GB_METRIC_MATTES ? k_bspline_chunks<true, kChunkBatch> : k_bspline_chunks<false, kChunkBatch>;
   const size_t smem = chunk_smem(m);
   int per_sm = 0;
   if ((smem > 0 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkTableMax) != cudaSuccess) ||
@@ -1013,7 +1013,7 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
 
   // ---- B-spline: chunks of same-cell samples for the derivative's per-cell reduction, each
   // cell's first chunk, and each chunk-kernel block's
-  m->chunk_blocks = 0;
+  m->chunk_blocks = m->chunk_warp_blocks = 0;
   if (bspline) {
     std::vector<uint64_t> hk((size_t)m->nsamples);
     if (m->nsamples > 0)
@@ -1051,6 +1051,8 @@ extern "C" int gb_metric_initialize(gb_metric* m) {
       }
     }
     m->chunk_blocks = (int)chunk_first.size();
+    const bool by_warps = (int64_t)chunks.size() * kWarpChunk > m->nsamples && (int64_t)chunks.size() >= kWarpChunks * wave;
+    m->chunk_warp_blocks = by_warps ? (int)wave : 0;
     chunk_first.push_back((int)chunks.size());
     for (size_t c = 1; c < cell_first.size(); ++c) cell_first[c] += cell_first[c - 1];
     if (chunks.size() * 64 > (size_t)0x7fffffff)
@@ -1329,17 +1331,24 @@ static cudaError_t launch_pass2(gb_metric* m, const EvalArgs& a) {
 // pass (MeanSquares or Mattes pass 1), then the value (Mattes without the
 // derivative: finalize) or the per-chunk and per-parameter reductions.
 // The chunk sums (Mattes: at least one block per value group).
-static cudaError_t launch_chunks(gb_metric* m, const EvalArgs& a) {
+template <int TEAM>
+static cudaError_t launch_chunks_by(gb_metric* m, const EvalArgs& a, int blocks) {
   const bool mattes = m->kind == GB_METRIC_MATTES;
-  const int blocks = mattes ? std::max(m->chunk_blocks, mattes_groups((int)m->bins)) : m->chunk_blocks;
+  if (mattes) blocks = std::max(blocks, mattes_groups((int)m->bins));
   if (blocks == 0) return cudaSuccess;
   const size_t smem = chunk_smem(m);
   cudaError_t e = cudaSuccess;
-  if (mattes) e = cudaFuncSetAttribute(k_bspline_chunks<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkTableMax);
+  if (mattes)
+    e = cudaFuncSetAttribute(k_bspline_chunks<true, TEAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkTableMax);
   if (e == cudaSuccess)
-    e = launch_chain(m, mattes ? k_bspline_chunks<true> : k_bspline_chunks<false>, (unsigned)blocks, kChunkBatch, smem, a);
+    e = launch_chain(m, mattes ? k_bspline_chunks<true, TEAM> : k_bspline_chunks<false, TEAM>, (unsigned)blocks,
+                     kChunkBatch, smem, a);
   if (e == cudaSuccess) m->mark();
   return e;
+}
+static cudaError_t launch_chunks(gb_metric* m, const EvalArgs& a) {
+  return m->chunk_warp_blocks > 0 ? launch_chunks_by<32>(m, a, m->chunk_warp_blocks)
+                                  : launch_chunks_by<kChunkBatch>(m, a, m->chunk_blocks);
 }
 
 // Two samples to a thread (bspline_positions): where a cell holds enough samples that pairs 32
