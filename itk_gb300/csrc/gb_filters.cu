@@ -375,7 +375,7 @@ __device__ __forceinline__ void rg_second_half(const RGPass& a, int o, RGHalf& h
 
 template <bool X, int NOUT>
 __global__ void __launch_bounds__(64 * NOUT) k_rg_pass(RGPass a) {
-  extern __shared__ float tile[];
+  extern __shared__ __align__(16) float tile[];
   const int ln = a.ln, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t l0 = (int64_t)blockIdx.x * kRGLines, l = l0 + lane;
   const bool live = l < a.lines;
@@ -565,7 +565,7 @@ struct RGGradZ {
 static size_t rgz_array(int ln) { return (size_t)kRGzLines * (size_t)ln; }
 
 __global__ void __launch_bounds__(96) k_rg_grad_z(RGGradZ a) {
-  extern __shared__ float tile[];
+  extern __shared__ __align__(16) float tile[];
   constexpr int kInc = 2 * kRGzLines;
   const int ln = a.ln, lane = threadIdx.x & 31, comp = threadIdx.x >> 5;
   const int line = lane & (kRGzLines - 1), back = lane >> 4;
