@@ -367,8 +367,8 @@ __global__ void __launch_bounds__(kBlock, SMEM && R == 1 ? 4 : 3) k_mattes_pass1
 // The sum phase is bound by its shared-memory reads and its FMAs alike: a sample costs 13
 // wavefronts and 8 x 63 FMAs to eight lanes.  With a row of 4 nodes to a thread it cost 40
 // wavefronts, and a sum over the slices and one set of partial sums for each 256 samples.  933k
-// samples in 512 cells: 28.3 -> 22.1 us, the parameters (k_bspline_params) 14.3 -> 10.2 us; 5.2M in
-// 27: 120 -> 93 and 59 -> 12.3 us.
+// samples in 512 cells: 28.3 -> 22.1 us (23 with the fold), the parameters (k_bspline_params)
+// 14.3 -> 10.2 us; 5.2M in 27: 120 -> 93 and 59 -> 12.3 us.
 //
 // A block spends 2 us on a chunk whatever its size.  546k samples, by blocks and by warps: 21,952
 // cells 86 and 22.5 us, 8000 36.5 and 18.2; MeanSquares calls 282 and 224 us, 142 and 124, 4096 cells 105
